@@ -216,7 +216,7 @@ struct gg_ctx {
     // tree
     int ncap = 0;
     DevBuf<int> t_start, t_end, t_level, t_parent, t_sys, t_nch, t_child, t_bnd, t_depth, t_nnodes;
-    DevBuf<unsigned> t_bstat, t_ticket;
+    DevBuf<unsigned> t_bstat;
     DevBuf<double> t_mass64;
     DevBuf<GGNode> nodes;
     // walk
@@ -299,7 +299,7 @@ struct gg_ctx {
         f(poff); f(in_rec); f(part); f(dom); f(extent_mm); f(hmm); f(tkey); f(tval); f(tlist2); f(tout2);
         f(keys); f(perm); f(rank); f(sort_scratch);
         f(t_start); f(t_end); f(t_level); f(t_parent); f(t_sys); f(t_nch); f(t_child); f(t_bnd);
-        f(t_depth); f(t_nnodes); f(t_bstat); f(t_ticket); f(t_mass64); f(nodes);
+        f(t_depth); f(t_nnodes); f(t_bstat); f(t_mass64); f(nodes);
         f(oldacc); f(vel); f(newpos); f(kin); f(kin_counter); f(dts); f(oldacc_save); f(tcost); f(gkey); f(gorder);
         f(e_chunks); f(e_first); f(e_part); f(e_out);
         f(groups); f(ngroups); f(gscan); f(toff); f(flag); f(flagscan); f(tlist); f(tout); f(scan_scratch);
@@ -611,8 +611,7 @@ static gg_status ensure_tree(gg_ctx *c)
         (st = c->t_parent.ensure(cap)) || (st = c->t_sys.ensure(cap)) || (st = c->t_nch.ensure(cap)) ||
         (st = c->t_child.ensure(cap)) || (st = c->t_bnd.ensure(cap * 8)) ||
         (st = c->t_mass64.ensure(cap)) || (st = c->nodes.ensure(cap)) || (st = c->t_depth.ensure(GG_MAX_DEPTH + 4)) ||
-        (st = c->t_nnodes.ensure(4)) || (st = c->t_bstat.ensure((size_t)GG_MAX_DEPTH * G)) ||
-        (st = c->t_ticket.ensure(GG_MAX_DEPTH)))
+        (st = c->t_nnodes.ensure(4)) || (st = c->t_bstat.ensure((size_t)GG_MAX_DEPTH * G + 2)))
         return st;
     c->ncap = (int)cap;
     return GG_OK;
@@ -624,7 +623,7 @@ static TreeBuf tree_buf(gg_ctx *c)
     tb.start = c->t_start.p; tb.end = c->t_end.p; tb.level = c->t_level.p; tb.parent = c->t_parent.p;
     tb.sys = c->t_sys.p; tb.nch = c->t_nch.p; tb.child = c->t_child.p;
     tb.bnd = c->t_bnd.p; tb.mass64 = c->t_mass64.p; tb.depth_beg = c->t_depth.p; tb.nnodes = c->t_nnodes.p;
-    tb.bstat = c->t_bstat.p; tb.ticket = c->t_ticket.p; tb.err = c->err.p;
+    tb.bstat = c->t_bstat.p; tb.barrier = nullptr; tb.err = c->err.p;
     tb.cap = c->ncap;
     return tb;
 }
@@ -668,7 +667,9 @@ extern "C" gg_status gg_build(gg_ctx *c, const gg_domain *domains)
     }
     if (N > 0 && !gathered) gg_launch_permute(c->perm.p, c->in_rec.p, c->part.p, c->rank.p, N, s);
     if (timing) cudaEventRecord(c->ev[2], s);
-    gg_launch_tree(c->keys.p, c->poff.p, S, c->cfg.leaf_size, c->ncap, tree_buf(c), c->part.p, c->dom.p, c->nodes.p, s);
+    if ((st = gg_launch_tree(c->keys.p, c->poff.p, S, N, c->cfg.leaf_size, c->ncap, tree_buf(c), c->part.p, c->dom.p,
+                             c->nodes.p, s)))
+        return st;
     if (timing) cudaEventRecord(c->ev[3], s);
     GG_CUDA_TRY(cudaGetLastError());
     c->built = true;

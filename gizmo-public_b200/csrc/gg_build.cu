@@ -21,14 +21,19 @@
 //     into chunks of leaf_size (the reference splits such near-coincident
 //     particles at random, forcetree.c:219-231).
 // Moments are FP64 sums (mass, mass-weighted position), children summed in
-// key order, one depth per launch from the deepest up, with the centre of mass
+// key order, one depth after the other from the deepest up, with the centre of mass
 // falling back to the geometric centre for empty cells (forcetree.c:764-781).
+#include <algorithm>
+
 #include "gg_internal.cuh"
 #include "gg_kernels.cuh"
 
-#define TB_THREADS 256
-#define TB_GROUP 8                      // threads per node in the count/write kernels
+#define TB_THREADS 512
+#define TB_GROUP 8                      // threads per node when children are looked for
 #define TB_NODES (TB_THREADS / TB_GROUP)
+#define TB_PER_SM 4                     // blocks per SM that find children: 2,048 threads of 32 registers hide the
+                                        // searches' dependent loads
+#define TB_MOM_PER_SM 2                 // blocks per SM that form moments (64 registers)
 
 __global__ void k_permute(const unsigned *__restrict__ perm, const GGPart *__restrict__ in, GGPart *__restrict__ out,
                           unsigned *__restrict__ rank, int n)
@@ -39,23 +44,6 @@ __global__ void k_permute(const unsigned *__restrict__ perm, const GGPart *__res
         out[i] = in[src];
         rank[src] = (unsigned)i;
     }
-}
-
-// roots: one per system, geometric level 0 (the domain cube), depth 0
-__global__ void k_tree_roots(int S, const int *__restrict__ poff, TreeBuf tb)
-{
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) {
-        tb.depth_beg[0] = 0;
-        tb.depth_beg[1] = S;
-        tb.nnodes[0] = S;
-    }
-    if (s >= S) return;
-    tb.start[s] = poff[s];
-    tb.end[s] = poff[s + 1];
-    tb.level[s] = 0;
-    tb.parent[s] = -1;
-    tb.sys[s] = s;
 }
 
 // deepest common level of two keys (0..21)
@@ -106,239 +94,300 @@ __device__ __forceinline__ void tb_st_status(unsigned *p, unsigned v)
 #define TB_PUBLISHED 0x80000000u
 #define TB_SPIN_LIMIT (1 << 22)
 
-// One depth of the build in one launch.  Blocks take their chunk of the
-// depth's nodes in ticket order (an atomic counter, so that every block a
-// block waits for has already started).  Count: 8 threads per node find the
-// 7 digit boundaries (or the chunk split of a full-depth cell) and the child
-// count; the block publishes its children total.  Then each block adds up the
-// totals of the blocks before it -- they publish before they wait on anyone,
-// so the bounded wait ends -- and writes its nodes' children at contiguous
-// indices from there; the last block also sets the next depth's range.  A
-// child index at or past the node capacity is not written and sets
-// GG_EBIT_NODE_OVERFLOW (the capacity is sized so that it cannot happen).
-__global__ void __launch_bounds__(TB_THREADS) k_tree_depth(int depth, const unsigned long long *__restrict__ keys,
-                                                           TreeBuf tb, int leaf)
+// Barrier of the whole (cooperatively launched) grid: the blocks count up one
+// word, and the n-th barrier is passed once n * gridDim.x have arrived.  A wait
+// that reaches its limit records GG_EBIT_SORT_TIMEOUT and returns false; the
+// block then leaves the kernel.
+__device__ __forceinline__ bool tb_grid_barrier(unsigned *word, unsigned &target, int *err)
 {
-    __shared__ int s_sum, s_ticket, s_off, s_tot;
+    __syncthreads();
+    if (gridDim.x == 1) return true;
+    __shared__ int s_ok;
+    if (threadIdx.x == 0) {
+        target += gridDim.x;
+        __threadfence();
+        atomicAdd(word, 1u);
+        int spins = 0;
+        while (tb_ld_status(word) < target && ++spins < TB_SPIN_LIMIT) __nanosleep(20);
+        s_ok = spins < TB_SPIN_LIMIT;
+        if (!s_ok) atomicOr(err, GG_EBIT_SORT_TIMEOUT);
+        __threadfence();
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// node k's record and FP64 mass from its sums
+__device__ __forceinline__ void tb_finish_node(int k, const TreeBuf &tb, const GGPart *__restrict__ parts,
+                                               const GGDomainDev *__restrict__ dom, GGNode *nodes, double M, double sx,
+                                               double sy, double sz, float maxsoft, int a, int b)
+{
+    const int lev = tb.level[k], s = tb.start[k];
+    const GGDomainDev d = dom[tb.sys[k]];
+    // geometric cell: level `lev` cell containing the node's first particle
+    const int gl = lev > GG_MAX_LEVEL ? GG_MAX_LEVEL : lev;
+    const double len = ldexp(d.len, -gl);
+    double cen[3];
+    if (gl == 0) {
+        cen[0] = d.center[0]; cen[1] = d.center[1]; cen[2] = d.center[2];
+    } else {
+        const GGPart p0 = parts[s];
+        const double pv[3] = {p0.x, p0.y, p0.z};
+        for (int q = 0; q < 3; q++) {
+            const unsigned cell = gg_quantize(pv[q], d.corner[q], d.len) >> (GG_MAX_LEVEL - gl);
+            cen[q] = d.corner[q] + ((double)cell + 0.5) * len;
+        }
+    }
+    double cx, cy, cz;
+    if (M > 0) { cx = sx / M; cy = sy / M; cz = sz / M; }
+    else { cx = cen[0]; cy = cen[1]; cz = cen[2]; }
+    GGNode nd;
+    nd.cx = cx; nd.cy = cy; nd.cz = cz;
+    nd.mass = (float)M; nd.len = (float)len; nd.maxsoft = maxsoft;
+    nd.gx = (float)(cen[0] - cx); nd.gy = (float)(cen[1] - cy); nd.gz = (float)(cen[2] - cz);
+    nd.a = a; nd.b = b; nd.level = lev; nd.parent = tb.parent[k];
+    nodes[k] = nd;
+    tb.mass64[k] = M;
+}
+
+// The tree's nodes in one cooperative launch: roots, then one depth after the
+// other.  Every dependence between blocks is a grid barrier (about 1.5 us)
+// instead of a kernel boundary, and the loop stops at the tree's own depth.  One
+// launch per depth and direction made 57 launches, most of them of empty depths
+// in a small tree.  Tree and moments together, B200: 1,000 particles 352 -> 62 us,
+// 65,536 430 -> 171, 16.8M 2.02 -> 1.82 ms (in one launch of both, at 64 registers and
+// half the threads per SM, 2.34 ms).
+//
+// One depth: 8 threads per node find the 7 digit boundaries by binary search
+// (or the chunk split of a full-depth cell) and the child count; a block
+// publishes its children total, adds up the totals of the blocks before it
+// (they publish before they wait on anyone) and writes its nodes' children at
+// contiguous indices from there.  The last block with nodes sets the next
+// depth's range.  A child index at or past the node capacity is not written and
+// sets GG_EBIT_NODE_OVERFLOW (the capacity is sized so that it cannot happen).
+__global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
+    k_tree_nodes(const unsigned long long *__restrict__ keys, const int *__restrict__ poff, int S, TreeBuf tb, int leaf)
+{
+    __shared__ int s_sum, s_off, s_tot;
     __shared__ int s_red[TB_THREADS / 32];
     __shared__ int s_nch[TB_NODES];
     __shared__ int s_excl[TB_NODES];
-    const int lb = tb.depth_beg[depth], le = tb.depth_beg[depth + 1];
-    const int nl = le - lb;
-    const int G = gridDim.x;
-    if (threadIdx.x == 0) {
-        s_ticket = (int)atomicAdd(tb.ticket + depth, 1u);
-        s_sum = 0;
-    }
-    __syncthreads();
-    const int blk = s_ticket;
-    if (nl == 0) {   // nothing at this depth: the next one is empty too
-        if (blk == G - 1 && threadIdx.x == 0) {
-            tb.depth_beg[depth + 2] = le;
-            tb.nnodes[0] = le;
-        }
-        return;
-    }
-    const int chunk = (nl + G - 1) / G;
-    const int cb = lb + blk * chunk, ce = min(le, cb + chunk);
-    const int g = threadIdx.x / TB_GROUP, j = threadIdx.x % TB_GROUP;
-    const int gbase = (threadIdx.x & 31) & ~(TB_GROUP - 1);
+    const int G = gridDim.x, blk = blockIdx.x, tid = threadIdx.x;
+    const int gtid = blk * TB_THREADS + tid, gthreads = G * TB_THREADS;
+    unsigned target = 0;
 
-    // ---- count
-    int my = 0;
-    for (int base = cb; base < ce; base += TB_NODES) {
-        const int k = base + g;
-        const bool valid = k < ce;
-        int s = 0, e = 0, lev = 0;
-        if (valid) { s = tb.start[k]; e = tb.end[k]; lev = tb.level[k]; }
-        const int cnt = e - s;
-        const bool split = valid && cnt > leaf && depth < GG_MAX_DEPTH - 1;
-        const bool digit_mode = split && lev < GG_MAX_LEVEL;
-        const bool chunk_mode = split && lev >= GG_MAX_LEVEL;
-        int b = s;
-        if (digit_mode && j > 0) {
-            int shift = 3 * (GG_MAX_LEVEL - (lev + 1));
-            unsigned long long prefix = keys[s] >> (shift + 3);
-            b = lower_bound_key(keys, s, e, ((prefix << 3) | (unsigned long long)j) << shift);
-        }
-        if (digit_mode) tb.bnd[(size_t)k * 8 + j] = b;
-        const int nb = __shfl_down_sync(0xffffffffu, b, 1, TB_GROUP);
-        const int bn = (j < 7) ? nb : e;
-        const unsigned m = __ballot_sync(0xffffffffu, digit_mode && bn > b);
-        int nch = 0;
-        if (digit_mode) nch = __popc((m >> gbase) & 0xFFu);
-        else if (chunk_mode) nch = chunk_children(cnt, leaf);
-        if (valid && j == 0) {
-            tb.nch[k] = nch;
-            tb.child[k] = -1;
-            my += nch;
-        }
+    // roots: one per system, geometric level 0 (the domain cube), depth 0
+    for (int s = gtid; s < S; s += gthreads) {
+        tb.start[s] = poff[s];
+        tb.end[s] = poff[s + 1];
+        tb.level[s] = 0;
+        tb.parent[s] = -1;
+        tb.sys[s] = s;
     }
-    if (my) atomicAdd(&s_sum, my);
-    __syncthreads();
-    if (threadIdx.x == 0) tb_st_status(tb.bstat + (size_t)depth * G + blk, TB_PUBLISHED | (unsigned)s_sum);
+    if (gtid == 0) {
+        tb.depth_beg[0] = 0;
+        tb.depth_beg[1] = S;
+    }
+    if (!tb_grid_barrier(tb.barrier, target, tb.err)) return;
 
-    // ---- this block's first child index: the totals of the blocks before it
-    int before = 0;
-    for (int i = threadIdx.x; i < blk; i += TB_THREADS) {
-        const unsigned *w = tb.bstat + (size_t)depth * G + i;
-        unsigned v = tb_ld_status(w);
-        int spins = 0;
-        while (!(v & TB_PUBLISHED)) {
-            if (++spins > TB_SPIN_LIMIT) {
-                atomicOr(tb.err, GG_EBIT_SORT_TIMEOUT);
-                break;
-            }
-            __nanosleep(64);
-            v = tb_ld_status(w);
-        }
-        before += (int)(v & ~TB_PUBLISHED);
-    }
-    before = __reduce_add_sync(0xffffffffu, before);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = before;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int off = 0;
-        for (int w = 0; w < TB_THREADS / 32; w++) off += s_red[w];
-        s_off = off;
-        if (blk == G - 1) {   // the last chunk: the depth's total is known
-            long long nxt = (long long)le + off + s_sum;
-            if (nxt > tb.cap) {
-                atomicOr(tb.err, GG_EBIT_NODE_OVERFLOW);
-                nxt = tb.cap;
-            }
-            tb.depth_beg[depth + 2] = (int)nxt;
-            tb.nnodes[0] = (int)nxt;
-        }
-    }
-    __syncthreads();   // also orders this block's count-phase stores before the reads below
-    if (s_sum == 0) return;
+    int lb = 0, le = S, depth = 0;
+    const int g = tid / TB_GROUP, j = tid % TB_GROUP;
+    const int gbase = (tid & 31) & ~(TB_GROUP - 1);
+    for (;; depth++) {   // depths 0 .. GG_MAX_DEPTH - 1; the last is all leaves
+        const int nl = le - lb;
+        const int chunk = max((nl + G - 1) / G, TB_NODES);   // nodes per block: whole passes of the block
+        const int cb = lb + blk * chunk, ce = min(le, cb + chunk);
+        if (cb < le) {
+            const bool one = chunk <= TB_NODES;   // one node per 8 threads: boundaries stay in registers
+            if (tid == 0) s_sum = 0;
+            __syncthreads();
 
-    // ---- write
-    int run = le + s_off;
-    for (int base = cb; base < ce; base += TB_NODES) {
-        int k = base + g;
-        bool valid = k < ce;
-        if (j == 0) s_nch[g] = valid ? tb.nch[k] : 0;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            int v = threadIdx.x < TB_NODES ? s_nch[threadIdx.x] : 0, x = v;
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(0xffffffffu, x, o);
-                if ((int)threadIdx.x >= o) x += y;
+            // ---- count
+            int my = 0, s = 0, e = 0, lev = 0, b = 0, bn = 0, nch = 0;
+            for (int base = cb; base < ce; base += TB_NODES) {
+                const int k = base + g;
+                const bool valid = k < ce;
+                s = e = lev = 0;
+                if (valid) { s = tb.start[k]; e = tb.end[k]; lev = tb.level[k]; }
+                const int cnt = e - s;
+                const bool split = valid && cnt > leaf && depth < GG_MAX_DEPTH - 1;
+                const bool digit_mode = split && lev < GG_MAX_LEVEL;
+                const bool chunk_mode = split && lev >= GG_MAX_LEVEL;
+                b = s;
+                if (digit_mode && j > 0) {
+                    const int shift = 3 * (GG_MAX_LEVEL - (lev + 1));
+                    const unsigned long long prefix = keys[s] >> (shift + 3);
+                    b = lower_bound_key(keys, s, e, ((prefix << 3) | (unsigned long long)j) << shift);
+                }
+                if (digit_mode && !one) tb.bnd[(size_t)k * 8 + j] = b;
+                const int nb = __shfl_down_sync(0xffffffffu, b, 1, TB_GROUP);
+                bn = (j < 7) ? nb : e;
+                const unsigned m = __ballot_sync(0xffffffffu, digit_mode && bn > b);
+                nch = 0;
+                if (digit_mode) nch = __popc((m >> gbase) & 0xFFu);
+                else if (chunk_mode) nch = chunk_children(cnt, leaf);
+                if (valid && j == 0) {
+                    tb.nch[k] = nch;
+                    if (!nch) tb.child[k] = -1;
+                    my += nch;
+                }
             }
-            if (threadIdx.x < TB_NODES) s_excl[threadIdx.x] = x - v;
-            if (threadIdx.x == 31) s_tot = x;
-        }
-        __syncthreads();
-        if (valid) {
-            int nch = s_nch[g];
-            int first = run + s_excl[g];
-            if (j == 0) tb.child[k] = nch ? first : -1;
-            if (nch) {
-                int s = tb.start[k], e = tb.end[k], lev = tb.level[k], sys = tb.sys[k];
-                if (lev >= GG_MAX_LEVEL) {
-                    const int csz = chunk_size(e - s, leaf);
-                    for (int c = j; c < nch; c += TB_GROUP) {
-                        int idx = first + c;
-                        if (idx >= tb.cap) { atomicOr(tb.err, GG_EBIT_NODE_OVERFLOW); continue; }
-                        int cs = s + c * csz, ce2 = min(e, cs + csz);
-                        tb.start[idx] = cs; tb.end[idx] = ce2; tb.level[idx] = GG_CHUNK_LEVEL;
-                        tb.parent[idx] = k; tb.sys[idx] = sys;
+            if (my) atomicAdd(&s_sum, my);
+            __syncthreads();
+            unsigned *const bstat = tb.bstat + (size_t)depth * G;
+            if (tid == 0) tb_st_status(bstat + blk, TB_PUBLISHED | (unsigned)s_sum);
+
+            // ---- this block's first child index: the totals of the blocks before it
+            int before = 0;
+            for (int i = tid; i < blk; i += TB_THREADS) {
+                unsigned v = tb_ld_status(bstat + i);
+                int spins = 0;
+                while (!(v & TB_PUBLISHED)) {
+                    if (++spins > TB_SPIN_LIMIT) {
+                        atomicOr(tb.err, GG_EBIT_SORT_TIMEOUT);
+                        break;
                     }
-                } else {
-                    int b = tb.bnd[(size_t)k * 8 + j];
-                    int bn = (j < 7) ? tb.bnd[(size_t)k * 8 + j + 1] : e;
-                    int rank = 0;
-                    for (int jj = 0; jj < j; jj++) {
-                        int b0 = tb.bnd[(size_t)k * 8 + jj];
-                        int b1 = (jj < 7) ? tb.bnd[(size_t)k * 8 + jj + 1] : e;
-                        rank += b1 > b0;
+                    __nanosleep(20);
+                    v = tb_ld_status(bstat + i);
+                }
+                before += (int)(v & ~TB_PUBLISHED);
+            }
+            before = __reduce_add_sync(0xffffffffu, before);
+            if ((tid & 31) == 0) s_red[tid >> 5] = before;
+            __syncthreads();
+            if (tid == 0) {
+                int off = 0;
+                for (int w = 0; w < TB_THREADS / 32; w++) off += s_red[w];
+                s_off = off;
+                if (ce == le) {   // the last block with nodes: the depth's total is known
+                    long long nxt = (long long)le + off + s_sum;
+                    if (nxt > tb.cap) {
+                        atomicOr(tb.err, GG_EBIT_NODE_OVERFLOW);
+                        nxt = tb.cap;
                     }
-                    if (bn > b) {
-                        int idx = first + rank;
-                        if (idx >= tb.cap) {
-                            atomicOr(tb.err, GG_EBIT_NODE_OVERFLOW);
+                    tb.depth_beg[depth + 2] = (int)nxt;
+                    tb.nnodes[0] = (int)nxt;
+                }
+            }
+            __syncthreads();   // also orders this block's count-phase stores before the reads below
+
+            // ---- write
+            int run = le + s_off;
+            if (s_sum != 0) {
+                for (int base = cb; base < ce; base += TB_NODES) {
+                    const int k = base + g;
+                    const bool valid = k < ce;
+                    if (!one && valid) {
+                        s = tb.start[k];
+                        e = tb.end[k];
+                        lev = tb.level[k];
+                        nch = tb.nch[k];
+                    }
+                    if (j == 0) s_nch[g] = valid ? nch : 0;
+                    __syncthreads();
+                    if (tid < 32) {   // exclusive prefix of the TB_NODES = 64 counts, two per lane
+                        const int v0 = s_nch[2 * tid], v1 = s_nch[2 * tid + 1];
+                        int x = v0 + v1;
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int y = __shfl_up_sync(0xffffffffu, x, o);
+                            if (tid >= o) x += y;
+                        }
+                        s_excl[2 * tid] = x - v0 - v1;
+                        s_excl[2 * tid + 1] = x - v1;
+                        if (tid == 31) s_tot = x;
+                    }
+                    __syncthreads();
+                    if (valid && nch) {
+                        const int first = run + s_excl[g], sys = tb.sys[k];
+                        if (j == 0) tb.child[k] = first;
+                        if (lev >= GG_MAX_LEVEL) {
+                            const int csz = chunk_size(e - s, leaf);
+                            for (int c = j; c < nch; c += TB_GROUP) {
+                                const int idx = first + c;
+                                if (idx >= tb.cap) { atomicOr(tb.err, GG_EBIT_NODE_OVERFLOW); continue; }
+                                const int cs = s + c * csz, ce2 = min(e, cs + csz);
+                                tb.start[idx] = cs; tb.end[idx] = ce2; tb.level[idx] = GG_CHUNK_LEVEL;
+                                tb.parent[idx] = k; tb.sys[idx] = sys;
+                            }
                         } else {
-                            tb.start[idx] = b; tb.end[idx] = bn;
-                            tb.level[idx] = common_level(keys[b], keys[bn - 1]);
-                            tb.parent[idx] = k; tb.sys[idx] = sys;
+                            if (!one) {
+                                b = tb.bnd[(size_t)k * 8 + j];
+                                bn = (j < 7) ? tb.bnd[(size_t)k * 8 + j + 1] : e;
+                            }
+                            const unsigned gm = 0xFFu << gbase;
+                            const unsigned m = __ballot_sync(gm, bn > b);   // the node's 8 threads
+                            if (bn > b) {
+                                const int idx = first + __popc(m & gm & ((1u << (tid & 31)) - 1u));
+                                if (idx >= tb.cap) {
+                                    atomicOr(tb.err, GG_EBIT_NODE_OVERFLOW);
+                                } else {
+                                    tb.start[idx] = b; tb.end[idx] = bn;
+                                    tb.level[idx] = common_level(keys[b], keys[bn - 1]);
+                                    tb.parent[idx] = k; tb.sys[idx] = sys;
+                                }
+                            }
                         }
                     }
+                    const int tot = s_tot;
+                    __syncthreads();
+                    run += tot;
                 }
             }
         }
-        int tot = s_tot;
-        __syncthreads();
-        run += tot;
+        if (!tb_grid_barrier(tb.barrier, target, tb.err)) return;
+        lb = le;
+        le = __ldcg(tb.depth_beg + depth + 2);
+        if (le <= lb || depth + 1 >= GG_MAX_DEPTH) break;   // no nodes at the next depth
     }
+    if (gtid == 0) tb.nnodes[1] = depth;   // the deepest depth: all leaves
 }
 
-// Bottom-up moments, one depth per launch from the deepest up: a leaf sums its
-// particles, an internal node its children (one depth deeper, computed by the
-// previous launch), each in index order in FP64.  Nodes are numbered depth by
-// depth with the children of consecutive nodes consecutive, so the lanes of a
-// warp read one contiguous stretch of child records (or of particles).
-__global__ void k_tree_moments_depth(int depth, const GGPart *__restrict__ parts,
-                                     const GGDomainDev *__restrict__ dom, TreeBuf tb, GGNode *__restrict__ nodes)
+// Moments, in one cooperative launch: every leaf sums its particles, then one
+// depth after the other from the deepest up, an internal node sums its
+// children, each in index order in FP64.  Nodes are numbered depth by depth
+// with the children of consecutive nodes consecutive, so the lanes of a warp
+// read one contiguous stretch of child records (or of particles).
+__global__ void __launch_bounds__(TB_THREADS, TB_MOM_PER_SM)
+    k_tree_moments(TreeBuf tb, const GGPart *__restrict__ parts, const GGDomainDev *__restrict__ dom, GGNode *nodes)
 {
-    const int lb = tb.depth_beg[depth], le = tb.depth_beg[depth + 1];
-    for (int k = lb + blockIdx.x * blockDim.x + threadIdx.x; k < le; k += gridDim.x * blockDim.x) {
-        const int lev = tb.level[k], sys = tb.sys[k];
-        const GGDomainDev d = dom[sys];
+    const int gtid = blockIdx.x * TB_THREADS + threadIdx.x, gthreads = gridDim.x * TB_THREADS;
+    // (clamped: the node kernel leaves them unset when a wait of its own gave up)
+    const int total = min(tb.nnodes[0], tb.cap), depth = min(max(tb.nnodes[1], 0), GG_MAX_DEPTH - 1);
+    unsigned target = 0;
+    for (int k = gtid; k < total; k += gthreads) {
+        if (tb.child[k] >= 0) continue;
         double M = 0, sx = 0, sy = 0, sz = 0;
         float maxsoft = 0;
-        int a, b;
-        const int s = tb.start[k];
-        const int c0 = tb.child[k];
-        if (c0 < 0) {   // leaf: its particles
-            const int e = tb.end[k];
-            for (int i = s; i < e; i++) {
-                const GGPart p = parts[i];
-                const double m = (double)p.m;
-                M += m;
-                sx += m * p.x; sy += m * p.y; sz += m * p.z;
-                maxsoft = fmaxf(maxsoft, p.h);
-            }
-            a = s;
-            b = -(e - s);
-        } else {        // internal: its children
+        const int s = tb.start[k], e = tb.end[k];
+        for (int i = s; i < e; i++) {
+            const GGPart p = parts[i];
+            const double m = (double)p.m;
+            M += m;
+            sx += m * p.x; sy += m * p.y; sz += m * p.z;
+            maxsoft = fmaxf(maxsoft, p.h);
+        }
+        tb_finish_node(k, tb, parts, dom, nodes, M, sx, sy, sz, maxsoft, s, -(e - s));
+    }
+    // internal nodes, deepest first
+    for (int d = depth - 1; d >= 0; d--) {
+        if (!tb_grid_barrier(tb.barrier + 1, target, tb.err)) return;
+        const int db = __ldcg(tb.depth_beg + d), de = __ldcg(tb.depth_beg + d + 1);
+        for (int k = db + gtid; k < de; k += gthreads) {
+            const int c0 = tb.child[k];
+            if (c0 < 0) continue;
+            double M = 0, sx = 0, sy = 0, sz = 0;
+            float maxsoft = 0;
             const int nc = tb.nch[k];
-            for (int c = c0; c < c0 + nc; c++) {
-                const double m = tb.mass64[c];
+            for (int c = c0; c < c0 + nc; c++) {   // written by other blocks of this launch: read through L2
+                const double m = __ldcg(tb.mass64 + c);
+                const double2 xy = __ldcg(reinterpret_cast<const double2 *>(&nodes[c].cx));
+                const double z = __ldcg(&nodes[c].cz);
                 M += m;
-                sx += m * nodes[c].cx;
-                sy += m * nodes[c].cy;
-                sz += m * nodes[c].cz;
-                maxsoft = fmaxf(maxsoft, nodes[c].maxsoft);
+                sx += m * xy.x; sy += m * xy.y; sz += m * z;
+                maxsoft = fmaxf(maxsoft, __ldcg(&nodes[c].maxsoft));
             }
-            a = c0;
-            b = nc;
+            tb_finish_node(k, tb, parts, dom, nodes, M, sx, sy, sz, maxsoft, c0, nc);
         }
-        // geometric cell: level `lev` cell containing the node's first particle
-        const int gl = lev > GG_MAX_LEVEL ? GG_MAX_LEVEL : lev;
-        const double len = ldexp(d.len, -gl);
-        double cen[3];
-        if (gl == 0) {
-            cen[0] = d.center[0]; cen[1] = d.center[1]; cen[2] = d.center[2];
-        } else {
-            const GGPart p0 = parts[s];
-            const double pv[3] = {p0.x, p0.y, p0.z};
-            for (int q = 0; q < 3; q++) {
-                const unsigned cell = gg_quantize(pv[q], d.corner[q], d.len) >> (GG_MAX_LEVEL - gl);
-                cen[q] = d.corner[q] + ((double)cell + 0.5) * len;
-            }
-        }
-        double cx, cy, cz;
-        if (M > 0) { cx = sx / M; cy = sy / M; cz = sz / M; }
-        else { cx = cen[0]; cy = cen[1]; cz = cen[2]; }
-        GGNode nd;
-        nd.cx = cx; nd.cy = cy; nd.cz = cz;
-        nd.mass = (float)M; nd.len = (float)len; nd.maxsoft = maxsoft;
-        nd.gx = (float)(cen[0] - cx); nd.gy = (float)(cen[1] - cy); nd.gz = (float)(cen[2] - cz);
-        nd.a = a; nd.b = b; nd.level = lev; nd.parent = tb.parent[k];
-        nodes[k] = nd;
-        tb.mass64[k] = M;
     }
 }
 
@@ -351,21 +400,25 @@ void gg_launch_permute(const unsigned *perm, const GGPart *in, GGPart *out, unsi
     gg_note_launches(1);
 }
 
-// blocks of the per-depth count and write kernels: 8 per SM keeps enough binary
-// searches in flight to hide their dependent loads
-int gg_tree_grid() { return gg_num_sms() * 8; }
+// blocks of the node kernel at most (its look-back words are sized for them)
+int gg_tree_grid() { return gg_num_sms() * TB_PER_SM; }
 
-void gg_launch_tree(const unsigned long long *keys, const int *poff, int S, int leaf, int cap, TreeBuf tb,
-                    const GGPart *parts, const GGDomainDev *dom, GGNode *nodes, cudaStream_t st)
+gg_status gg_launch_tree(const unsigned long long *keys, const int *poff, int S, int n, int leaf, int cap, TreeBuf tb,
+                         const GGPart *parts, const GGDomainDev *dom, GGNode *nodes, cudaStream_t st)
 {
-    const int G = gg_tree_grid();
-    k_tree_roots<<<(S + 127) / 128, 128, 0, st>>>(S, poff, tb);
+    // about 1,024 particles per block: few blocks for a small tree, as a barrier
+    // of one block costs nothing (1,000 particles: 53 us in one block, 76 us in
+    // two; 65,536: 165 us in 64 blocks, 192 us in 16)
+    const long long want = ((long long)n + S + 1023) / 1024;
+    const int G = (int)std::min((long long)gg_tree_grid(), want);
+    const int Gm = (int)std::min((long long)gg_num_sms() * TB_MOM_PER_SM, want);
     tb.cap = cap;
-    cudaMemsetAsync(tb.ticket, 0, GG_MAX_DEPTH * sizeof(unsigned), st);
-    cudaMemsetAsync(tb.bstat, 0, (size_t)GG_MAX_DEPTH * G * sizeof(unsigned), st);
-    for (int depth = 0; depth < GG_MAX_DEPTH; depth++) k_tree_depth<<<G, TB_THREADS, 0, st>>>(depth, keys, tb, leaf);
-    const int threads = 256, blocks = gg_num_sms() * 8;
-    for (int depth = GG_MAX_DEPTH - 1; depth >= 0; depth--)
-        k_tree_moments_depth<<<blocks, threads, 0, st>>>(depth, parts, dom, tb, nodes);
-    gg_note_launches(1 + 2 * GG_MAX_DEPTH);
+    GG_CUDA_TRY(cudaMemsetAsync(tb.bstat, 0, ((size_t)GG_MAX_DEPTH * G + 2) * sizeof(unsigned), st));
+    tb.barrier = tb.bstat + (size_t)GG_MAX_DEPTH * G;
+    void *args[] = {&keys, &poff, &S, &tb, &leaf};
+    GG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_tree_nodes, dim3(G), dim3(TB_THREADS), args, 0, st));
+    void *margs[] = {&tb, &parts, &dom, &nodes};
+    GG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_tree_moments, dim3(Gm), dim3(TB_THREADS), margs, 0, st));
+    gg_note_launches(2);
+    return GG_OK;
 }

@@ -10,9 +10,9 @@ struct TreeBuf {
     int *bnd;          // 8 digit boundaries per node
     double *mass64;    // FP64 node mass (parent sums)
     int *depth_beg;    // GG_MAX_DEPTH + 2 entries
-    int *nnodes;       // total nodes (device)
-    unsigned *bstat;   // per depth and block: published children totals (GG_MAX_DEPTH x grid)
-    unsigned *ticket;  // per depth: block tickets
+    int *nnodes;       // total nodes, deepest depth (device)
+    unsigned *bstat;   // per depth and block: published children totals (GG_MAX_DEPTH x grid), then two barrier words
+    unsigned *barrier; // set by gg_launch_tree
     int cap;           // node capacity (set by gg_launch_tree)
     int *err;
 };
@@ -41,8 +41,8 @@ gg_status gg_sort_pairs_run(unsigned long long *keys, unsigned *vals, long long 
 
 void gg_launch_permute(const unsigned *perm, const GGPart *in, GGPart *out, unsigned *rank, int n, cudaStream_t st);
 int gg_tree_grid();
-void gg_launch_tree(const unsigned long long *keys, const int *poff, int S, int leaf, int cap, TreeBuf tb,
-                    const GGPart *parts, const GGDomainDev *dom, GGNode *nodes, cudaStream_t st);
+gg_status gg_launch_tree(const unsigned long long *keys, const int *poff, int S, int n, int leaf, int cap, TreeBuf tb,
+                         const GGPart *parts, const GGDomainDev *dom, GGNode *nodes, cudaStream_t st);
 
 struct WalkParams {
     const GGNode *nodes;

@@ -1,0 +1,51 @@
+"""The tree kernels at the sizes where their work split changes: one block or
+several, whole and partial blocks of nodes, chunked full-depth cells, empty
+systems.  A walk that opens every node must meet each particle exactly once; a
+Barnes-Hut walk with a huge opening angle must see each system's own total
+mass at its centre of mass."""
+import numpy as np
+import pytest
+
+import ggb200
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(n, seed, duplicates):
+    rng = np.random.default_rng(seed)
+    pos = rng.normal(size=(n, 3))
+    if duplicates and n > 3:
+        pos[1: n // 2] = pos[n // 2]      # one full-depth cell, split into chunks
+    pos[:1] = [100.0, 1.0, -2.0]          # the far target
+    mass = rng.uniform(0.5, 1.5, n).astype(np.float32).astype(np.float64)
+    return pos, mass, np.full(n, 1e-3)
+
+
+@pytest.mark.parametrize("duplicates", [False, True])
+@pytest.mark.parametrize("sizes", [[1], [2], [8], [9], [63, 65], [1023], [1024], [1025], [5, 0, 700, 3000], [2049],
+                                   [33000]])
+def test_every_particle_is_in_the_tree_once(sizes, duplicates):
+    parts = [_system(n, 10 + i, duplicates) for i, n in enumerate(sizes)]
+    pos, mass, h = (np.concatenate([p[k] for p in parts]) for k in range(3))
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    with ggb200.GravityTree() as t:
+        t.load(pos, mass, h, counts=sizes)
+        t.build()
+        _, _, nint, st = t.evaluate(old_acc=np.zeros(len(mass)), err_tol_force_acc=0.001, want_ninter=True)
+        assert st["error_word"] == 0
+        first = np.array([off[i] for i, n in enumerate(sizes) if n > 8], dtype=np.int32)
+        mono = t.evaluate(active=first, err_tol_theta=1e9)[0] if len(first) else []
+    for s, n in enumerate(sizes):
+        # pairs at r = 0 are not counted: the particle itself and its duplicates
+        same = np.ones(n)
+        if duplicates and n > 3:
+            same[1: n // 2 + 1] = n // 2
+        assert np.array_equal(nint[off[s]:off[s + 1]], n - same)
+    # a root of more than one leaf bucket is used whole at this opening angle
+    for got, a in zip(mono, first):
+        b = off[np.searchsorted(off, a, side="right")]
+        com = (mass[a:b, None] * pos[a:b]).sum(0) / mass[a:b].sum()
+        d = com - pos[a]
+        want = mass[a:b].sum() * d / np.linalg.norm(d) ** 3
+        # FP32 offset, 1/r and mass: a few roundings of 6e-8
+        assert np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(want)
