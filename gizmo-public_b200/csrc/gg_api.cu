@@ -804,9 +804,8 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
     p.gorder = gorder;
     p.node_staging = c->cfg.node_staging;
     p.cost_out = c->cfg.group_order ? c->tcost.p : nullptr;
-    int tpl = c->cfg.group_size > 32 ? 2 : 1;
     if (c->cfg.timing) cudaEventRecord(c->ev[4], s);
-    gg_launch_walk(p, tpl, c->walk_blocks, s);
+    gg_launch_walk(p, c->walk_blocks, s);
     if (c->cfg.timing) cudaEventRecord(c->ev[5], s);
     if (!pot_only) c->oldacc_valid = true;
     if (c->cfg.group_order) c->tcost_valid = true;

@@ -70,8 +70,7 @@ struct WalkParams {
     float *cost_out;            // per particle (load order): its group's cycles per target, may be NULL
     int node_staging;           // 0: per-lane cp.async, 1: bulk copies (TMA) per run of consecutive nodes
 };
-int gg_walk_smem_bytes(int flush, int tpl);
-void gg_launch_walk(const WalkParams &p, int tpl, int blocks_per_sm, cudaStream_t st);
+void gg_launch_walk(const WalkParams &p, int blocks_per_sm, cudaStream_t st);
 int gg_walk_threads();
 
 // groups of `gs` consecutive targets per system; toff[S+1] target offsets per system

@@ -1,7 +1,7 @@
 // gg_walk.cu -- warp-cooperative tree walk (force_treeevaluate, forcetree.c:1633-2807).
 //
-// A warp serves one group of up to 32*TPL targets that are consecutive in
-// Peano-Hilbert order (TPL targets per lane).  The warp walks the tree once
+// A warp serves one group of up to 64 targets that are consecutive in
+// Peano-Hilbert order (two targets per lane; see Targets).  The warp walks the tree once
 // for the whole group with an explicit node stack: each round pops up to 32
 // nodes, one per lane, and tests them against the group's bounding box with
 // the reference's opening rules made conservative over the group
@@ -36,11 +36,13 @@
 //     runs of consecutive records on an mbarrier);
 //   - stack pushes use prefix counts from bit ballots; the particles of opened
 //     leaves go through a per-warp queue and are classified 32 at a time;
-//   - the lists are pair-interleaved and evaluated two entries per packed
+//   - the lists are one array per component, evaluated two entries per packed
 //     FP32x2 instruction;
 //   - the persistent warps take groups in the order the host side planned
 //     (most expensive first, from the previous walk's measured cost), and each
 //     group records its own cost for the next walk.
+#include <climits>
+
 #include "gg_internal.cuh"
 #include "gg_kernels.cuh"
 
@@ -50,29 +52,36 @@
 
 int gg_walk_threads() { return WALK_THREADS; }
 
-// Per-warp shared memory, in float4 units:
-//   far list float4[cap] | near list float4[cap] | near softening float4[cap] |
-//   node stack int[WALK_SSTACK] | node slots GGNode[32] | particle queue int[PQ_CAP] |
+// Per-warp shared memory, in floats:
+//   far list [FAR_ARRAYS][FAR_CAP] | near list [NEAR_ARRAYS][NEAR_CAP] | node stack int[WALK_SSTACK] |
+//   node slots GGNode[32 NH] | runs of a window int[32] | queued runs int[2][RUNS] |
 //   mbarrier of the node copies (16 bytes)
-// with cap = list_cap(flush) entries of 4 floats.  The stack spills to the warp's global stack area
-// when it overflows (deep or wide traversals only).
+// The stack spills to the warp's global stack area when it overflows (deep or
+// wide traversals only).
 #define WALK_SSTACK 512
-// particle queue: indices of the particles of opened leaves, evaluated 32 at a time
-#define PQ_CAP 224
-// list capacity in entries: a flush threshold plus one ballot's worth, even
-// (the lists are stored in pairs)
-__host__ __device__ __forceinline__ int list_cap(int flush) { return (flush + 33) & ~1; }
-__host__ __device__ __forceinline__ int walk_warp_float4s(int flush)
-{
-    const int cap = list_cap(flush);
-    return 3 * cap + WALK_SSTACK / 4 + 32 * 4 + PQ_CAP / 4 + 1;
-}
-
-int gg_walk_smem_bytes(int flush, int tpl)
-{
-    (void)tpl;
-    return WALK_WARPS * walk_warp_float4s(flush) * 16;
-}
+// Queue of the runs of particles of opened leaves (a ring): its particles are
+// taken 32 at a time.  Fewer than 32 particles, so at most 31 runs, wait when a
+// round adds its own (up to 32 NH).
+#define RUNS 128
+// The lists are arrays of one component each ({x, y, z, m}; near: {x, y, z} and
+// a softening record of three): lanes append to consecutive words, and a
+// flush loads two or four consecutive entries of a component at once.
+#define FAR_ARRAYS 4
+#define NEAR_ARRAYS 6
+// Nodes per lane and round: with two, the round's fixed part (loop, scan,
+// windows) is paid once for 64 nodes.  Per 1M clustered walk, groups of 32:
+// 2.15e9 -> 2.00e9 warp instructions, 3.07 -> 2.88 ms.
+#define NH 2
+// A list is evaluated when it holds this many entries (or the configured
+// threshold, if smaller).  Between two looks at the thresholds a round appends
+// up to 32 NH nodes and a batch of 32 particles.  Longer lists would save some of
+// the flushes' fixed part; two blocks' shared memory is all there is.
+#define FAR_FLUSH_MAX 96
+#define NEAR_FLUSH_MAX 64
+#define FAR_CAP (FAR_FLUSH_MAX + 32 * NH + 32)
+#define NEAR_CAP (NEAR_FLUSH_MAX + 32 * NH + 32)
+#define WALK_WARP_FLOATS \
+    (FAR_ARRAYS * FAR_CAP + NEAR_ARRAYS * NEAR_CAP + WALK_SSTACK + NH * 32 * 16 + 32 + 2 * RUNS + 4)
 
 // ---- staging of node records
 // The next round's node records are copied into shared memory, one 64-byte slot
@@ -84,13 +93,26 @@ int gg_walk_smem_bytes(int flush, int tpl)
 //     L1, where the top levels of the tree, which every group visits, hit);
 //  1: the bulk-copy (TMA) engine, one copy per run of consecutive records.
 // (Staging two rounds ahead, in two slots, measured no faster.)
-__device__ __forceinline__ void stage_node(int4 *slot, const GGNode *src)
+// Slots are 64 bytes apart, so the lanes' i-th 16-byte pieces would meet in two
+// of the eight 16-byte bank groups: piece i of slot l lies at piece
+// i ^ ((l >> 1) & 3), which spreads every eight lanes over all banks.  (A bulk
+// copy writes records as they are.  Four lanes per record, which looks up each
+// cache line once instead of four times, measured no faster: the walk is bound by
+// instruction issue, and the lanes then have to exchange their node indices.)
+__device__ __forceinline__ void stage_lanes(unsigned slot0, const GGNode *nodes, const int (&node)[NH], int k, int lane)
 {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(slot);
-    const int4 *s = reinterpret_cast<const int4 *>(src);
+    const int swz = (lane >> 1) & 3;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d + 16 * i), "l"(s + i) : "memory");
+    for (int h = 0; h < NH; h++)
+        if (32 * h + lane < k) {
+            const int4 *src = reinterpret_cast<const int4 *>(nodes + node[h]);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(slot0 + 64u * (32 * h + lane) +
+                                                                              16u * (i ^ swz)),
+                             "l"(src + i)
+                             : "memory");
+        }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
@@ -104,23 +126,28 @@ __device__ __forceinline__ void stage_node(int4 *slot, const GGNode *src)
 // its copies and leaves the kernel.
 #define WALK_WAIT_LIMIT (1 << 20)
 
-__device__ __forceinline__ void stage_nodes(unsigned bar, unsigned slot0, const GGNode *nodes, int node, int k,
-                                            int lane)
+__device__ __forceinline__ void stage_nodes(unsigned bar, unsigned slot0, const GGNode *nodes, const int (&node)[NH],
+                                            int k, int lane)
 {
-    const int prev = __shfl_up_sync(FULL, node, 1);
-    const bool start = lane < k && (lane == 0 || node != prev + 1);
-    const unsigned starts = __ballot_sync(FULL, start);
     // the slots were read by this round's tests, whose values were consumed
-    // before the pop above (warp-synchronous): the copies may overwrite them
+    // before the next nodes were known (warp-synchronous): the copies may overwrite them
     if (lane == 0)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(k * 64) : "memory");
     __syncwarp();
-    if (start) {
-        const unsigned later = starts & ~((2u << lane) - 1u);   // run starts after this lane
-        const int end = later ? __ffs(later) - 1 : k;
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(slot0 + 64u * lane), "l"(nodes + node), "r"(64u * (end - lane)), "r"(bar)
-                     : "memory");
+#pragma unroll
+    for (int h = 0; h < NH; h++) {
+        const int kh = min(k - 32 * h, 32);   // nodes of this part
+        if (kh <= 0) break;
+        const int prev = __shfl_up_sync(FULL, node[h], 1);
+        const bool start = lane < kh && (lane == 0 || node[h] != prev + 1);
+        const unsigned starts = __ballot_sync(FULL, start);
+        if (start) {
+            const unsigned later = starts & ~((2u << lane) - 1u);   // run starts after this lane
+            const int end = later ? __ffs(later) - 1 : kh;
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(slot0 + 64u * (32 * h + lane)), "l"(nodes + node[h]), "r"(64u * (end - lane)), "r"(bar)
+                         : "memory");
+        }
     }
 }
 
@@ -140,13 +167,14 @@ __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity)
     return false;
 }
 
+// a particle record in one 256-bit load
 __device__ __forceinline__ GGPart load_part(const GGPart *p)
 {
     GGPart r;
-    const int4 *src = reinterpret_cast<const int4 *>(p);
-    int4 *dst = reinterpret_cast<int4 *>(&r);
-    dst[0] = __ldg(src);
-    dst[1] = __ldg(src + 1);
+    double mh;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(mh) : "l"(p));
+    r.m = __int_as_float(__double2loint(mh));
+    r.h = __int_as_float(__double2hiint(mh));
     return r;
 }
 
@@ -181,21 +209,28 @@ __device__ __forceinline__ float2 sel2(bool px, bool py, float2 a, float2 b)
     return make_float2(px ? a.x : b.x, py ? a.y : b.y);
 }
 
-// Interaction lists are stored pair-interleaved: entries 2p and 2p+1 occupy
-// the eight floats {x0, x1, y0, y1, z0, z1, w0, w1} (w: mass), so that one
-// 128-bit shared-memory load gives the register pairs the packed instructions
-// take.  The softening records of the near list use the same layout.
+// component arrays of a list: entry j
 __device__ __forceinline__ void list_put(float *list, int j, float4 v)
 {
-    float *b = list + ((j >> 1) << 3) + (j & 1);
-    b[0] = v.x;
-    b[2] = v.y;
-    b[4] = v.z;
-    b[6] = v.w;
+    list[j] = v.x;
+    list[FAR_CAP + j] = v.y;
+    list[2 * FAR_CAP + j] = v.z;
+    list[3 * FAR_CAP + j] = v.w;
 }
-// A list of odd length is evaluated with one more entry: massless and 1e18 away
-// (its r^2 is finite and its terms are exactly zero).  The lists have room.
+// near entry j: position, and its softening record (see near_soft)
+__device__ __forceinline__ void near_put(float *list, int j, float4 v, float4 soft)
+{
+    list[j] = v.x;
+    list[NEAR_CAP + j] = v.y;
+    list[2 * NEAR_CAP + j] = v.z;
+    list[3 * NEAR_CAP + j] = soft.x;
+    list[4 * NEAR_CAP + j] = soft.y;
+    list[5 * NEAR_CAP + j] = soft.z;
+}
+// A flush takes a whole number of quanta; the last one of a group is filled up
+// with massless entries 1e18 away (r^2 is finite and the terms exactly zero).
 #define PAD_ENTRY make_float4(1e18f, 1e18f, 1e18f, 0.f)
+#define PAD_SOFT make_float4(1.f, 0.f, 0.f, 0.f)
 
 // Cubic-spline softened force and potential factors for u = r/h < 1
 // (kernel.h:452-470), without a branch or a per-piece coefficient choice.  The
@@ -222,51 +257,34 @@ __device__ __forceinline__ float2 spline_wf2(float2 u, float2 iu, float2 *wp)
     return fma2(dup2(-256.f), mul2(mul2(mul2(q, iu), iu), iu), fin);
 }
 
+// Targets per lane (TPL) and lane parts (SPLIT): the warp's SPLIT parts of
+// 32 / SPLIT lanes all hold the same TPL * 32 / SPLIT targets, and each part
+// evaluates its share of the list entries.  Groups of up to 32 targets use
+// TPL = SPLIT = 2, larger ones TPL = 2, SPLIT = 1.  With two targets per lane a
+// load of entries serves both, and the parts load different entries at once:
+// half the loads per target of one target per lane, and half the L1 cycles (a
+// uniform 128-bit shared-memory load returns 512 bytes to the warp: with one
+// target per lane L1 was 82% busy in the far flush).
+//
+// What bounds the walk is instruction issue.  A packed FP32x2 instruction takes
+// two issue slots; counting those twice, 91-93% of all slots are taken (issue
+// active 60% + half of the FMA pipe's 63%).  The far flush alone runs at 15.1
+// slots per entry and 32 targets (13 FP32 operations, one rsqrt, a share of the
+// loads), the near flush at 43 (49.9 before its softening record was {h^-2, m/h,
+// m/h^3}).
 template <int TPL>
 struct Targets {
     float x[TPL], y[TPL], z[TPL], h[TPL], hinv[TPL];
     bool valid[TPL];
     Kahan ax[TPL], ay[TPL], az[TPL], pot[TPL];
-    int nint[TPL];
+    int self[TPL];   // near entries at r = 0: the target itself or a coincident particle
 };
 
-// Far list: Newtonian for every target of the group, two entries per packed
-// instruction.  Each flush keeps one partial sum per entry parity and adds
-// both into the Kahan totals.
-// POT: the potential-only walk (force_treeevaluate_potential, forcetree.c:3169-3474)
+// The per-entry sums of a flush, added to the targets' Kahan totals.
 template <int TPL, bool POT>
-__device__ __forceinline__ void flush_far(float *__restrict__ far, int nf, Targets<TPL> &T)
+__device__ __forceinline__ void add_sums(Targets<TPL> &T, const float2 (&px)[TPL], const float2 (&py)[TPL],
+                                         const float2 (&pz)[TPL], const float2 (&pp)[TPL])
 {
-    if ((nf & 1) && (threadIdx.x & 31) == 0) list_put(far, nf, PAD_ENTRY);
-    __syncwarp();
-    const float4 *L = reinterpret_cast<const float4 *>(far);
-    float2 px[TPL], py[TPL], pz[TPL], pp[TPL], nx[TPL], ny[TPL], nz[TPL];
-#pragma unroll
-    for (int s = 0; s < TPL; s++) {
-        px[s] = py[s] = pz[s] = pp[s] = dup2(0.f);
-        nx[s] = dup2(-T.x[s]); ny[s] = dup2(-T.y[s]); nz[s] = dup2(-T.z[s]);
-    }
-    const int np = (nf + 1) >> 1;
-#pragma unroll 2
-    for (int q = 0; q < np; q++) {
-        const float4 A = L[2 * q], B = L[2 * q + 1];
-        const float2 ex = make_float2(A.x, A.y), ey = make_float2(A.z, A.w);
-        const float2 ez = make_float2(B.x, B.y), em = make_float2(B.z, B.w);
-#pragma unroll
-        for (int s = 0; s < TPL; s++) {
-            const float2 dx = add2(ex, nx[s]), dy = add2(ey, ny[s]), dz = add2(ez, nz[s]);
-            const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-            const float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-            const float2 mr = mul2(em, rinv);
-            if (!POT) {
-                const float2 fac = mul2(mul2(mr, rinv), rinv);
-                px[s] = fma2(dx, fac, px[s]);
-                py[s] = fma2(dy, fac, py[s]);
-                pz[s] = fma2(dz, fac, pz[s]);
-            }
-            pp[s] = fma2(mr, dup2(-1.f), pp[s]);
-        }
-    }
 #pragma unroll
     for (int s = 0; s < TPL; s++) {
         if (!POT) {
@@ -275,9 +293,51 @@ __device__ __forceinline__ void flush_far(float *__restrict__ far, int nf, Targe
             T.az[s].add(pz[s].x + pz[s].y);
         }
         T.pot[s].add(pp[s].x + pp[s].y);
-        T.nint[s] += nf;
     }
-    __syncwarp();
+}
+
+// Far list: Newtonian for every target of the group, two entries per packed
+// instruction, four per load.  n is a whole number of quanta (4 * SPLIT
+// entries).  Each flush keeps one partial sum per entry parity and adds both
+// into the Kahan totals.
+// POT: the potential-only walk (force_treeevaluate_potential, forcetree.c:3169-3474)
+template <int TPL, int SPLIT, bool POT>
+__device__ __forceinline__ void flush_far(const float *__restrict__ far, int n, int part, Targets<TPL> &T)
+{
+    float2 px[TPL], py[TPL], pz[TPL], pp[TPL], nx[TPL], ny[TPL], nz[TPL];
+#pragma unroll
+    for (int s = 0; s < TPL; s++) {
+        px[s] = py[s] = pz[s] = pp[s] = dup2(0.f);
+        nx[s] = dup2(-T.x[s]); ny[s] = dup2(-T.y[s]); nz[s] = dup2(-T.z[s]);
+    }
+    const float4 *X = reinterpret_cast<const float4 *>(far) + part;
+    constexpr int c4 = FAR_CAP / 4;
+#pragma unroll 1
+    for (int q = n / (4 * SPLIT); q > 0; q--, X += SPLIT) {
+        const float4 x4 = X[0], y4 = X[c4], z4 = X[2 * c4], m4 = X[3 * c4];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const float2 ex = e ? make_float2(x4.z, x4.w) : make_float2(x4.x, x4.y);
+            const float2 ey = e ? make_float2(y4.z, y4.w) : make_float2(y4.x, y4.y);
+            const float2 ez = e ? make_float2(z4.z, z4.w) : make_float2(z4.x, z4.y);
+            const float2 em = e ? make_float2(m4.z, m4.w) : make_float2(m4.x, m4.y);
+#pragma unroll
+            for (int s = 0; s < TPL; s++) {
+                const float2 dx = add2(ex, nx[s]), dy = add2(ey, ny[s]), dz = add2(ez, nz[s]);
+                const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                const float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+                const float2 mr = mul2(em, rinv);
+                if (!POT) {
+                    const float2 fac = mul2(mul2(mr, rinv), rinv);
+                    px[s] = fma2(dx, fac, px[s]);
+                    py[s] = fma2(dy, fac, py[s]);
+                    pz[s] = fma2(dz, fac, pz[s]);
+                }
+                pp[s] = fma2(mr, dup2(-1.f), pp[s]);
+            }
+        }
+    }
+    add_sums<TPL, POT>(T, px, py, pz, pp);
 }
 
 // Near list: entries within the softening of some target of the group.  Most
@@ -288,107 +348,136 @@ __device__ __forceinline__ void flush_far(float *__restrict__ far, int nf, Targe
 // counted.
 // POT: the potential-only walk, which has no r^2 > 0 condition: an r = 0 pair
 // adds m w_pot(0) / h like any other (the caller removes the self term).
-// HOMOG: every target of the group has the same kernel radius h_t, so the
-// pair's softening h_g = max(h_t, h_source) and its products are per entry,
-// formed when the entry was listed: nearH = {h_g, 1/h_g, m/h_g, m/h_g^3}.
-// Otherwise nearH = {h_source, 1/h_source} and h_g is formed per pair.
-template <int TPL, bool POT, bool HOMOG>
-__device__ __forceinline__ void flush_near(float *__restrict__ nearE, float *__restrict__ nearH, int nn,
-                                           Targets<TPL> &T)
+//
+// This form is for groups of one kernel radius h_t (most groups): the pair's
+// softening h_g = max(h_t, h_source) and its products are per entry, formed
+// when the entry was listed: {h_g^-2, m/h_g, m/h_g^3}.  u^2 = r^2 / h_g^2 and its
+// rsqrt give u and 1/u, and force and potential share t^4/u (t and the spline:
+// see spline_wf2).
+// r^2 = 0 gives u = 1e-18: a finite force factor, times an offset of zero.
+template <int TPL, int SPLIT, bool POT>
+__device__ __forceinline__ void flush_near(const float *__restrict__ near, int n, int part, Targets<TPL> &T)
 {
-    if ((nn & 1) && (threadIdx.x & 31) == 0) {
-        list_put(nearE, nn, PAD_ENTRY);
-        list_put(nearH, nn, make_float4(1.f, 1.f, 0.f, 0.f));
-    }
-    __syncwarp();
-    const float4 *LE = reinterpret_cast<const float4 *>(nearE);
-    const float4 *LH = reinterpret_cast<const float4 *>(nearH);
     float2 px[TPL], py[TPL], pz[TPL], pp[TPL], nx[TPL], ny[TPL], nz[TPL];
-    int self[TPL];
 #pragma unroll
     for (int s = 0; s < TPL; s++) {
         px[s] = py[s] = pz[s] = pp[s] = dup2(0.f);
         nx[s] = dup2(-T.x[s]); ny[s] = dup2(-T.y[s]); nz[s] = dup2(-T.z[s]);
-        self[s] = 0;
     }
-    const int np = (nn + 1) >> 1;
-#pragma unroll 2
-    for (int q = 0; q < np; q++) {
-        const float4 A = LE[2 * q], B = LE[2 * q + 1], C = LH[2 * q], D = LH[2 * q + 1];
-        const float2 ex = make_float2(A.x, A.y), ey = make_float2(A.z, A.w);
-        const float2 ez = make_float2(B.x, B.y), em = make_float2(B.z, B.w);
-        const float2 hs = make_float2(C.x, C.y), hsinv = make_float2(C.z, C.w);
-        const float2 mh = make_float2(D.x, D.y), mh3 = make_float2(D.z, D.w);
+    const float2 *X = reinterpret_cast<const float2 *>(near) + part;
+    constexpr int c2 = NEAR_CAP / 2;
+#pragma unroll 1
+    for (int q = n / (2 * SPLIT); q > 0; q--, X += SPLIT) {
+        const float2 ex = X[0], ey = X[c2], ez = X[2 * c2], h2 = X[3 * c2], mh = X[4 * c2], mh3 = X[5 * c2];
 #pragma unroll
         for (int s = 0; s < TPL; s++) {
             const float2 dx = add2(ex, nx[s]), dy = add2(ey, ny[s]), dz = add2(ez, nz[s]);
             const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-            const float2 hg = HOMOG ? hs : make_float2(fmaxf(T.h[s], hs.x), fmaxf(T.h[s], hs.y));
+            float2 u2 = mul2(r2, h2);
+            u2 = make_float2(fmaxf(u2.x, 1e-36f), fmaxf(u2.y, 1e-36f));
+            const float2 iu = make_float2(rsqrtf(u2.x), rsqrtf(u2.y));
+            const float2 u = mul2(u2, iu), iu2 = mul2(iu, iu);
+            // saturated above 1, where the Newtonian form is selected
+            const float2 t = make_float2(__saturatef(u.x - 0.5f), __saturatef(u.y - 0.5f));
+            const float2 t2 = mul2(t, t), t4u = mul2(mul2(t2, t2), iu);
+            const float2 pin =
+                fma2(u2, fma2(u2, fma2(u, dup2(6.4f), dup2(-9.6f)), dup2(5.333333333333f)), dup2(-2.8f));
+            const float2 wp = fma2(mul2(t4u, t), fma2(t, dup2(-8.533333333333f), dup2(-6.4f)), pin);
+            // spline for u = r/h_g < 1 (kernel.h:452-470), Newtonian beyond (:391-398);
+            // the two meet at u = 1, where the spline's force factor is 1/u^3
+            const bool sx = u.x < 1.f, sy = u.y < 1.f;
+            float2 fp = sel2(sx, sy, wp, make_float2(-iu.x, -iu.y));
+            if (!POT) {
+                const float2 fin = fma2(u2, fma2(u, dup2(32.f), dup2(-38.4f)), dup2(10.666666666667f));
+                const float2 out = fma2(t, fma2(t, dup2(-42.666666666667f), dup2(-51.2f)), dup2(-16.f));
+                const float2 wf = fma2(mul2(t4u, iu2), out, fin);
+                const float2 fac = mul2(mh3, sel2(sx, sy, wf, mul2(iu2, iu)));
+                const bool ux = r2.x > 0.f, uy = r2.y > 0.f;
+                fp = sel2(ux, uy, fp, dup2(0.f));
+                T.self[s] += (ux ? 0 : 1) + (uy ? 0 : 1);
+                px[s] = fma2(dx, fac, px[s]);
+                py[s] = fma2(dy, fac, py[s]);
+                pz[s] = fma2(dz, fac, pz[s]);
+            }
+            pp[s] = fma2(mh, fp, pp[s]);
+        }
+    }
+    add_sums<TPL, POT>(T, px, py, pz, pp);
+}
+
+// The same for groups of several kernel radii: h_g is formed per pair from the
+// entry's {h_source, 1/h_source, m}.
+template <int TPL, int SPLIT, bool POT>
+__device__ __forceinline__ void flush_near_mixed(const float *__restrict__ near, int n, int part, Targets<TPL> &T)
+{
+    float2 px[TPL], py[TPL], pz[TPL], pp[TPL], nx[TPL], ny[TPL], nz[TPL];
+#pragma unroll
+    for (int s = 0; s < TPL; s++) {
+        px[s] = py[s] = pz[s] = pp[s] = dup2(0.f);
+        nx[s] = dup2(-T.x[s]); ny[s] = dup2(-T.y[s]); nz[s] = dup2(-T.z[s]);
+    }
+    const float2 *X = reinterpret_cast<const float2 *>(near) + part;
+    constexpr int c2 = NEAR_CAP / 2;
+#pragma unroll 1
+    for (int q = n / (2 * SPLIT); q > 0; q--, X += SPLIT) {
+        const float2 ex = X[0], ey = X[c2], ez = X[2 * c2], hs = X[3 * c2], hsinv = X[4 * c2], em = X[5 * c2];
+#pragma unroll
+        for (int s = 0; s < TPL; s++) {
+            const float2 dx = add2(ex, nx[s]), dy = add2(ey, ny[s]), dz = add2(ez, nz[s]);
+            const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+            const float2 hg = make_float2(fmaxf(T.h[s], hs.x), fmaxf(T.h[s], hs.y));
             // 1/h_g: the inverses are rounded alike
-            const float2 hinv = HOMOG ? hsinv : make_float2(fminf(T.hinv[s], hsinv.x), fminf(T.hinv[s], hsinv.y));
+            const float2 hinv = make_float2(fminf(T.hinv[s], hsinv.x), fminf(T.hinv[s], hsinv.y));
             // finite at r = 0 when it counts
             const float2 rinv = make_float2(rsqrtf(POT ? fmaxf(r2.x, 1e-30f) : r2.x),
                                             rsqrtf(POT ? fmaxf(r2.y, 1e-30f) : r2.y));
-            // spline for u = r/h_g < 1 (kernel.h:452-470), Newtonian beyond (:391-398);
-            // the two meet at u = 1, where the spline's force factor is 1/u^3
             const float2 u = mul2(mul2(r2, rinv), hinv), iu = mul2(hg, rinv);
             float2 wp;
             const float2 wf = spline_wf2(u, iu, &wp);
             const bool sx = u.x < 1.f, sy = u.y < 1.f;
-            float2 fpot, fac = dup2(0.f);
-            if (HOMOG) {   // Newtonian as m/h_g^3 (1/u)^3 and -m/h_g (1/u), on the entry's products
-                fpot = mul2(mh, sel2(sx, sy, wp, make_float2(-iu.x, -iu.y)));
-                if (!POT) fac = mul2(mh3, sel2(sx, sy, wf, mul2(mul2(iu, iu), iu)));
-            } else {
-                const float2 mr = mul2(em, rinv);
-                fpot = sel2(sx, sy, mul2(mul2(em, wp), hinv), make_float2(-mr.x, -mr.y));
-                if (!POT)
-                    fac = sel2(sx, sy, mul2(mul2(em, wf), mul2(mul2(hinv, hinv), hinv)), mul2(mul2(mr, rinv), rinv));
-            }
-            if (POT) {
-                pp[s] = add2(pp[s], fpot);
-            } else {
+            const float2 mr = mul2(em, rinv);
+            float2 fp = sel2(sx, sy, mul2(mul2(em, wp), hinv), make_float2(-mr.x, -mr.y));
+            if (!POT) {
+                float2 fac =
+                    sel2(sx, sy, mul2(mul2(em, wf), mul2(mul2(hinv, hinv), hinv)), mul2(mul2(mr, rinv), rinv));
                 const bool ux = r2.x > 0.f, uy = r2.y > 0.f;
                 fac = sel2(ux, uy, fac, dup2(0.f));
-                fpot = sel2(ux, uy, fpot, dup2(0.f));
-                self[s] += (ux ? 0 : 1) + (uy ? 0 : 1);
+                fp = sel2(ux, uy, fp, dup2(0.f));
+                T.self[s] += (ux ? 0 : 1) + (uy ? 0 : 1);
                 px[s] = fma2(dx, fac, px[s]);
                 py[s] = fma2(dy, fac, py[s]);
                 pz[s] = fma2(dz, fac, pz[s]);
-                pp[s] = add2(pp[s], fpot);
             }
+            pp[s] = add2(pp[s], fp);
         }
     }
+    add_sums<TPL, POT>(T, px, py, pz, pp);
+}
+
+// moves the r < 8 entries from m on to the front of a list of NA arrays (m >= 24)
+template <int NA, int CAP>
+__device__ __forceinline__ void list_shift(float *list, int m, int r, int lane)
+{
+    __syncwarp();
+    if (lane < r) {
 #pragma unroll
-    for (int s = 0; s < TPL; s++) {
-        if (!POT) {
-            T.ax[s].add(px[s].x + px[s].y);
-            T.ay[s].add(py[s].x + py[s].y);
-            T.az[s].add(pz[s].x + pz[s].y);
-        }
-        T.pot[s].add(pp[s].x + pp[s].y);
-        T.nint[s] += nn - self[s];
+        for (int a = 0; a < NA; a++) list[a * CAP + lane] = list[a * CAP + m + lane];
     }
     __syncwarp();
 }
 
-template <int TPL, bool POT>
-__device__ __forceinline__ void flush_near_sel(bool homog, float *__restrict__ nearE, float *__restrict__ nearH,
-                                               int nn, Targets<TPL> &T)
-{
-    if (homog) flush_near<TPL, POT, true>(nearE, nearH, nn, T);
-    else flush_near<TPL, POT, false>(nearE, nearH, nn, T);
-}
-
-// softening record of a near-list entry with kernel radius hsrc and mass m (see flush_near)
-__device__ __forceinline__ float4 near_soft(float hsrc, float m, bool homog, float hgroup)
+// Softening record of a near-list entry with kernel radius hsrc and mass m (see
+// flush_near).  hzero: the kernel radius that takes the place of zero, far below
+// the distances in the group's box, so that the products stay finite.
+__device__ __forceinline__ float4 near_soft(float hsrc, float m, bool homog, float hgroup, float hzero)
 {
     if (homog) {
-        const float hg = fmaxf(hgroup, hsrc);
-        const float hinv = hg > 0.f ? __frcp_rn(hg) : INFINITY;
-        return make_float4(hg, hinv, m * hinv, m * (hinv * hinv * hinv));
+        float hg = fmaxf(hgroup, hsrc);
+        if (hg == 0.f) hg = hzero;
+        const float hinv = __frcp_rn(hg);
+        return make_float4(hinv * hinv, m * hinv, m * (hinv * hinv * hinv), 0.f);
     }
-    return make_float4(hsrc, hsrc > 0.f ? __frcp_rn(hsrc) : INFINITY, 0.f, 0.f);
+    return make_float4(hsrc, hsrc > 0.f ? __frcp_rn(hsrc) : INFINITY, m, 0.f);
 }
 
 __device__ __forceinline__ double warp_min_d(double v)
@@ -412,39 +501,29 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane)
     }
     return v;
 }
-// exclusive prefix sum over the warp of v in [0, 2^BITS) from one ballot per
-// bit, and the total from one reduction: the votes are independent, so the
-// latency is that of one vote, not of a chain of shuffles
-template <int BITS>
-__device__ __forceinline__ int warp_excl_bits(int v, unsigned lt_mask, int *total)
-{
-    int ex = 0;
-#pragma unroll
-    for (int b = 0; b < BITS; b++) ex += __popc(__ballot_sync(FULL, (v >> b) & 1) & lt_mask) << b;
-    *total = (int)__reduce_add_sync(FULL, (unsigned)v);
-    return ex;
-}
-
-// MINB: resident blocks per SM the register allocation must allow (1..3): a
-// tuning knob trading registers (spills) against warps in flight.
 // F64T: opening tests in FP64 (used for one-target groups, where the tests are
 // exactly the reference's); otherwise the tests run in FP32 on FP64-formed
 // offsets from the group centre, against a bounding box rounded outwards.
-template <int TPL, int MINB, bool F64T, bool POT, bool TMA = false>
-__global__ void __launch_bounds__(WALK_THREADS, MINB) k_walk(WalkParams p)
+template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA = false>
+__global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
 {
     extern __shared__ float4 walk_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
-    const int FL = p.flush, cap = list_cap(FL);
-    float *far = reinterpret_cast<float *>(walk_smem + (size_t)warp * walk_warp_float4s(FL));
-    float *nearE = far + 4 * cap;
-    float *nearH = nearE + 4 * cap;
-    int *sstack = reinterpret_cast<int *>(far + 12 * cap);
-    int4 *const nslot = reinterpret_cast<int4 *>(far + 12 * cap + WALK_SSTACK) + 4 * lane;
-    const unsigned slot0 = (unsigned)__cvta_generic_to_shared(far + 12 * cap + WALK_SSTACK);
-    int *pq = reinterpret_cast<int *>(far + 12 * cap + WALK_SSTACK + 32 * 16);
-    const unsigned bar = (unsigned)__cvta_generic_to_shared(far + 12 * cap + WALK_SSTACK + 32 * 16 + PQ_CAP);
+    constexpr int LP = 32 / SPLIT;   // lanes per part
+    constexpr int QUANTUM = 4 * SPLIT;
+    const int part = lane / LP;
+    const int swz = TMA ? 0 : (lane >> 1) & 3;   // node slot pieces, see stage_node
+    const int FL = min(p.flush, FAR_FLUSH_MAX), NL = min(p.flush, NEAR_FLUSH_MAX);
+    float *far = reinterpret_cast<float *>(walk_smem) + (size_t)warp * WALK_WARP_FLOATS;
+    float *near = far + FAR_ARRAYS * FAR_CAP;
+    float *rest = near + NEAR_ARRAYS * NEAR_CAP;
+    int *sstack = reinterpret_cast<int *>(rest);
+    int4 *const nslot = reinterpret_cast<int4 *>(rest + WALK_SSTACK) + 4 * lane;
+    const unsigned slot0 = (unsigned)__cvta_generic_to_shared(rest + WALK_SSTACK);
+    int *run = reinterpret_cast<int *>(rest + WALK_SSTACK + NH * 32 * 16);   // see expand
+    int *qbase = run + 32, *qend = qbase + RUNS;   // queued runs: first particle less its position, end position
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(qend + RUNS);
     if (lane == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -473,10 +552,10 @@ __global__ void __launch_bounds__(WALK_THREADS, MINB) k_walk(WalkParams p)
         float hmin = INFINITY, hmax = 0.f;
 #pragma unroll
         for (int s = 0; s < TPL; s++) {
-            int k = s * 32 + lane;
+            int k = s * LP + lane % LP;
             bool v = k < grp.count;
             T.valid[s] = v;
-            T.nint[s] = 0;
+            T.self[s] = 0;
             T.ax[s] = {0.f, 0.f}; T.ay[s] = {0.f, 0.f}; T.az[s] = {0.f, 0.f}; T.pot[s] = {0.f, 0.f};
             tpi[s] = -1;
             tx[s] = ty[s] = tz[s] = 0.0;
@@ -520,44 +599,304 @@ __global__ void __launch_bounds__(WALK_THREADS, MINB) k_walk(WalkParams p)
         const float hwf[3] = {__double2float_ru(hw[0]), __double2float_ru(hw[1]), __double2float_ru(hw[2])};
         const float aoldf = (float)aold_min, thetaf = (float)theta;
         const bool homog = hmin == hmax;   // one kernel radius in the group (warp-uniform)
+        const float hwmax = fmaxf(hwf[0], fmaxf(hwf[1], hwf[2])), hzero = hwmax > 0.f ? 1e-6f * hwmax : 1.f;
 
         // ---- traversal
-        // The node stack lives in shared memory (sp entries) on top of a spill
-        // area in global memory (gsp entries).  Each round pops up to 32 nodes;
-        // the next round's node records are staged (cp.async) before this
-        // round's leaf particles and list flushes are processed, which hides
-        // their latency.
-        int sp = 1, gsp = 0, nf = 0, nn = 0;
+        // Each round tests up to 32 NH nodes, NH per lane.  The next round's nodes
+        // are the last of {node stack, children of this round's opened
+        // nodes}; only what is left over goes to the stack, which lives in shared
+        // memory (sp entries) on top of a spill area in global memory (gsp
+        // entries).  Their records are staged (cp.async) before this round's leaf
+        // particles and list flushes are processed, and a batch of particle
+        // records is in flight during the tests.  One loop does whatever is due,
+        // so that every part appears in the code once (the kernel is large
+        // against the instruction cache).
+        int sp = 0, gsp = 0, nf = 0, nn = 0;
+        int qhead = 0, qtail = 0;     // runs of particles in the queue
+        int pw = 0, pt = 0;           // positions of the queue's particles: next, end
         int list_far = 0, list_near = 0, tested = 0;   // warp-uniform statistics of this group
-        bool overflow = false;
-        if (lane == 0) sstack[0] = grp.root;
-        __syncwarp();
-        // pop up to 32 nodes (one per lane); returns the count (warp-uniform)
-        auto pop_nodes = [&](int &node) -> int {
-            if (sp == 0 && gsp > 0) {   // refill from the spill area, keeping stack order
-                const int m = min(gsp, WALK_SSTACK / 2);
-                for (int i = lane; i < m; i += 32) sstack[i] = gstack[gsp - m + i];
-                gsp -= m;
-                sp = m;
-                __syncwarp();
-            }
-            const int k = min(sp, 32);
-            node = -1;
-            if (lane < k) node = sstack[sp - k + lane];
-            sp -= k;
-            __syncwarp();
-            return k;
+        int limit = FL, nlimit = NL;  // the lists are flushed at these lengths; 1 once the traversal is over
+        bool overflow = false, timed_out = false;
+        int k = 1;                    // nodes staged for the next round
+        auto stage = [&](const int (&node)[NH], int kn) {
+            if (kn == 0) return;
+            if (tma) stage_nodes(bar, slot0, p.nodes, node, kn, lane);   // one barrier phase per staged round
+            else stage_lanes(slot0, p.nodes, node, kn, lane);
         };
-        // evaluate the top m (<= 32) particles of the queue, one per lane:
-        // classify them against the group box and append them to the lists
-        int qn = 0;
-        auto take_particles = [&](int m) {
-            bool use = false, pfar = false;
-            float4 pe = make_float4(0.f, 0.f, 0.f, 0.f);
-            float ph = 0.f;
-            if (lane < m) {
-                const GGPart pp = load_part(p.parts + pq[qn - m + lane]);
-                if (pp.m > 0.f) {
+        {
+            int node[NH];
+            node[0] = lane == 0 ? grp.root : -1;
+            stage(node, k);
+        }
+        // appends one entry per lane with `use`: to the far list, or to the near list with its softening
+        auto append = [&](bool use, bool isfar, const float4 &e, float h) {
+            const unsigned mu = __ballot_sync(FULL, use), mf = __ballot_sync(FULL, use && isfar), mn = mu & ~mf;
+            if (use && isfar) list_put(far, nf + __popc(mf & lt_mask), e);
+            if (mn) {   // warp-uniform
+                if (use && !isfar) near_put(near, nn + __popc(mn & lt_mask), e, near_soft(h, e.w, homog, hmax, hzero));
+                nn += __popc(mn);
+                list_near += __popc(mn);
+            }
+            nf += __popc(mf);
+            list_far += __popc(mf);
+        };
+        // Runs of consecutive indices laid end to end: a run maps its positions q
+        // to base + q.  The lane that owns a run's first position in a window of 32
+        // has stored its base at run[position] and set its bit; each lane then looks
+        // back to the nearest such position.  Returns the index at the lane's
+        // position, or -1 before the first run.  (Conversions, population counts
+        // and bit searches run at a quarter of the rate of other integer work, in
+        // the pipe that the flushes' rsqrt needs: one search per window, instead of
+        // counts per bit of the run lengths.)
+        auto lookup = [&](unsigned bits, int w) -> int {
+            const unsigned starts = __reduce_or_sync(FULL, bits) & (lt_mask | (1u << lane));
+            __syncwarp();
+            const int index = starts ? run[31 - __clz((int)starts)] + w + lane : -1;
+            __syncwarp();   // the next window writes run
+            return index;
+        };
+        // the lane's NH runs of positions beg to end - 1; the window starts at position w
+        auto expand = [&](const int (&base)[NH], const int (&beg)[NH], const int (&end)[NH], int w) -> int {
+            unsigned bits = 0;
+#pragma unroll
+            for (int h = 0; h < NH; h++) {
+                const int d = max(beg[h] - w, 0);
+                if (end[h] > w && d < 32 && end[h] > beg[h]) {
+                    run[d] = base[h];
+                    bits |= 1u << d;
+                }
+            }
+            return lookup(bits, w);
+        };
+        for (;;) {
+            // ---- full lists: their whole quanta are evaluated, the rest moves to the front
+            if (nf >= limit) {
+                const int m = nf & ~(QUANTUM - 1);
+                __syncwarp();
+                flush_far<TPL, SPLIT, POT>(far, m, part, T);
+                nf -= m;
+                list_shift<FAR_ARRAYS, FAR_CAP>(far, m, nf, lane);
+            }
+            if (nn >= nlimit) {
+                const int m = nn & ~(QUANTUM - 1);
+                __syncwarp();
+                if (homog) flush_near<TPL, SPLIT, POT>(near, m, part, T);
+                else flush_near_mixed<TPL, SPLIT, POT>(near, m, part, T);
+                nn -= m;
+                list_shift<NEAR_ARRAYS, NEAR_CAP>(near, m, nn, lane);
+            }
+            // ---- the next 32 queued particles, one per lane: their records are loaded here and used below
+            const bool batch = pt - pw >= 32 || (pt > pw && k == 0);
+            GGPart pp;
+            bool have = false;
+            if (batch) {
+                const int m = min(32, pt - pw);
+                const bool queued = qhead + lane < qtail;
+                const int slot = (qhead + lane) & (RUNS - 1);
+                const int end = queued ? qend[slot] - pw : INT_MAX;   // runs are not empty: 32 of them suffice
+                int d = __shfl_up_sync(FULL, end, 1);
+                if (lane == 0) d = 0;
+                unsigned bits = 0;
+                if (queued && d < 32) {
+                    run[d] = qbase[slot];
+                    bits = 1u << d;
+                }
+                const int i = lookup(bits, pw);
+                have = lane < m;
+                if (have) pp = load_part(p.parts + i);
+                pw += m;
+                qhead += __popc(__ballot_sync(FULL, end <= m));
+            }
+            // ---- a round of node tests
+            if (k > 0 && pt - pw < 32) {
+                tested += k;
+                if (tma) {
+                    if (!bar_wait(bar, phase)) {
+                        timed_out = true;
+                        break;
+                    }
+                    phase ^= 1u;
+                } else {
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    __syncwarp();   // other lanes' copies too
+                }
+                int na[NH], nc[NH], np[NH];
+                float4 ent[NH];
+                float soft[NH];
+                bool used[NH], isfar[NH];
+#pragma unroll
+                for (int h = 0; h < NH; h++) {
+                    na[h] = nc[h] = np[h] = 0;
+                    ent[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    soft[h] = 0.f;
+                    used[h] = isfar[h] = false;
+                    if (k <= 32 * h) continue;   // warp-uniform
+                    GGNode nd;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) reinterpret_cast<int4 *>(&nd)[i] = nslot[32 * 4 * h + (i ^ swz)];
+                    const int nb = nd.b;
+                    const float ms = nd.maxsoft, L = nd.len;
+                    bool open;
+                    if (!F64T) {
+                        const float dx = (float)(nd.cx - cg[0]), dy = (float)(nd.cy - cg[1]),
+                                    dz = (float)(nd.cz - cg[2]);
+                        const float ex = fmaxf(fabsf(dx) - hwf[0], 0.f), ey = fmaxf(fabsf(dy) - hwf[1], 0.f),
+                                    ez = fmaxf(fabsf(dz) - hwf[2], 0.f);
+                        const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+                        const float hh = fmaxf(hmax, ms);
+                        if (thetaf > 0.f) {
+                            open = ((hmin < ms) && (r2 < ms * ms)) || (L * L > r2 * thetaf * thetaf);
+                        } else {
+                            // r < soft + 0.6 len for the larger of the two softenings, which
+                            // also covers r < maxsoft
+                            const float a1 = fmaf(0.6f, L, hh);
+                            open = (r2 < a1 * a1) | (nd.mass * L * L > r2 * r2 * aoldf) |
+                                   ((fabsf(dx + nd.gx) < fmaf(0.6f, L, hwf[0])) &
+                                    (fabsf(dy + nd.gy) < fmaf(0.6f, L, hwf[1])) &
+                                    (fabsf(dz + nd.gz) < fmaf(0.6f, L, hwf[2])));
+                        }
+                        ent[h] = make_float4(dx, dy, dz, nd.mass);
+                        isfar[h] = (r2 >= hh * hh) && (r2 > FAR_MIN_R2);
+                    } else {
+                        const double dx = nd.cx - cg[0], dy = nd.cy - cg[1], dz = nd.cz - cg[2];
+                        const double ex = fmax(fabs(dx) - hw[0], 0.0), ey = fmax(fabs(dy) - hw[1], 0.0),
+                                     ez = fmax(fabs(dz) - hw[2], 0.0);
+                        const double r2 = ex * ex + ey * ey + ez * ez;
+                        const double msd = (double)ms, Ld = (double)L;
+                        open = (hmind < msd) && (r2 < msd * msd);
+                        if (!open) {
+                            if (theta > 0.0) {
+                                open = Ld * Ld > r2 * theta * theta;
+                            } else {
+                                const double a1 = hmaxd + 0.6 * Ld, a2 = msd + 0.6 * Ld;
+                                open = (r2 < a1 * a1) || (r2 < a2 * a2) ||
+                                       ((double)nd.mass * Ld * Ld > r2 * r2 * aold_min);
+                                if (!open) {
+                                    const double gx = fabs(dx + (double)nd.gx), gy = fabs(dy + (double)nd.gy),
+                                                 gz = fabs(dz + (double)nd.gz);
+                                    open = (gx < 0.6 * Ld + hw[0]) && (gy < 0.6 * Ld + hw[1]) &&
+                                           (gz < 0.6 * Ld + hw[2]);
+                                }
+                            }
+                        }
+                        ent[h] = make_float4((float)dx, (float)dy, (float)dz, nd.mass);
+                        const double hh = fmax(hmaxd, msd);
+                        isfar[h] = (r2 >= hh * hh) && (r2 > (double)FAR_MIN_R2);
+                    }
+                    const bool some = 32 * h + lane < k && nd.mass > 0.f;   // massless nodes are skipped
+                    open = open || nb == -1;                                // one particle: always opened
+                    used[h] = some && !open;
+                    soft[h] = ms;
+                    na[h] = nd.a;
+                    nc[h] = some && open ? max(nb, 0) : 0;    // children of an opened node
+                    np[h] = some && open ? max(-nb, 0) : 0;   // particles of an opened leaf
+                }
+#pragma unroll
+                for (int h = 0; h < NH; h++) append(used[h], isfar[h], ent[h], soft[h]);
+                // the opened nodes' children (particles) laid end to end over the warp, from one scan of both counts
+                int cl = 0, pl = 0;   // this lane's
+#pragma unroll
+                for (int h = 0; h < NH; h++) { cl += nc[h]; pl += np[h]; }
+                int cend, ctot, pend;
+                int ptot;
+                if (__any_sync(FULL, pl > 1023)) {   // an unsplit leaf at the depth limit
+                    cend = warp_incl_scan(cl, lane);
+                    pend = warp_incl_scan(pl, lane);
+                    ctot = __shfl_sync(FULL, cend, 31);
+                    ptot = __shfl_sync(FULL, pend, 31);
+                } else {
+                    const int both = warp_incl_scan(cl | (pl << 16), lane), sum = __shfl_sync(FULL, both, 31);
+                    cend = both & 0xffff;
+                    pend = both >> 16;
+                    ctot = sum & 0xffff;
+                    ptot = sum >> 16;
+                }
+                int cbase[NH], cbeg[NH], cfin[NH];
+                int c = cend - cl, q = pt + pend - pl;
+#pragma unroll
+                for (int h = 0; h < NH; h++) {
+                    cbase[h] = na[h] - c;
+                    cbeg[h] = c;
+                    c += nc[h];
+                    cfin[h] = c;
+                }
+                if (ptot > 0) {   // the opened leaves' runs join the queue, in the order of their positions
+                    int slot = qtail;
+#pragma unroll
+                    for (int h = 0; h < NH; h++) {
+                        const unsigned ml = __ballot_sync(FULL, np[h] > 0);
+                        slot += __popc(ml & lt_mask);
+                        qtail += __popc(ml);
+                    }
+#pragma unroll
+                    for (int h = 0; h < NH; h++) {
+                        if (np[h] > 0) {
+                            qbase[slot & (RUNS - 1)] = na[h] - q;
+                            q += np[h];
+                            qend[slot & (RUNS - 1)] = q;
+                            slot++;
+                        }
+                    }
+                    pt += ptot;
+                }
+                if (sp == 0 && ctot == 0 && gsp > 0) {   // refill from the spill area, keeping stack order
+                    const int m = min(gsp, WALK_SSTACK / 2);
+                    for (int i = lane; i < m; i += 32) sstack[i] = gstack[gsp - m + i];
+                    gsp -= m;
+                    sp = m;
+                }
+                __syncwarp();
+                k = min(sp + ctot, 32 * NH);
+                const int w0 = ctot - k;   // first position taken now; negative: from the stack
+                int node[NH];
+#pragma unroll
+                for (int h = 0; h < NH; h++) {
+                    const int w = w0 + 32 * h;
+                    node[h] = -1;
+                    if (w + 32 > 0 && w < ctot) node[h] = expand(cbase, cbeg, cfin, w);
+                    if (w + lane < 0) node[h] = sstack[sp + w + lane];
+                }
+                sp += min(w0, 0);
+                stage(node, k);
+                if (w0 > 0) {   // the other children go to the stack
+                    while (sp + w0 > WALK_SSTACK) {   // up to half of it spills to global memory, oldest first (w0 < WALK_SSTACK)
+                        const int m = min(sp, WALK_SSTACK / 2);
+                        if (gsp + m > p.stack_cap) {
+                            overflow = true;
+                            break;
+                        }
+                        for (int i = lane; i < m; i += 32) gstack[gsp + i] = sstack[i];
+                        __syncwarp();
+                        for (int i = lane; i < sp - m; i += 32) sstack[i] = sstack[m + i];   // sp - m <= m: no overlap
+                        __syncwarp();
+                        gsp += m;
+                        sp -= m;
+                    }
+                    if (overflow) break;
+                    for (int w = 0; w < w0; w += 32) {
+                        const int c = expand(cbase, cbeg, cfin, w);
+                        if (w + lane < w0) sstack[sp + w + lane] = c;
+                    }
+                    sp += w0;
+                }
+                __syncwarp();   // stack and queued runs are read by other lanes next
+            } else if (!batch) {
+                if (limit == 1) break;
+                // the traversal is over: the lists' last, partial quanta are filled with massless entries
+                const int fe = (nf + QUANTUM - 1) & ~(QUANTUM - 1), ne = (nn + QUANTUM - 1) & ~(QUANTUM - 1);
+                __syncwarp();
+                if (nf + lane < fe) list_put(far, nf + lane, PAD_ENTRY);
+                if (nn + lane < ne) near_put(near, nn + lane, PAD_ENTRY, PAD_SOFT);
+                nf = fe;
+                nn = ne;
+                limit = nlimit = 1;
+                continue;
+            }
+            if (batch) {   // the batch's particles are classified against the group box
+                bool use = false, pfar = false;
+                float4 pe = make_float4(0.f, 0.f, 0.f, 0.f);
+                float ph = 0.f;
+                if (have) {
                     const float dx = (float)(pp.x - cg[0]), dy = (float)(pp.y - cg[1]), dz = (float)(pp.z - cg[2]);
                     const float ex = fmaxf(fabsf(dx) - hwf[0], 0.f), ey = fmaxf(fabsf(dy) - hwf[1], 0.f),
                                 ez = fmaxf(fabsf(dz) - hwf[2], 0.f);
@@ -565,204 +904,11 @@ __global__ void __launch_bounds__(WALK_THREADS, MINB) k_walk(WalkParams p)
                     const float hh = fmaxf(hmax, pp.h);
                     pe = make_float4(dx, dy, dz, pp.m);
                     ph = pp.h;
-                    use = true;
+                    use = pp.m > 0.f;
                     pfar = (r2 >= hh * hh) && (r2 > FAR_MIN_R2);
                 }
+                append(use, pfar, pe, ph);
             }
-            qn -= m;
-            const unsigned mf = __ballot_sync(FULL, use && pfar);   // also orders the queue reads before reuse
-            const unsigned mn = __ballot_sync(FULL, use && !pfar);
-            if (use) {
-                if (pfar) list_put(far, nf + __popc(mf & lt_mask), pe);
-                else {
-                    const int pos = nn + __popc(mn & lt_mask);
-                    list_put(nearE, pos, pe);
-                    list_put(nearH, pos, near_soft(ph, pe.w, homog, hmax));
-                }
-            }
-            nf += __popc(mf);
-            nn += __popc(mn);
-            list_far += __popc(mf);
-            list_near += __popc(mn);
-            if (nf >= FL) { flush_far<TPL, POT>(far, nf, T); nf = 0; }
-            if (nn >= FL) { flush_near_sel<TPL, POT>(homog, nearE, nearH, nn, T); nn = 0; }
-            __syncwarp();
-        };
-        int node = -1;
-        int k = pop_nodes(node);
-        if (tma) {
-            if (k > 0) stage_nodes(bar, slot0, p.nodes, node, k, lane);   // one barrier phase per staged round
-        } else if (lane < k) {
-            stage_node(nslot, p.nodes + node);
-        }
-        bool timed_out = false;
-        while (k > 0) {
-            tested += k;
-            if (tma) {
-                if (!bar_wait(bar, phase)) {
-                    timed_out = true;
-                    break;
-                }
-                phase ^= 1u;
-            } else {
-                asm volatile("cp.async.wait_all;" ::: "memory");
-            }
-
-            int act = 0, na = 0, nb = 0;
-            bool isfar = false;
-            float4 ent = make_float4(0.f, 0.f, 0.f, 0.f);
-            float hp = 0.f;
-            if (lane < k) {
-                GGNode nd;
-#pragma unroll
-                for (int i = 0; i < 4; i++) reinterpret_cast<int4 *>(&nd)[i] = nslot[i];
-                na = nd.a;
-                nb = nd.b;
-                if (nd.mass > 0.f) {
-                    if (nb == -1) {
-                        act = 3;
-                    } else if (!F64T) {
-                        const float dx = (float)(nd.cx - cg[0]), dy = (float)(nd.cy - cg[1]), dz = (float)(nd.cz - cg[2]);
-                        const float ex = fmaxf(fabsf(dx) - hwf[0], 0.f), ey = fmaxf(fabsf(dy) - hwf[1], 0.f),
-                                    ez = fmaxf(fabsf(dz) - hwf[2], 0.f);
-                        const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-                        const float ms = nd.maxsoft, L = nd.len;
-                        bool open = (hmin < ms) && (r2 < ms * ms);
-                        if (!open) {
-                            if (thetaf > 0.f) {
-                                open = L * L > r2 * thetaf * thetaf;
-                            } else {
-                                const float a1 = fmaf(0.6f, L, hmax), a2 = fmaf(0.6f, L, ms);
-                                open = (r2 < a1 * a1) || (r2 < a2 * a2) || (nd.mass * L * L > r2 * r2 * aoldf);
-                                if (!open)
-                                    open = (fabsf(dx + nd.gx) < fmaf(0.6f, L, hwf[0])) &&
-                                           (fabsf(dy + nd.gy) < fmaf(0.6f, L, hwf[1])) &&
-                                           (fabsf(dz + nd.gz) < fmaf(0.6f, L, hwf[2]));
-                            }
-                        }
-                        if (open) {
-                            act = (nb > 0) ? 2 : 3;
-                        } else {
-                            act = 1;
-                            ent = make_float4(dx, dy, dz, nd.mass);
-                            hp = ms;
-                            const float hh = fmaxf(hmax, ms);
-                            isfar = (r2 >= hh * hh) && (r2 > FAR_MIN_R2);
-                        }
-                    } else {
-                        double dx = nd.cx - cg[0], dy = nd.cy - cg[1], dz = nd.cz - cg[2];
-                        double ex = fmax(fabs(dx) - hw[0], 0.0), ey = fmax(fabs(dy) - hw[1], 0.0),
-                               ez = fmax(fabs(dz) - hw[2], 0.0);
-                        double r2 = ex * ex + ey * ey + ez * ez;
-                        double ms = (double)nd.maxsoft, L = (double)nd.len;
-                        bool open = (hmind < ms) && (r2 < ms * ms);
-                        if (!open) {
-                            if (theta > 0.0) {
-                                open = L * L > r2 * theta * theta;
-                            } else {
-                                double a1 = hmaxd + 0.6 * L, a2 = ms + 0.6 * L;
-                                open = (r2 < a1 * a1) || (r2 < a2 * a2) || ((double)nd.mass * L * L > r2 * r2 * aold_min);
-                                if (!open) {
-                                    double gx = fabs(dx + (double)nd.gx), gy = fabs(dy + (double)nd.gy),
-                                           gz = fabs(dz + (double)nd.gz);
-                                    open = (gx < 0.6 * L + hw[0]) && (gy < 0.6 * L + hw[1]) && (gz < 0.6 * L + hw[2]);
-                                }
-                            }
-                        }
-                        if (open) {
-                            act = (nb > 0) ? 2 : 3;
-                        } else {
-                            act = 1;
-                            ent = make_float4((float)dx, (float)dy, (float)dz, nd.mass);
-                            hp = nd.maxsoft;
-                            double hh = fmax(hmaxd, ms);
-                            isfar = (r2 >= hh * hh) && (r2 > (double)FAR_MIN_R2);
-                        }
-                    }
-                }
-            }
-            // used nodes -> lists
-            {
-                unsigned mf = __ballot_sync(FULL, act == 1 && isfar);
-                unsigned mn = __ballot_sync(FULL, act == 1 && !isfar);
-                if (act == 1) {
-                    if (isfar) list_put(far, nf + __popc(mf & lt_mask), ent);
-                    else {
-                        int pos = nn + __popc(mn & lt_mask);
-                        list_put(nearE, pos, ent);
-                        list_put(nearH, pos, near_soft(hp, ent.w, homog, hmax));
-                    }
-                }
-                nf += __popc(mf);
-                nn += __popc(mn);
-                list_far += __popc(mf);
-                list_near += __popc(mn);
-            }
-            // opened internal nodes -> children on the stack (spilling its
-            // bottom half to global memory when it would overflow)
-            {
-                const int nch = (act == 2) ? nb : 0;   // 1..8 children
-                int total;
-                const int ex = warp_excl_bits<4>(nch, lt_mask, &total);
-                if (sp + total > WALK_SSTACK) {
-                    const int m = WALK_SSTACK / 2;
-                    if (gsp + m > p.stack_cap) {
-                        overflow = true;
-                        break;
-                    }
-                    for (int i = lane; i < m; i += 32) gstack[gsp + i] = sstack[i];
-                    __syncwarp();
-                    for (int i = lane; i < sp - m; i += 32) sstack[i] = sstack[m + i];   // sp - m <= m: no overlap
-                    __syncwarp();
-                    gsp += m;
-                    sp -= m;
-                }
-                const int o = sp + ex;
-                for (int c = 0; c < nch; c++) sstack[o + c] = na + c;
-                sp += total;
-                __syncwarp();
-            }
-            // next round's node records are staged now; the copies complete behind
-            // this round's flushes and leaf particles
-            int next_node = -1;
-            const int next_k = pop_nodes(next_node);
-            if (tma) {
-                if (next_k > 0) stage_nodes(bar, slot0, p.nodes, next_node, next_k, lane);
-            } else if (lane < next_k) {
-                stage_node(nslot, p.nodes + next_node);
-            }
-            if (nf >= FL) { flush_far<TPL, POT>(far, nf, T); nf = 0; }
-            if (nn >= FL) { flush_near_sel<TPL, POT>(homog, nearE, nearH, nn, T); nn = 0; }
-            // opened leaves -> their particles onto the particle queue, which
-            // is evaluated 32 particles at a time (leftovers wait for later
-            // rounds).  A push that does not fit is taken in parts, the queue
-            // drained between them.
-            {
-                int first = na, rem = (act == 3) ? -nb : 0;
-                while (__any_sync(FULL, rem > 0)) {
-                    int P, ex;
-                    const unsigned big = __ballot_sync(FULL, rem >= 16);
-                    if (!big) {
-                        ex = warp_excl_bits<4>(rem, lt_mask, &P);   // leaves of up to 15 particles
-                    } else if (!__any_sync(FULL, rem >= 64)) {
-                        ex = warp_excl_bits<6>(rem, lt_mask, &P);
-                    } else {
-                        const int incl = warp_incl_scan(rem, lane);
-                        P = __shfl_sync(FULL, incl, 31);
-                        ex = incl - rem;
-                    }
-                    const int room = PQ_CAP - qn;
-                    const int take = min(max(room - ex, 0), rem);
-                    for (int c = 0; c < take; c++) pq[qn + ex + c] = first + c;
-                    qn += min(P, room);
-                    first += take;
-                    rem -= take;
-                    __syncwarp();
-                    while (qn >= 32) take_particles(32);
-                }
-            }
-            k = next_k;
-            node = next_node;
         }
         if (!tma) asm volatile("cp.async.wait_all;" ::: "memory");   // no copy into the slot outlives its group
         if (timed_out) {   // copies may still be in flight: wait once more, then leave
@@ -771,12 +917,16 @@ __global__ void __launch_bounds__(WALK_THREADS, MINB) k_walk(WalkParams p)
             return;
         }
         if (overflow) {
+            if (tma && !bar_wait(bar, phase)) {   // the copies staged for a round that will not run
+                if (lane == 0) atomicOr(p.err, GG_EBIT_WALK_TIMEOUT);
+                return;
+            }
+            if (tma) phase ^= 1u;
             if (lane == 0) atomicOr(p.err, GG_EBIT_STACK_OVERFLOW);
+            __syncwarp();
             continue;
         }
-        if (qn > 0) take_particles(qn);
-        if (nf > 0) flush_far<TPL, POT>(far, nf, T);
-        if (nn > 0) flush_near_sel<TPL, POT>(homog, nearE, nearH, nn, T);
+        __syncwarp();   // the next group's entries overwrite the lists
 
         // ---- results
         // this group's device cycles per target: the cost the next walk orders its groups by
@@ -784,8 +934,23 @@ __global__ void __launch_bounds__(WALK_THREADS, MINB) k_walk(WalkParams p)
         int mycount = 0;
 #pragma unroll
         for (int s = 0; s < TPL; s++) {
-            if (!T.valid[s]) continue;
-            int t = grp.first + s * 32 + lane;
+            double ax = 0.0, ay = 0.0, az = 0.0;
+            if (!POT) { ax = T.ax[s].value(); ay = T.ay[s].value(); az = T.az[s].value(); }
+            double ph = T.pot[s].value();
+            int self = T.self[s];
+#pragma unroll
+            for (int o = LP; o < 32; o <<= 1) {   // the parts' shares of the lists
+                if (!POT) {
+                    ax += __shfl_xor_sync(FULL, ax, o);
+                    ay += __shfl_xor_sync(FULL, ay, o);
+                    az += __shfl_xor_sync(FULL, az, o);
+                }
+                ph += __shfl_xor_sync(FULL, ph, o);
+                self += __shfl_xor_sync(FULL, self, o);
+            }
+            if (!T.valid[s] || (SPLIT > 1 && part != s)) continue;   // part s writes target s
+            const int nint = list_far + list_near - self;
+            int t = grp.first + s * LP + lane % LP;
             int pi = tpi[s];
             unsigned li = p.perm[pi];
             int o = p.tout ? p.tout[t] : (int)li;
@@ -793,18 +958,17 @@ __global__ void __launch_bounds__(WALK_THREADS, MINB) k_walk(WalkParams p)
                 // compute_potential removes the self term m_i kernel(0) / h_i
                 // (potential.c:137-145); subtract the FP32 value the walk added
                 const float mi = p.parts[pi].m;
-                p.pot[o] = T.pot[s].value() - (double)((mi * -2.8f) * T.hinv[s]);
+                p.pot[o] = ph - (double)((mi * -2.8f) * T.hinv[s]);
             } else {
-                double ax = T.ax[s].value(), ay = T.ay[s].value(), az = T.az[s].value();
                 p.acc[3 * (size_t)o] = ax;
                 p.acc[3 * (size_t)o + 1] = ay;
                 p.acc[3 * (size_t)o + 2] = az;
-                if (p.pot) p.pot[o] = T.pot[s].value();
+                if (p.pot) p.pot[o] = ph;
                 if (p.oldacc_out) p.oldacc_out[li] = sqrt(ax * ax + ay * ay + az * az);
             }
-            if (p.ninter) p.ninter[o] = T.nint[s];
+            if (p.ninter) p.ninter[o] = nint;
             if (p.cost_out) p.cost_out[li] = tcost;
-            mycount += T.nint[s];
+            mycount += nint;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mycount += __shfl_xor_sync(FULL, mycount, o);
@@ -817,42 +981,32 @@ __global__ void __launch_bounds__(WALK_THREADS, MINB) k_walk(WalkParams p)
     }
 }
 
-template <int TPL, int MINB, bool F64T, bool POT = false, bool TMA = false>
-static void launch_walk_t(const WalkParams &p, int blocks, int smem, cudaStream_t st)
+template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA>
+static void launch_walk_t(const WalkParams &p, int blocks, cudaStream_t st)
 {
-    cudaFuncSetAttribute(k_walk<TPL, MINB, F64T, POT, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_walk<TPL, MINB, F64T, POT, TMA><<<blocks, WALK_THREADS, smem, st>>>(p);
+    const int smem = WALK_WARPS * WALK_WARP_FLOATS * (int)sizeof(float);
+    cudaFuncSetAttribute(k_walk<TPL, SPLIT, F64T, POT, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_walk<TPL, SPLIT, F64T, POT, TMA><<<blocks, WALK_THREADS, smem, st>>>(p);
 }
 
-// blocks_per_sm selects the register budget of the instantiation (1..3) and
-// the persistent grid is that many blocks per SM
-void gg_launch_walk(const WalkParams &p, int tpl, int blocks_per_sm, cudaStream_t st)
+// The persistent grid is blocks_per_sm (1..3) blocks per SM, of which two are
+// resident at a time (registers and shared memory).
+void gg_launch_walk(const WalkParams &p, int blocks_per_sm, cudaStream_t st)
 {
-    int smem = gg_walk_smem_bytes(p.flush, tpl);
-    int minb = blocks_per_sm < 1 ? 1 : (blocks_per_sm > 3 ? 3 : blocks_per_sm);
-    int blocks = gg_num_sms() * blocks_per_sm;
-    if (p.pot_only) {   // the potential-only walk: one register budget per mode
-        if (p.group_size == 1) launch_walk_t<1, 2, true, true>(p, blocks, smem, st);
-        else if (tpl == 2) launch_walk_t<2, 2, false, true>(p, blocks, smem, st);
-        else launch_walk_t<1, 2, false, true>(p, blocks, smem, st);
-    } else if (p.group_size == 1) {
-        launch_walk_t<1, 2, true>(p, blocks, smem, st);   // exact mode: the reference's tests
-    } else if (p.node_staging == 1) {   // bulk-copy node staging (the force walk's tuned forms)
-        if (tpl == 2) {
-            if (minb == 3) launch_walk_t<2, 3, false, false, true>(p, blocks, smem, st);
-            else launch_walk_t<2, 2, false, false, true>(p, blocks, smem, st);
-        } else {
-            if (minb == 3) launch_walk_t<1, 3, false, false, true>(p, blocks, smem, st);
-            else launch_walk_t<1, 2, false, false, true>(p, blocks, smem, st);
-        }
-    } else if (tpl == 2) {
-        if (minb == 1) launch_walk_t<2, 1, false>(p, blocks, smem, st);
-        else if (minb == 2) launch_walk_t<2, 2, false>(p, blocks, smem, st);
-        else launch_walk_t<2, 3, false>(p, blocks, smem, st);
+    const int blocks = gg_num_sms() * blocks_per_sm;
+    const bool wide = p.group_size > 32, bulk = p.node_staging == 1;
+    if (p.group_size == 1) {   // exact mode: the reference's tests
+        if (p.pot_only) launch_walk_t<1, 1, true, true, false>(p, blocks, st);
+        else launch_walk_t<1, 1, true, false, false>(p, blocks, st);
+    } else if (p.pot_only) {
+        if (wide) launch_walk_t<2, 1, false, true, false>(p, blocks, st);
+        else launch_walk_t<2, 2, false, true, false>(p, blocks, st);
+    } else if (bulk) {
+        if (wide) launch_walk_t<2, 1, false, false, true>(p, blocks, st);
+        else launch_walk_t<2, 2, false, false, true>(p, blocks, st);
     } else {
-        if (minb == 1) launch_walk_t<1, 1, false>(p, blocks, smem, st);
-        else if (minb == 2) launch_walk_t<1, 2, false>(p, blocks, smem, st);
-        else launch_walk_t<1, 3, false>(p, blocks, smem, st);
+        if (wide) launch_walk_t<2, 1, false, false, false>(p, blocks, st);
+        else launch_walk_t<2, 2, false, false, false>(p, blocks, st);
     }
     gg_note_launches(1);
 }
