@@ -4,7 +4,7 @@
 // (mysort_peano, system/peano.c:414-462; mysort_domain, domain.c:2674-2723).
 // Design (one-sweep): one up-front pass builds the digit histograms of every
 // pass; each pass is then a single kernel in which a CTA ranks a tile of
-// SORT_TILE keys in shared memory, publishes its per-digit counts, sums its
+// keys in shared memory, publishes its per-digit counts, sums its
 // predecessors' counts with a decoupled look-back, and writes the tile out
 // digit-sorted so that global stores are contiguous runs.  SORT_BITS-bit
 // digits (8: the 63-bit Peano-Hilbert keys take 8 passes).  For several
@@ -42,8 +42,16 @@
 #endif
 
 #define SORT_THREADS 256
-#define SORT_ITEMS GG_SORT_ITEMS
-#define SORT_TILE (SORT_THREADS * SORT_ITEMS)
+// Tiles of 2560 keys fill the GPU (592 resident blocks) from about 1.5M pairs
+// on.  Below that a pass lasts as long as one tile's chain of load, rank, look
+// back and scatter, so up to SMALL_MAX_N pairs are sorted in tiles of 512: a
+// fifth of the items to rank one after the other, five times the blocks.  A
+// build's sort, tiles of 2560 -> 512 keys: 1,000 pairs 85 -> 67 us, 65,536 121 ->
+// 83 us, 262,144 143 -> 139 us; at 303,104 pairs the small tiles fill the GPU once.
+#define SMALL_ITEMS 2
+#define SMALL_TILE (SORT_THREADS * SMALL_ITEMS)
+#define SMALL_MAX_N (SMALL_TILE * 592)
+#define LARGE_TILE (SORT_THREADS * GG_SORT_ITEMS)
 #define SORT_WARPS (SORT_THREADS / 32)
 #define SORT_BITS GG_SORT_BITS
 #define RADIX (1 << SORT_BITS)
@@ -143,10 +151,11 @@ __device__ __forceinline__ void st_status(unsigned *p, unsigned v)
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+template <int TILE>
 struct SortSmem {
-    unsigned long long keys[SORT_TILE];
-    unsigned vals[SORT_TILE];
-    unsigned short dig[SORT_TILE];
+    unsigned long long keys[TILE];
+    unsigned vals[TILE];
+    unsigned short dig[TILE];
     unsigned whist[SORT_WARPS][RADIX];
     unsigned bhist[RADIX];   // the tile's digit counts, published before the ranking
     unsigned texcl[RADIX];
@@ -160,15 +169,16 @@ struct SortSmem {
 // this tile clears its own (nullptr for the last pass).  GATHER (the last pass
 // of a build's sort): each pair's value is a record index, and the pass also
 // moves that record to the pair's sorted position and records the position.
-template <bool GATHER>
+template <bool GATHER, int SORT_ITEMS>
 __global__ void __launch_bounds__(SORT_THREADS, GG_SORT_MINB) k_sort_pass(
     const unsigned long long *__restrict__ kin, const unsigned *__restrict__ vin, unsigned long long *__restrict__ kout,
     unsigned *__restrict__ vout, int n, int shift, int sys_mode, const int *__restrict__ poff, int S,
     const unsigned *__restrict__ g_off, unsigned *status, unsigned *status_next, unsigned *tile_counter, int *err,
     SortGather gather)
 {
+    constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;
     extern __shared__ __align__(16) unsigned char sort_smem_raw[];
-    SortSmem &sm = *reinterpret_cast<SortSmem *>(sort_smem_raw);
+    SortSmem<SORT_TILE> &sm = *reinterpret_cast<SortSmem<SORT_TILE> *>(sort_smem_raw);
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (tid == 0) sm.tile = (int)atomicAdd(tile_counter, 1u);
@@ -336,7 +346,9 @@ static int sort_passes(int bits) { return bits <= 0 ? 0 : (bits + SORT_BITS - 1)
 // GG_SORT_MAX_PASSES), so that one buffer serves every sort of up to n pairs.
 size_t gg_sort_scratch_bytes(long long n)
 {
-    const long long ntiles = (n + SORT_TILE - 1) / SORT_TILE;
+    // a smaller sort may have more (small) tiles than a larger one
+    const long long small = (std::min(n, (long long)SMALL_MAX_N) + SMALL_TILE - 1) / SMALL_TILE;
+    const long long ntiles = std::max(small, (n + LARGE_TILE - 1) / LARGE_TILE);
     size_t b = 0;
     b += (size_t)n * 8 + 256;                                // alternate keys
     b += (size_t)n * 4 + 256;                                // alternate values
@@ -346,7 +358,21 @@ size_t gg_sort_scratch_bytes(long long n)
     return b;
 }
 
-static int sort_smem_bytes() { return (int)sizeof(SortSmem); }
+template <bool GATHER, int ITEMS>
+static gg_status launch_pass(long long ntiles, const unsigned long long *ka, const unsigned *va, unsigned long long *kb,
+                             unsigned *vb, int n, int shift, int sys_mode, const int *poff, int S, const unsigned *off,
+                             unsigned *status, unsigned *status_next, unsigned *counter, int *err,
+                             const SortGather &gather, cudaStream_t st)
+{
+    const int smem = (int)sizeof(SortSmem<SORT_THREADS * ITEMS>);
+    // the attribute is per device: set it on every call (cheap)
+    GG_CUDA_TRY(cudaFuncSetAttribute(k_sort_pass<GATHER, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_sort_pass<GATHER, ITEMS><<<(unsigned)ntiles, SORT_THREADS, smem, st>>>(ka, va, kb, vb, n, shift, sys_mode, poff, S,
+                                                                             off, status, status_next, counter, err,
+                                                                             gather);
+    gg_note_launches(1);
+    return GG_OK;
+}
 
 // Sorts (keys, vals) of length n by the low key_bits bits of the key, then
 // stably by the low sys_bits bits of each value's system id (the system whose
@@ -361,7 +387,9 @@ gg_status gg_sort_pairs_run(unsigned long long *keys, unsigned *vals, long long 
     const int nkey = sort_passes(key_bits), nsys = sort_passes(sys_bits), np = nkey + nsys;
     if (np <= 0 || n <= 1) return GG_OK;
     if (np > GG_SORT_MAX_PASSES || n >= (1ll << 30)) return GG_ERR_TOO_LARGE;
-    const long long ntiles = (n + SORT_TILE - 1) / SORT_TILE;
+    const bool small = n <= SMALL_MAX_N;
+    const int tile = small ? SMALL_TILE : LARGE_TILE;
+    const long long ntiles = (n + tile - 1) / tile;
     char *p = (char *)scratch;
     auto take = [&](size_t bytes) {
         char *r = p;
@@ -370,14 +398,14 @@ gg_status gg_sort_pairs_run(unsigned long long *keys, unsigned *vals, long long 
     };
     unsigned long long *kalt = (unsigned long long *)take((size_t)n * 8);
     unsigned *valt = (unsigned *)take((size_t)n * 4);
-    unsigned *hist = (unsigned *)take((size_t)np * RADIX * 4);
     unsigned *off = (unsigned *)take((size_t)np * RADIX * 4);
+    // cleared together
+    unsigned *hist = (unsigned *)take((size_t)np * RADIX * 4);
     unsigned *counters = (unsigned *)take(256);
-    unsigned *status[2] = {(unsigned *)take((size_t)ntiles * RADIX * 4), (unsigned *)take((size_t)ntiles * RADIX * 4)};
-
-    GG_CUDA_TRY(cudaMemsetAsync(hist, 0, (size_t)np * RADIX * 4, st));
-    GG_CUDA_TRY(cudaMemsetAsync(counters, 0, 256, st));
-    GG_CUDA_TRY(cudaMemsetAsync(status[0], 0, (size_t)ntiles * RADIX * 4, st));
+    unsigned *status[2] = {(unsigned *)take((size_t)ntiles * RADIX * 4), nullptr};
+    const size_t cleared = (size_t)(p - (char *)hist);
+    status[1] = (unsigned *)take((size_t)ntiles * RADIX * 4);
+    GG_CUDA_TRY(cudaMemsetAsync(hist, 0, cleared, st));
     {
         int threads = 256, blocks = gg_num_sms() * 4;
         const long long need = (n + threads - 1) / threads;
@@ -388,27 +416,19 @@ gg_status gg_sort_pairs_run(unsigned long long *keys, unsigned *vals, long long 
         k_sort_hist_scan<<<np, SORT_THREADS, 0, st>>>(hist, off);
         gg_note_launches(2);
     }
-    // the attribute is per device: set it on every call (cheap)
-    GG_CUDA_TRY(cudaFuncSetAttribute(k_sort_pass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_smem_bytes()));
-    if (gather) {
-        GG_CUDA_TRY(cudaFuncSetAttribute(k_sort_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         sort_smem_bytes()));
-    }
     const SortGather none = {nullptr, nullptr, nullptr};
     unsigned long long *ka = keys, *kb = kalt;
     unsigned *va = vals, *vb = valt;
     for (int pass = 0; pass < np; pass++) {
         const int sys_mode = pass >= nkey;
         const int shift = sys_mode ? SORT_BITS * (pass - nkey) : SORT_BITS * pass;
-        if (gather && pass == np - 1)
-            k_sort_pass<true><<<(unsigned)ntiles, SORT_THREADS, sort_smem_bytes(), st>>>(
-                ka, va, kb, vb, (int)n, shift, sys_mode, poff, S, off + pass * RADIX, status[pass & 1], nullptr,
-                counters + pass, err, *gather);
-        else
-            k_sort_pass<false><<<(unsigned)ntiles, SORT_THREADS, sort_smem_bytes(), st>>>(
-                ka, va, kb, vb, (int)n, shift, sys_mode, poff, S, off + pass * RADIX, status[pass & 1],
-                pass + 1 < np ? status[(pass + 1) & 1] : nullptr, counters + pass, err, none);
-        gg_note_launches(1);
+        const bool last = pass == np - 1, move = gather && last;
+        const auto launch = move ? (small ? launch_pass<true, SMALL_ITEMS> : launch_pass<true, GG_SORT_ITEMS>)
+                                 : (small ? launch_pass<false, SMALL_ITEMS> : launch_pass<false, GG_SORT_ITEMS>);
+        const gg_status e = launch(ntiles, ka, va, kb, vb, (int)n, shift, sys_mode, poff, S, off + pass * RADIX,
+                                   status[pass & 1], last ? nullptr : status[(pass + 1) & 1], counters + pass, err,
+                                   move ? *gather : none, st);
+        if (e) return e;
         unsigned long long *tk = ka; ka = kb; kb = tk;
         unsigned *tv = va; va = vb; vb = tv;
     }
@@ -428,7 +448,7 @@ gg_status gg_sort_pairs_run(unsigned long long *keys, unsigned *vals, long long 
 // completed (it cannot), or a CUDA error.
 gg_status gg_sort_timeout_selftest(cudaStream_t st)
 {
-    const int n = 2 * SORT_TILE;
+    const int n = 2 * LARGE_TILE;
     char *base = nullptr;
     const size_t bytes = (size_t)n * 24 + 2 * RADIX * 4 + RADIX * 4 + 4096;
     GG_CUDA_TRY(cudaMallocAsync((void **)&base, bytes, st));
@@ -445,11 +465,9 @@ gg_status gg_sort_timeout_selftest(cudaStream_t st)
     cudaMemsetAsync(base, 0, (size_t)(p - base), st);
     const unsigned one = 1;   // the CTA takes tile 1; tile 0 is never started
     cudaMemcpyAsync(counter, &one, sizeof one, cudaMemcpyHostToDevice, st);
-    cudaFuncSetAttribute(k_sort_pass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sort_smem_bytes());
     const SortGather none = {nullptr, nullptr, nullptr};
-    k_sort_pass<false><<<1, SORT_THREADS, sort_smem_bytes(), st>>>(kin, vin, kout, vout, n, 0, 0, nullptr, 1, off, status,
-                                                             nullptr, counter, err, none);
-    gg_note_launches(1);
+    launch_pass<false, GG_SORT_ITEMS>(1, kin, vin, kout, vout, n, 0, 0, nullptr, 1, off, status, nullptr, counter, err,
+                                      none, st);
     int herr = 0;
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof herr, cudaMemcpyDeviceToHost, st);
