@@ -513,7 +513,7 @@ static gg_status set_systems(gg_ctx *c, int S, const int64_t *counts)
     if ((st = c->poff.ensure(S + 1))) return st;
     GG_CUDA_TRY(cudaMemcpyAsync(c->poff.p, poff.data(), (S + 1) * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     if ((st = c->in_rec.ensure(N)) || (st = c->part.ensure(N)) || (st = c->dom.ensure(S)) ||
-        (st = c->extent_mm.ensure((size_t)S * 6)) || (st = c->hmm.ensure((size_t)S * 2)) || (st = c->keys.ensure(N)) || (st = c->perm.ensure(N)) ||
+        (st = c->extent_mm.ensure(gg_extent_words(S))) || (st = c->hmm.ensure((size_t)S * 2)) || (st = c->keys.ensure(N)) || (st = c->perm.ensure(N)) ||
         (st = c->rank.ensure(N)) || (st = c->oldacc.ensure(N)))
         return st;
     return GG_OK;

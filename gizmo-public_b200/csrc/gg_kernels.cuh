@@ -17,6 +17,7 @@ struct TreeBuf {
     int *err;
 };
 
+size_t gg_extent_words(int S);   // 64-bit words of gg_launch_extent's scratch mm
 void gg_launch_extent(const GGPart *rec, int n, const int *poff, int S, unsigned long long *mm, unsigned *hmm,
                       GGDomainDev *dom, int *err, cudaStream_t st);
 void gg_launch_keys(const GGPart *rec, int n, const int *poff, int S, const GGDomainDev *dom,

@@ -6,6 +6,8 @@
 // then the Peano-Hilbert key (system/peano.c:303-319).  At 21 bits the key is
 // exactly the reference's 42-bit key shifted right by 63 bits, because the
 // reference's key is built most-significant level first.
+#include <algorithm>
+
 #include "gg_internal.cuh"
 #include "gg_ph_table.h"
 #include "gg_kernels.cuh"
@@ -21,29 +23,50 @@ __device__ __forceinline__ int gg_sys_of(const int *__restrict__ poff, int S, in
     return lo;
 }
 
-__global__ void k_extent_init(unsigned long long *mm, unsigned *hmm, int S)
+// Root cube of one system from its min/max, with the reference's expressions.
+__device__ __forceinline__ GGDomainDev extent_domain(const unsigned long long *mm)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < S * 6) mm[t] = (t % 6) < 3 ? ~0ull : 0ull;   // [min x,y,z | max x,y,z] in ordered encoding
-    if (hmm && t < S * 2) hmm[t] = (t & 1) ? 0u : 0x7f800000u;
+    double mn[3], mx[3], len = 0;
+    for (int k = 0; k < 3; k++) {
+        mn[k] = gg_ordered_to_dbl(~__ldcg(mm + k));
+        mx[k] = gg_ordered_to_dbl(__ldcg(mm + 3 + k));
+        if (!(mn[k] <= mx[k])) { mn[k] = 0; mx[k] = 0; }   // empty system
+    }
+    for (int k = 0; k < 3; k++) {
+        double e = __dsub_rn(mx[k], mn[k]);
+        if (e > len) len = e;
+    }
+    len = __dmul_rn(len, 1.001);
+    if (len <= 0) len = 1.0;   // a single particle or empty system: any cube works
+    GGDomainDev d;
+    for (int k = 0; k < 3; k++) {
+        double mid = __dmul_rn(0.5, __dadd_rn(mn[k], mx[k]));
+        d.center[k] = mid;
+        d.corner[k] = __dsub_rn(mid, __dmul_rn(0.5, len));
+    }
+    d.len = len;
+    d.pad = 0;
+    return d;
 }
 
 // Each warp reduces a contiguous chunk of particles, reading it coalesced
 // (lane l takes every 32nd record), one system segment at a time, and flushes
-// the segment's min/max with 64-bit atomics on an order-preserving encoding:
-// order-independent, so the result is exact and deterministic.  The per-system
-// range of kernel radii (positive floats, ordered as their bit patterns) goes
-// to hmm[2s], hmm[2s+1].
-#define EXTENT_CHUNK 4096
-__global__ void k_extent(const GGPart *__restrict__ rec, int n, const int *__restrict__ poff, int S,
-                         unsigned long long *mm, unsigned *hmm, int *err)
+// the segment's extremes with 64-bit atomics on an order-preserving encoding:
+// order-independent, so the result is exact and deterministic.  mm[8 s ..]:
+// system s's complemented min x, y, z, max x, y, z, complemented min h and max h
+// (kernel radii are not negative: their bit patterns are ordered), all from
+// zero, so that one memset prepares every one.  The block that finishes last
+// (`done` counts them) forms the root cubes and the ranges of kernel radii: one
+// launch instead of three.
+__global__ void k_extent(const GGPart *__restrict__ rec, int n, const int *__restrict__ poff, int S, int chunk,
+                         unsigned long long *mm, unsigned *done, unsigned *hmm, GGDomainDev *dom, int *err)
 {
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     bool bad = false;
-    for (long long c0 = (long long)warp * EXTENT_CHUNK; c0 < n; c0 += (long long)nwarps * EXTENT_CHUNK) {
-        const int cb = (int)c0, ce = (int)min((long long)n, c0 + EXTENT_CHUNK);
+    for (long long c0 = (long long)warp * chunk; c0 < n; c0 += (long long)nwarps * chunk) {
+        const int cb = (int)c0, ce = (int)min((long long)n, c0 + chunk);
         int s = gg_sys_of(poff, S, cb);
         for (int seg = cb; seg < ce; s++) {
             const int se = min(ce, __ldg(poff + s + 1));
@@ -71,48 +94,31 @@ __global__ void k_extent(const GGPart *__restrict__ rec, int n, const int *__res
                 hmin = fminf(hmin, __shfl_xor_sync(0xffffffffu, hmin, o));
                 hmax = fmaxf(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
             }
-            if (lane == 0 && se > seg) {
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    atomicMin(&mm[s * 6 + k], gg_dbl_to_ordered(mn[k]));
-                    atomicMax(&mm[s * 6 + 3 + k], gg_dbl_to_ordered(mx[k]));
-                }
-                if (hmm) {
-                    atomicMin(&hmm[2 * s], __float_as_uint(fmaxf(hmin, 0.f)));
-                    atomicMax(&hmm[2 * s + 1], __float_as_uint(fmaxf(hmax, 0.f)));
-                }
+            if (lane < 8 && se > seg) {   // one of the eight extremes each
+                unsigned long long v;
+                if (lane < 3) v = ~gg_dbl_to_ordered(lane == 0 ? mn[0] : lane == 1 ? mn[1] : mn[2]);
+                else if (lane < 6) v = gg_dbl_to_ordered(lane == 3 ? mx[0] : lane == 4 ? mx[1] : mx[2]);
+                else if (lane == 6) v = ~(unsigned long long)__float_as_uint(fmaxf(hmin, 0.f));
+                else v = __float_as_uint(fmaxf(hmax, 0.f));
+                atomicMax(mm + 8 * (size_t)s + lane, v);
             }
             seg = se;
         }
     }
     if (bad) atomicOr(err, GG_EBIT_BAD_INPUT);
-}
-
-__global__ void k_extent_finalize(const unsigned long long *mm, int S, GGDomainDev *dom)
-{
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    double mn[3], mx[3], len = 0;
-    for (int k = 0; k < 3; k++) {
-        mn[k] = gg_ordered_to_dbl(mm[s * 6 + k]);
-        mx[k] = gg_ordered_to_dbl(mm[s * 6 + 3 + k]);
-        if (!(mn[k] <= mx[k])) { mn[k] = 0; mx[k] = 0; }   // empty system
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int s = threadIdx.x; s < S; s += blockDim.x) {
+        dom[s] = extent_domain(mm + 8 * (size_t)s);
+        const unsigned long long lo = ~__ldcg(mm + 8 * (size_t)s + 6);
+        hmm[2 * s] = lo >> 32 ? 0x7f800000u : (unsigned)lo;   // infinite for an empty system
+        hmm[2 * s + 1] = (unsigned)__ldcg(mm + 8 * (size_t)s + 7);
     }
-    for (int k = 0; k < 3; k++) {
-        double e = __dsub_rn(mx[k], mn[k]);
-        if (e > len) len = e;
-    }
-    len = __dmul_rn(len, 1.001);
-    if (len <= 0) len = 1.0;   // a single particle or empty system: any cube works
-    GGDomainDev d;
-    for (int k = 0; k < 3; k++) {
-        double mid = __dmul_rn(0.5, __dadd_rn(mn[k], mx[k]));
-        d.center[k] = mid;
-        d.corner[k] = __dsub_rn(mid, __dmul_rn(0.5, len));
-    }
-    d.len = len;
-    d.pad = 0;
-    dom[s] = d;
 }
 
 // 21 levels: the top one from the one-level table, then ten steps of two
@@ -186,17 +192,23 @@ __global__ void k_keys_plain(const double *__restrict__ pos, long long n, GGDoma
     if (bad && err) atomicOr(err, GG_EBIT_BAD_INPUT);
 }
 
+size_t gg_extent_words(int S) { return 8 * (size_t)S + 1; }
+
 void gg_launch_extent(const GGPart *rec, int n, const int *poff, int S, unsigned long long *mm, unsigned *hmm,
                       GGDomainDev *dom, int *err, cudaStream_t st)
 {
-    k_extent_init<<<(S * 6 + 255) / 256, 256, 0, st>>>(mm, hmm, S);
-    int threads = 256, blocks = gg_num_sms() * 4;
-    long long chunks = ((long long)n + EXTENT_CHUNK - 1) / EXTENT_CHUNK;
-    if ((long long)blocks * (threads / 32) > chunks) blocks = (int)((chunks + (threads / 32) - 1) / (threads / 32));
-    if (blocks < 1) blocks = 1;
-    k_extent<<<blocks, threads, 0, st>>>(rec, n, poff, S, mm, hmm, err);
-    k_extent_finalize<<<(S + 127) / 128, 128, 0, st>>>(mm, S, dom);
-    gg_note_launches(3);
+    cudaMemsetAsync(mm, 0, gg_extent_words(S) * sizeof(*mm), st);
+    // particles per warp: small systems spread over the SMs (65,536 particles in
+    // chunks of 4,096 used 16 warps, 39 us; in chunks of 128, 5 us), large ones
+    // flush to the same few words less often
+    int chunk = (n + 2047) / 2048;
+    chunk = chunk < 128 ? 128 : chunk > 4096 ? 4096 : (chunk + 31) & ~31;
+    const int threads = 256;
+    const long long chunks = ((long long)n + chunk - 1) / chunk;
+    const int blocks = (int)std::min((long long)gg_num_sms() * 4, (chunks + threads / 32 - 1) / (threads / 32));
+    k_extent<<<std::max(blocks, 1), threads, 0, st>>>(rec, n, poff, S, chunk, mm, (unsigned *)(mm + 8 * (size_t)S), hmm, dom,
+                                                      err);
+    gg_note_launches(1);
 }
 
 void gg_launch_keys(const GGPart *rec, int n, const int *poff, int S, const GGDomainDev *dom,
