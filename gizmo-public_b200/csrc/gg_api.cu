@@ -245,7 +245,8 @@ struct gg_ctx {
     DevBuf<unsigned> gorder;
     DevBuf<GGGroup> groups;
     DevBuf<int> ngroups, gscan, toff, flag, flagscan, tlist, tout, scan_scratch, active_d;
-    DevBuf<int> g_node, g_flag, g_seg, g_segstart;   // group building scratch
+    DevBuf<int> g_node;                    // group building scratch
+    DevBuf<unsigned> g_stat;
     DevBuf<int> counters;                  // [0] group counter
     DevBuf<unsigned long long> inter;      // interaction total
     DevBuf<int> stack;
@@ -303,7 +304,7 @@ struct gg_ctx {
         f(oldacc); f(vel); f(newpos); f(kin); f(kin_counter); f(dts); f(oldacc_save); f(tcost); f(gkey); f(gorder);
         f(e_chunks); f(e_first); f(e_part); f(e_out);
         f(groups); f(ngroups); f(gscan); f(toff); f(flag); f(flagscan); f(tlist); f(tout); f(scan_scratch);
-        f(g_node); f(g_flag); f(g_seg); f(g_segstart);
+        f(g_node); f(g_stat);
         f(active_d); f(counters); f(inter); f(stack); f(err); f(acc_d); f(pot_d); f(nint_d); f(oldacc_in);
         f(tune_tg); f(tune_rows); f(tune_acc); f(tune_pot); f(tune_mass); f(tune_gacc); f(tune_gpot);
     }
@@ -706,8 +707,7 @@ static gg_status walk_setup(gg_ctx *c)
     if ((st = c->groups.ensure(maxg)) || (st = c->ngroups.ensure(2)) || (st = c->gscan.ensure(c->S + 1)) ||
         (st = c->toff.ensure(c->S + 1)) ||
         (c->cfg.group_size > 1 &&
-         ((st = c->g_node.ensure(c->N + 1)) || (st = c->g_flag.ensure(c->N + 1)) || (st = c->g_seg.ensure(c->N + 1)) ||
-          (st = c->g_segstart.ensure(c->N + 1)))) ||
+         ((st = c->g_node.ensure(c->N + 1)) || (st = c->g_stat.ensure(gg_group_stat_words(c->N))))) ||
         (st = c->stack.ensure((size_t)c->walk_blocks * gg_num_sms() * (gg_walk_threads() / 32) * c->stack_cap)) ||
         (st = c->scan_scratch.ensure(gg_scan_scratch_ints())))
         return st;
@@ -761,15 +761,16 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
         const bool by_soft = c->h_mixed && c->order_by_softening;
         gg_launch_groups_tree(d_active ? n_active : N, tlist, d_active ? c->flagscan.p : nullptr, toff, S,
                               c->cfg.group_size, tree_buf(c), by_soft ? c->dom.p : nullptr, c->hmm.p,
-                              gg_target_order_lmax(S), c->g_node.p, c->g_flag.p, c->g_seg.p, c->g_segstart.p,
-                              (int)maxg, c->groups.p, c->ngroups.p, c->scan_scratch.p, c->err.p, s);
+                              gg_target_order_lmax(S), c->g_node.p, c->g_stat.p, (int)maxg, c->groups.p, c->ngroups.p,
+                              c->err.p, s);
     } else {
         gg_launch_groups(toff, S, c->cfg.group_size, c->groups.p, c->ngroups.p, c->gscan.p, s);
     }
     const unsigned *gorder = nullptr;
     if (c->cfg.group_order && !c->tcost_valid)   // a fresh history: targets not walked yet cost 0
         GG_CUDA_TRY(cudaMemsetAsync(c->tcost.p, 0, (size_t)c->N * sizeof(float), s));
-    if (c->cfg.group_order && c->tcost_valid) {
+    // (where every group gets a warp at once, the order does not matter)
+    if (c->cfg.group_order && c->tcost_valid && maxg > gg_num_sms() * 2 * (gg_walk_threads() / 32)) {
         if ((st = gg_order_groups_by_cost(c->groups.p, c->ngroups.p, (int)maxg, tlist, c->perm.p, c->tcost.p,
                                           c->gkey.p, c->gorder.p, c->sort_scratch.p, c->err.p, s)))
             return st;

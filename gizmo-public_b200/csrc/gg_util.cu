@@ -238,52 +238,132 @@ __global__ void k_group_nodes(TreeBuf tb, const int *__restrict__ tscan, int gs,
     }
 }
 
-// flag[t] = 1 where target t starts a new group node
-__global__ void k_group_seg_flags(int nt, const int *__restrict__ tlist, const int *__restrict__ gnode,
-                                  int *__restrict__ flag)
+// Groups in one launch: a group starts at every gs-th target of a segment (a
+// run of consecutive targets of one group node).  Tiles of GT_TILE targets are
+// taken in ticket order.  A tile needs two things of its predecessors: the last
+// segment start before it (its own targets tell where segments start, so the
+// nearest tile with a start suffices), and then the number of groups before it.
+// Both are found by looking back over the words the predecessors publish, which
+// they do before they wait on anyone, so every wait ends; the waits are bounded
+// all the same.  (Two device-wide scans and four passes over the targets made ten
+// launches of this, about 35 us at 65,536 targets.)
+#define GT_THREADS 256
+#define GT_ITEMS 4
+#define GT_TILE (GT_THREADS * GT_ITEMS)
+#define GT_SPIN_LIMIT (1 << 22)
+#define GT_SET 0x80000000u        // the word is published
+#define GT_SUM 0x40000000u        // ... and holds the groups up to and with the tile, not the tile's own
+
+__device__ __forceinline__ unsigned gt_wait(const unsigned *p, int *err)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
-        const int pi = tlist ? tlist[t] : t;
-        flag[t] = (t == 0 || gnode[pi] != gnode[tlist ? tlist[t - 1] : t - 1]) ? 1 : 0;
+    unsigned v;
+    for (int i = 0; i < GT_SPIN_LIMIT; i++) {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+        if (v & GT_SET) return v;
+        __nanosleep(20);
     }
+    atomicOr(err, GG_EBIT_SORT_TIMEOUT);
+    return GT_SET | GT_SUM;
+}
+__device__ __forceinline__ void gt_publish(unsigned *p, unsigned v)
+{
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// segstart[j] = first target of segment j; segstart[nseg] = nt
-__global__ void k_group_seg_starts(int nt, const int *__restrict__ flag, const int *__restrict__ segidx,
-                                   int *__restrict__ segstart)
+__global__ void __launch_bounds__(GT_THREADS) k_groups_tree(int nt, const int *__restrict__ tlist,
+                                                            const int *__restrict__ gnode, const int *__restrict__ toff,
+                                                            int S, int gs, int maxg, unsigned *__restrict__ stat,
+                                                            GGGroup *__restrict__ groups, int *__restrict__ ngroups,
+                                                            int *__restrict__ err)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
-        if (flag[t]) segstart[segidx[t]] = t;
-        if (t == 0) segstart[segidx[nt]] = nt;
+    __shared__ int ws[33];
+    __shared__ int s_tile, s_carry, s_before, s_wmax[GT_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    nt = min(nt, toff[S]);   // fewer when the list of active particles had invalid or repeated indices
+    const int ntiles = max(1, (nt + GT_TILE - 1) / GT_TILE);
+    unsigned *const seg = stat + 1, *const cnt = seg + ntiles;   // per tile: last segment start + 1, group counts
+    if (tid == 0) s_tile = (int)atomicAdd(stat, 1u);
+    __syncthreads();
+    const int tile = s_tile, t0 = tile * GT_TILE + tid * GT_ITEMS;
+    if (tile >= ntiles) return;
+    // ---- segment starts of the thread's targets; the last one so far, by an inclusive maximum over the tile
+    int gn[GT_ITEMS], start[GT_ITEMS], last = -1;
+    int prev = t0 > 0 && t0 < nt ? gnode[tlist ? tlist[t0 - 1] : t0 - 1] : -1;
+#pragma unroll
+    for (int j = 0; j < GT_ITEMS; j++) {
+        const int t = t0 + j;
+        gn[j] = t < nt ? gnode[tlist ? tlist[t] : t] : prev;
+        if (t < nt && (t == 0 || gn[j] != prev)) last = t;
+        prev = gn[j];
+        start[j] = last;
     }
-}
-
-// seg[t] becomes the segment holding target t, flag[t] 1 where t starts a
-// group: every gs-th target of its segment (both in place, one thread per t)
-__global__ void k_group_start_flags(int nt, int *__restrict__ flag, int *__restrict__ seg,
-                                    const int *__restrict__ segstart, int gs)
-{
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
-        const int j = seg[t] + flag[t] - 1;
-        seg[t] = j;
-        flag[t] = ((t - segstart[j]) % gs) == 0 ? 1 : 0;
+    int m = last;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, m, o);
+        if (lane >= o) m = max(m, y);
     }
-}
-
-__global__ void k_group_write_tree(int nt, const int *__restrict__ flag, const int *__restrict__ seg,
-                                   const int *__restrict__ segstart, const int *__restrict__ gidx,
-                                   const int *__restrict__ toff, int S, int gs, int maxg, GGGroup *__restrict__ groups,
-                                   int *__restrict__ ngroups, int *__restrict__ err)
-{
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
-        if (t == 0) *ngroups = min(gidx[nt], maxg);
-        if (!flag[t]) continue;
-        const int g = gidx[t];
+    if (lane == 31) s_wmax[w] = m;
+    int before = __shfl_up_sync(0xffffffffu, m, 1);
+    if (lane == 0) before = -1;
+    __syncthreads();
+    int tile_last = -1;
+#pragma unroll
+    for (int i = 0; i < GT_THREADS / 32; i++) {
+        if (i < w) before = max(before, s_wmax[i]);
+        tile_last = max(tile_last, s_wmax[i]);
+    }
+    // ---- the last segment start before the tile (target 0 starts one, so tile 0 has its own)
+    if (tid == 0) {
+        gt_publish(seg + tile, GT_SET | (unsigned)(tile_last + 1));
+        int c = -1;
+        for (int q = tile - 1; q >= 0 && c < 0; q--) c = (int)(gt_wait(seg + q, err) & 0x3fffffffu) - 1;
+        s_carry = c;
+    }
+    __syncthreads();
+    before = max(before, s_carry);
+    // ---- group starts
+    bool first[GT_ITEMS];
+    int mine = 0;
+#pragma unroll
+    for (int j = 0; j < GT_ITEMS; j++) {
+        const int t = t0 + j, s0 = max(start[j], before);
+        first[j] = t < nt && (t - s0) % gs == 0;
+        mine += first[j];
+    }
+    int total;
+    const int off = block_excl_scan(mine, ws, &total);
+    // ---- groups before the tile
+    if (w == 0) {
+        if (lane == 0) gt_publish(cnt + tile, GT_SET | (tile == 0 ? GT_SUM : 0u) | (unsigned)total);
+        int sum = 0;
+        for (int q = tile - 1; q >= 0; q -= 32) {   // 32 predecessors at a time, up to the nearest running sum
+            const unsigned v = q - lane >= 0 ? gt_wait(cnt + q - lane, err) : GT_SET | GT_SUM;
+            const unsigned sums = __ballot_sync(0xffffffffu, (v & GT_SUM) != 0);
+            const int stop = sums ? __ffs(sums) - 1 : 31;
+            sum += (int)__reduce_add_sync(0xffffffffu, lane <= stop ? v & 0x3fffffffu : 0u);
+            if (sums) break;
+        }
+        if (lane == 0) {
+            if (tile > 0) gt_publish(cnt + tile, GT_SET | GT_SUM | (unsigned)(sum + total));
+            s_before = sum;
+            if (tile == ntiles - 1) *ngroups = min(sum + total, maxg);
+        }
+    }
+    __syncthreads();
+    int g = s_before + off;
+#pragma unroll
+    for (int j = 0; j < GT_ITEMS; j++) {
+        if (!first[j]) continue;
+        const int t = t0 + j;
         if (g >= maxg) {   // cannot happen: the table is sized for the bound on group nodes
             atomicOr(err, GG_EBIT_NODE_OVERFLOW);
             continue;
         }
-        const int j = seg[t];
+        // the group ends with its segment or after gs targets
+        int end = t + 1;
+        const int most = min(nt, t + gs);
+        while (end < most && gnode[tlist ? tlist[end] : end] == gn[j]) end++;
         int lo = 0, hi = S - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -291,10 +371,10 @@ __global__ void k_group_write_tree(int nt, const int *__restrict__ flag, const i
         }
         GGGroup gr;
         gr.first = t;
-        gr.count = min(gs, segstart[j + 1] - t);
+        gr.count = end - t;
         gr.root = lo;
         gr.sys = lo;
-        groups[g] = gr;
+        groups[g++] = gr;
     }
 }
 
@@ -309,28 +389,21 @@ long long gg_max_groups(long long n, int S, int gs)
     return n / gs + 2LL * S + 1 + 8LL * GG_MAX_DEPTH * per_depth;
 }
 
-// Scratch: gnode n_particles + 1 ints (reused for the group index scan),
-// flag nt, seg and segstart nt + 1 each.
+size_t gg_group_stat_words(long long nt) { return 1 + 2 * (size_t)((nt + GT_TILE - 1) / GT_TILE); }
+
 void gg_launch_groups_tree(int nt, const int *tlist, const int *tscan, const int *toff, int S, int gs,
                            const TreeBuf &tb, const GGDomainDev *order_dom, const unsigned *hmm, int lmax, int *gnode,
-                           int *flag, int *seg, int *segstart, int maxg, GGGroup *groups, int *ngroups,
-                           int *scan_scratch, int *err, cudaStream_t st)
+                           unsigned *gstat, int maxg, GGGroup *groups, int *ngroups, int *err, cudaStream_t st)
 {
-    const int threads = 256, blocks = gg_num_sms() * 8;
     if (nt <= 0) {
         cudaMemsetAsync(ngroups, 0, sizeof(int), st);
         return;
     }
-    k_group_nodes<<<blocks, threads, 0, st>>>(tb, tscan, gs, order_dom, hmm, lmax, gnode);
-    k_group_seg_flags<<<blocks, threads, 0, st>>>(nt, tlist, gnode, flag);
-    scan_run(flag, seg, nt, 0, scan_scratch, st);
-    k_group_seg_starts<<<blocks, threads, 0, st>>>(nt, flag, seg, segstart);
-    k_group_start_flags<<<blocks, threads, 0, st>>>(nt, flag, seg, segstart, gs);
-    int *gidx = gnode;   // the group nodes are no longer needed
-    scan_run(flag, gidx, nt, 0, scan_scratch, st);
-    k_group_write_tree<<<blocks, threads, 0, st>>>(nt, flag, seg, segstart, gidx, toff, S, gs, maxg, groups, ngroups,
-                                                   err);
-    gg_note_launches(5);
+    cudaMemsetAsync(gstat, 0, gg_group_stat_words(nt) * sizeof(unsigned), st);
+    k_group_nodes<<<gg_num_sms() * 8, 256, 0, st>>>(tb, tscan, gs, order_dom, hmm, lmax, gnode);
+    k_groups_tree<<<(nt + GT_TILE - 1) / GT_TILE, GT_THREADS, 0, st>>>(nt, tlist, gnode, toff, S, gs, maxg, gstat, groups,
+                                                                       ngroups, err);
+    gg_note_launches(2);
 }
 
 int gg_target_order_lmax(int S)
@@ -355,19 +428,21 @@ __global__ void k_group_cost(const GGGroup *__restrict__ groups, const int *__re
                              const int *__restrict__ tlist, const unsigned *__restrict__ perm,
                              const float *__restrict__ cost, unsigned long long *key, unsigned *val)
 {
-    const int ng = *ngroups;
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < maxg; g += gridDim.x * blockDim.x) {
-        unsigned k = 255u;   // past the device count: last
-        if (g < ng) {
-            const GGGroup G = groups[g];
-            float c = 0.f;
-            for (int t = G.first; t < G.first + G.count; t++) c += cost[perm[tlist ? tlist[t] : t]];
-            // descending octave of the cost (the float's exponent field); a
-            // valid group never takes the last key
-            k = 255u - max(__float_as_uint(fmaxf(c, 0.f)) >> 23, 1u);
+    const int ng = *ngroups, j = threadIdx.x & 7;   // 8 lanes per group
+    for (int g0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; (g0 & ~3) < maxg; g0 += (gridDim.x * blockDim.x) >> 3) {
+        float c = 0.f;
+        if (g0 < ng) {
+            const GGGroup G = groups[g0];
+            for (int t = G.first + j; t < G.first + G.count; t += 8) c += cost[perm[tlist ? tlist[t] : t]];
         }
-        key[g] = k;
-        val[g] = (unsigned)g;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        // descending octave of the cost (the float's exponent field); a valid
+        // group never takes the last key, which those past the device count get
+        if (j == 0 && g0 < maxg) {
+            key[g0] = g0 < ng ? 255u - max(__float_as_uint(fmaxf(c, 0.f)) >> 23, 1u) : 255u;
+            val[g0] = (unsigned)g0;
+        }
     }
 }
 
@@ -376,7 +451,7 @@ gg_status gg_order_groups_by_cost(const GGGroup *groups, const int *ngroups, int
                                   unsigned *gorder, void *sort_scratch, int *err, cudaStream_t st)
 {
     if (maxg <= 0) return GG_OK;
-    const int blocks = std::max(1, std::min(gg_num_sms() * 4, (maxg + 255) / 256));
+    const int blocks = std::max(1, std::min(gg_num_sms() * 4, (maxg + 31) / 32));
     k_group_cost<<<blocks, 256, 0, st>>>(groups, ngroups, maxg, tlist, perm, cost, key, gorder);
     gg_note_launches(1);
     // one pass over the 8-bit key; the sort is stable, so the groups of one cost octave keep
