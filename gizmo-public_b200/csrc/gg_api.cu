@@ -247,6 +247,8 @@ struct gg_ctx {
     DevBuf<int> ngroups, gscan, toff, flag, flagscan, tlist, tout, scan_scratch, active_d;
     DevBuf<int> g_node;                    // group building scratch
     DevBuf<unsigned> g_stat;
+    DevBuf<WalkFork> forks;                // records of cut walks
+    DevBuf<char> own_forks;
     DevBuf<int> counters;                  // [0] group counter
     DevBuf<unsigned long long> inter;      // interaction total
     DevBuf<int> stack;
@@ -304,7 +306,7 @@ struct gg_ctx {
         f(oldacc); f(vel); f(newpos); f(kin); f(kin_counter); f(dts); f(oldacc_save); f(tcost); f(gkey); f(gorder);
         f(e_chunks); f(e_first); f(e_part); f(e_out);
         f(groups); f(ngroups); f(gscan); f(toff); f(flag); f(flagscan); f(tlist); f(tout); f(scan_scratch);
-        f(g_node); f(g_stat);
+        f(g_node); f(g_stat); f(forks); f(own_forks);
         f(active_d); f(counters); f(inter); f(stack); f(err); f(acc_d); f(pot_d); f(nint_d); f(oldacc_in);
         f(tune_tg); f(tune_rows); f(tune_acc); f(tune_pot); f(tune_mass); f(tune_gacc); f(tune_gpot);
     }
@@ -693,7 +695,19 @@ extern "C" gg_status gg_get_domains(gg_ctx *c, gg_domain *out)
 }
 
 // ---------------------------------------------------------------- walk
-static gg_status walk_setup(gg_ctx *c)
+// whether long walks may be cut: some system has as many targets as that takes
+// (of a subset, the targets per system are known on the device only)
+static bool may_fork(const gg_ctx *c, bool subset)
+{
+    if (c->cfg.group_size <= 1) return false;
+    for (int s = 0; s < c->S; s++) {
+        const long long n = c->h_poff[s + 1] - c->h_poff[s];
+        if (n >= FORK_MIN_TARGETS && (subset || n <= FORK_MAX_TARGETS)) return true;
+    }
+    return false;
+}
+
+static gg_status walk_setup(gg_ctx *c, bool subset)
 {
     gg_status st;
     if (!c->stack_cap) c->stack_cap = c->cfg.walk_stack_entries > 0 ? c->cfg.walk_stack_entries : GG_STACK_CAP;
@@ -711,6 +725,10 @@ static gg_status walk_setup(gg_ctx *c)
         (st = c->stack.ensure((size_t)c->walk_blocks * gg_num_sms() * (gg_walk_threads() / 32) * c->stack_cap)) ||
         (st = c->scan_scratch.ensure(gg_scan_scratch_ints())))
         return st;
+    if (may_fork(c, subset) &&
+        ((st = c->forks.ensure(FORK_RECORDS)) ||
+         (st = c->own_forks.ensure((size_t)c->walk_blocks * gg_num_sms() * (gg_walk_threads() / 32) * FORK_OWN_BYTES))))
+        return st;
     if (c->cfg.group_order &&
         ((st = c->tcost.ensure(c->N + 1)) || (st = c->gkey.ensure(maxg)) || (st = c->gorder.ensure(maxg)) ||
          (st = c->sort_scratch.ensure(gg_sort_scratch_bytes(maxg)))))
@@ -725,7 +743,7 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
 {
     gg_status st;
     cudaStream_t s = c->stream;
-    if ((st = walk_setup(c))) return st;
+    if ((st = walk_setup(c, d_active != nullptr))) return st;
     if ((st = resolve_h_mixed(c))) return st;
     const int S = c->S, N = (int)c->N;
     const int *tlist = nullptr, *tout = nullptr;
@@ -795,6 +813,12 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
     p.ninter = d_nint;
     p.interactions = c->inter.p;
     p.group_counter = c->counters.p;
+    p.toff = toff;
+    p.forks = c->forks.p;
+    p.own_forks = c->own_forks.p;
+    p.fork_max = (d_active ? n_active : N) <= FORK_TASK_TARGETS ? FORK_RECORDS : 0;
+    p.may_fork = may_fork(c, d_active != nullptr);
+    p.task_walk = 0;
     p.stack = c->stack.p;
     p.stack_cap = c->stack_cap;
     p.err = c->err.p;
@@ -1069,7 +1093,7 @@ extern "C" gg_status gg_graph_capture_step(gg_ctx *c, double tol, double theta, 
     if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
     if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
     // grow every buffer the walk may need, and read the kernel-radius ranges, before capturing
-    if ((st = walk_setup(c))) return st;
+    if ((st = walk_setup(c, false))) return st;
     if ((st = resolve_h_mixed(c))) return st;
     const int timing = c->cfg.timing;
     c->cfg.timing = 0;
@@ -1109,7 +1133,7 @@ extern "C" gg_status gg_graph_capture_parts(gg_ctx *c, double tol, double theta,
     gg_status st;
     if ((st = set_device(c))) return st;
     drop_part_graphs(c);
-    if ((st = walk_setup(c))) return st;
+    if ((st = walk_setup(c, false))) return st;
     if ((st = resolve_h_mixed(c))) return st;
     const int timing = c->cfg.timing;
     c->cfg.timing = 0;

@@ -1,5 +1,7 @@
 // gg_kernels.cuh -- launch functions shared between the kernel files and the API.
 #pragma once
+#include <cstddef>
+
 #include "gg_internal.cuh"
 
 #define GG_SORT_MAX_PASSES 12
@@ -45,6 +47,45 @@ int gg_tree_grid();
 gg_status gg_launch_tree(const unsigned long long *keys, const int *poff, int S, int n, int leaf, int cap, TreeBuf tb,
                          const GGPart *parts, const GGDomainDev *dom, GGNode *nodes, cudaStream_t st);
 
+// Long walks are cut (gg_walk.cu) in systems that have a few groups per resident
+// warp.  Smaller systems come in batches and gain little alone (with 65,536 in the
+// range a batch of 48 served systems took 7% longer); in larger ones the groups
+// outnumber the warps so far that the longest, started first, end with the rest
+// (cut at 500,000 targets, a 10% subset of 4.2M particles took 6.9 ms instead of
+// 5.6).
+#define FORK_MIN_TARGETS 98304
+#define FORK_MAX_TARGETS 300000
+// Work (node tests, list entries; a softened entry counts four) after which a walk
+// is cut: about twice a mean group's, or four times in systems above
+// FORK_HALF_TARGETS.  Walk ms uncut / cut at 8192 / 16384 / 32768: Plummer 65,536
+// 0.34 / 0.31 / 0.35 / 0.35, galaxy 100,000 0.97 / 0.78 / 0.81 / 0.95, galaxy
+// 262,144 2.06 / 2.73 / 1.38 / 1.56.
+#define FORK_HALF_TARGETS 131072
+#define FORK_WORK 16384
+#define FORK_WALKS 8        // sub-walks the pending nodes are dealt to
+#define FORK_PENDING 2048   // pending nodes at most
+#define FORK_RECORDS 512    // cuts whose sub-walks can run as tasks of their own
+// ... in launches of at most this many targets; with more, there is work enough
+// for every warp, and each runs its own sub-walks
+#define FORK_TASK_TARGETS 400000
+// the record of one cut
+struct WalkFork {
+    int group, npend;
+    float cost;
+    int pad;
+    int pending[FORK_PENDING];
+    // per target: acceleration and potential, interactions; of the walk up to the
+    // cut, and (not in the records of single warps, which end here) of the sub-walks
+    double4 sum0[64];
+    int nint0[64];
+    double4 sum[FORK_WALKS][64];
+    int nint[FORK_WALKS][64];
+};
+#define FORK_OWN_BYTES offsetof(WalkFork, sum)
+// places in WalkParams.group_counter: groups handed out, cuts made, tasks handed out
+#define WALK_FORK_COUNTER 1
+#define WALK_TASK_COUNTER 2
+
 struct WalkParams {
     const GGNode *nodes;
     const GGPart *parts;        // sorted
@@ -60,7 +101,13 @@ struct WalkParams {
     double *pot;                // per output slot, may be NULL
     int *ninter;                // per output slot, may be NULL
     unsigned long long *interactions;   // [0] interactions, [1] far / [2] near list entries, [3] nodes tested
-    int *group_counter;
+    int *group_counter;         // three counters, zero at the launch
+    const int *toff;            // target offsets per system
+    WalkFork *forks;            // fork_max records
+    char *own_forks;            // a record of FORK_OWN_BYTES per resident warp
+    int fork_max;
+    int may_fork;               // some walk of this launch may be cut
+    int task_walk;              // this launch runs the sub-walks of the cuts
     int *stack;
     int stack_cap;
     int *err;

@@ -81,7 +81,7 @@ int gg_walk_threads() { return WALK_THREADS; }
 #define FAR_CAP (FAR_FLUSH_MAX + 32 * NH + 32)
 #define NEAR_CAP (NEAR_FLUSH_MAX + 32 * NH + 32)
 #define WALK_WARP_FLOATS \
-    (FAR_ARRAYS * FAR_CAP + NEAR_ARRAYS * NEAR_CAP + WALK_SSTACK + NH * 32 * 16 + 32 + 2 * RUNS + 4)
+    (FAR_ARRAYS * FAR_CAP + NEAR_ARRAYS * NEAR_CAP + WALK_SSTACK + NH * 32 * 16 + 32 + 2 * RUNS + 4 + 8)
 
 // ---- staging of node records
 // The next round's node records are copied into shared memory, one 64-byte slot
@@ -492,6 +492,29 @@ __device__ __forceinline__ double warp_max_d(double v)
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(FULL, v, o));
     return v;
 }
+// one target's results: t its place in the target list, pi its sorted particle
+template <bool POT>
+__device__ __forceinline__ void write_target(const WalkParams &p, int t, int pi, float hinv, double ax, double ay,
+                                             double az, double ph, int nint, float tcost)
+{
+    const unsigned li = p.perm[pi];
+    const int o = p.tout ? p.tout[t] : (int)li;
+    if (POT) {
+        // compute_potential removes the self term m_i kernel(0) / h_i
+        // (potential.c:137-145); subtract the FP32 value the walk added
+        const float mi = p.parts[pi].m;
+        p.pot[o] = ph - (double)((mi * -2.8f) * hinv);
+    } else {
+        p.acc[3 * (size_t)o] = ax;
+        p.acc[3 * (size_t)o + 1] = ay;
+        p.acc[3 * (size_t)o + 2] = az;
+        if (p.pot) p.pot[o] = ph;
+        if (p.oldacc_out) p.oldacc_out[li] = sqrt(ax * ax + ay * ay + az * az);
+    }
+    if (p.ninter) p.ninter[o] = nint;
+    if (p.cost_out) p.cost_out[li] = tcost;
+}
+
 __device__ __forceinline__ int warp_incl_scan(int v, int lane)
 {
 #pragma unroll
@@ -504,7 +527,7 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane)
 // F64T: opening tests in FP64 (used for one-target groups, where the tests are
 // exactly the reference's); otherwise the tests run in FP32 on FP64-formed
 // offsets from the group centre, against a bounding box rounded outwards.
-template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA = false>
+template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA, bool CUT>
 __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
 {
     extern __shared__ float4 walk_smem[];
@@ -524,6 +547,9 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
     int *run = reinterpret_cast<int *>(rest + WALK_SSTACK + NH * 32 * 16);   // see expand
     int *qbase = run + 32, *qend = qbase + RUNS;   // queued runs: first particle less its position, end position
     const unsigned bar = (unsigned)__cvta_generic_to_shared(qend + RUNS);
+    // state of a cut walk (CUT): kept here, not in registers
+    struct CutState { WalkFork *fork; int sub, npend, own, group; };
+    CutState &cut = *reinterpret_cast<CutState *>(qend + RUNS + 4);
     if (lane == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -537,11 +563,36 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
 
     for (;;) {
         int g = 0;
-        if (lane == 0) g = atomicAdd(p.group_counter, 1);
+        if (lane == 0) g = atomicAdd(p.group_counter + (p.task_walk ? WALK_TASK_COUNTER : 0), 1);
         g = __shfl_sync(FULL, g, 0);
-        if (g >= ngroups) break;
-        const GGGroup grp = p.groups[p.gorder ? (int)p.gorder[g] : g];
+        if (CUT && p.task_walk) {
+            if (g >= min(p.group_counter[WALK_FORK_COUNTER], p.fork_max) * FORK_WALKS) break;
+            WalkFork *const fork = p.forks + g / FORK_WALKS;
+            if (lane == 0) cut = {fork, 1 + g % FORK_WALKS, fork->npend, 0, fork->group};
+            g = fork->group;
+        } else {
+            if (g >= ngroups) break;
+            if (p.gorder) g = (int)p.gorder[g];
+            if (CUT && lane == 0) cut = {nullptr, 0, 0, 0, g};
+        }
+        if (CUT) __syncwarp();
+        const GGGroup grp = p.groups[g];
         const long long t_start = clock64();
+        // Long walks.  A group with far more work than most (a dense centre, a box
+        // that reaches into one) would set the length of a walk that has only a few
+        // groups per warp.  Once its work (node tests, list entries) reaches
+        // FORK_WORK the nodes still pending are dealt out to FORK_WALKS sub-walks
+        // with sums of their own: tasks of a second launch, or, when the records of
+        // cuts are used up, the same warp's next work.  The sums are added in order
+        // either way, and whether and where a walk is cut depends on the group and
+        // its system's size alone, so a system's results do not depend on what it is
+        // batched with.
+        int cut_at = INT_MAX;
+        if (CUT && !p.task_walk) {
+            const int nt = p.toff[grp.sys + 1] - p.toff[grp.sys];
+            if (nt >= FORK_MIN_TARGETS && nt <= FORK_MAX_TARGETS)
+                cut_at = nt <= FORK_HALF_TARGETS ? FORK_WORK / 2 : FORK_WORK;
+        }
 
         // ---- targets of the group
         Targets<TPL> T;
@@ -555,8 +606,6 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             int k = s * LP + lane % LP;
             bool v = k < grp.count;
             T.valid[s] = v;
-            T.self[s] = 0;
-            T.ax[s] = {0.f, 0.f}; T.ay[s] = {0.f, 0.f}; T.az[s] = {0.f, 0.f}; T.pot[s] = {0.f, 0.f};
             tpi[s] = -1;
             tx[s] = ty[s] = tz[s] = 0.0;
             T.h[s] = 0.f;
@@ -611,6 +660,12 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         // records is in flight during the tests.  One loop does whatever is due,
         // so that every part appears in the code once (the kernel is large
         // against the instruction cache).
+      for (;;) {   // sub-walks
+#pragma unroll
+        for (int s = 0; s < TPL; s++) {
+            T.self[s] = 0;
+            T.ax[s] = {0.f, 0.f}; T.ay[s] = {0.f, 0.f}; T.az[s] = {0.f, 0.f}; T.pot[s] = {0.f, 0.f};
+        }
         int sp = 0, gsp = 0, nf = 0, nn = 0;
         int qhead = 0, qtail = 0;     // runs of particles in the queue
         int pw = 0, pt = 0;           // positions of the queue's particles: next, end
@@ -626,6 +681,15 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         {
             int node[NH];
             node[0] = lane == 0 ? grp.root : -1;
+            if (CUT && cut.sub > 0) {   // every FORK_WALKS-th pending node: at most FORK_PENDING / FORK_WALKS
+                const int sub = cut.sub, m = (cut.npend - sub + FORK_WALKS) / FORK_WALKS;
+                for (int i = lane; i < m; i += 32) sstack[i] = cut.fork->pending[sub - 1 + FORK_WALKS * i];
+                __syncwarp();
+                k = min(m, 32 * NH);
+                sp = m - k;
+#pragma unroll
+                for (int h = 0; h < NH; h++) node[h] = 32 * h + lane < k ? sstack[sp + 32 * h + lane] : -1;
+            }
             stage(node, k);
         }
         // appends one entry per lane with `use`: to the far list, or to the near list with its softening
@@ -846,6 +910,34 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
                     sp = m;
                 }
                 __syncwarp();
+                if (CUT && tested + list_far + 3 * list_near >= cut_at && gsp + sp + ctot >= 2 * FORK_WALKS &&
+                    gsp + sp + ctot <= FORK_PENDING) {
+                    int f = 0;
+                    if (lane == 0) f = atomicAdd(p.group_counter + WALK_FORK_COUNTER, 1);
+                    f = __shfl_sync(FULL, f, 0);
+                    const bool own = f >= p.fork_max;
+                    WalkFork *const fork =
+                        own ? reinterpret_cast<WalkFork *>(p.own_forks + (size_t)(blockIdx.x * WALK_WARPS + warp) *
+                                                                             FORK_OWN_BYTES)
+                            : p.forks + f;
+                    for (int i = lane; i < gsp; i += 32) fork->pending[i] = gstack[i];
+                    for (int i = lane; i < sp; i += 32) fork->pending[gsp + i] = sstack[i];
+                    sp += gsp;
+                    for (int w = 0; w < ctot; w += 32) {
+                        const int i = expand(cbase, cbeg, cfin, w);
+                        if (w + lane < ctot) fork->pending[sp + w + lane] = i;
+                    }
+                    if (lane == 0) {
+                        fork->group = cut.group;
+                        fork->npend = sp + ctot;
+                        cut.fork = fork;
+                        cut.npend = sp + ctot;
+                        cut.own = own;
+                    }
+                    cut_at = INT_MAX;
+                    gsp = sp = ctot = 0;   // the rest of this sub-walk: queued particles and lists
+                    __syncwarp();
+                }
                 k = min(sp + ctot, 32 * NH);
                 const int w0 = ctot - k;   // first position taken now; negative: from the stack
                 int node[NH];
@@ -924,7 +1016,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             if (tma) phase ^= 1u;
             if (lane == 0) atomicOr(p.err, GG_EBIT_STACK_OVERFLOW);
             __syncwarp();
-            continue;
+            break;   // to the next group
         }
         __syncwarp();   // the next group's entries overwrite the lists
 
@@ -949,25 +1041,28 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
                 self += __shfl_xor_sync(FULL, self, o);
             }
             if (!T.valid[s] || (SPLIT > 1 && part != s)) continue;   // part s writes target s
-            const int nint = list_far + list_near - self;
-            int t = grp.first + s * LP + lane % LP;
-            int pi = tpi[s];
-            unsigned li = p.perm[pi];
-            int o = p.tout ? p.tout[t] : (int)li;
-            if (POT) {
-                // compute_potential removes the self term m_i kernel(0) / h_i
-                // (potential.c:137-145); subtract the FP32 value the walk added
-                const float mi = p.parts[pi].m;
-                p.pot[o] = ph - (double)((mi * -2.8f) * T.hinv[s]);
-            } else {
-                p.acc[3 * (size_t)o] = ax;
-                p.acc[3 * (size_t)o + 1] = ay;
-                p.acc[3 * (size_t)o + 2] = az;
-                if (p.pot) p.pot[o] = ph;
-                if (p.oldacc_out) p.oldacc_out[li] = sqrt(ax * ax + ay * ay + az * az);
+            int nint = list_far + list_near - self;
+            const int slot = s * LP + lane % LP;
+            if (CUT && cut.fork) {
+                WalkFork *const fork = cut.fork;
+                const int sub = cut.sub;
+                const bool own = cut.own;
+                if (own && sub > 0) {   // the sums so far
+                    const double4 q = fork->sum0[slot];
+                    ax = q.x + ax; ay = q.y + ay; az = q.z + az; ph = q.w + ph;
+                    nint += fork->nint0[slot];
+                }
+                if (!own || sub < FORK_WALKS) {
+                    const bool first = own || sub == 0;
+                    double4 *const sum = first ? fork->sum0 : fork->sum[sub - 1];
+                    int *const cnt = first ? fork->nint0 : fork->nint[sub - 1];
+                    sum[slot] = make_double4(ax, ay, az, ph);
+                    cnt[slot] = nint;
+                    if (sub == 0 && slot == 0) fork->cost = tcost;
+                    continue;
+                }
             }
-            if (p.ninter) p.ninter[o] = nint;
-            if (p.cost_out) p.cost_out[li] = tcost;
+            write_target<POT>(p, grp.first + slot, tpi[s], T.hinv[s], ax, ay, az, ph, nint, tcost);
             mycount += nint;
         }
 #pragma unroll
@@ -978,15 +1073,64 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             atomicAdd(p.interactions + 2, (unsigned long long)list_near);
             atomicAdd(p.interactions + 3, (unsigned long long)tested);
         }
+        if (!CUT || !cut.own || cut.sub == FORK_WALKS) break;
+        __syncwarp();
+        if (lane == 0) cut.sub++;
+        __syncwarp();   // also the pending nodes, written by other lanes
+      }
     }
 }
 
+// The sums of the cut walks whose sub-walks ran as tasks, added in order: one
+// warp per cut.
+template <bool POT>
+__global__ void __launch_bounds__(WALK_THREADS) k_walk_join(WalkParams p)
+{
+    const int lane = threadIdx.x & 31, w = (blockIdx.x * WALK_THREADS + threadIdx.x) >> 5;
+    if (w >= min(p.group_counter[WALK_FORK_COUNTER], p.fork_max)) return;
+    const WalkFork &f = p.forks[w];
+    const GGGroup grp = p.groups[f.group];
+    int mycount = 0;
+    for (int slot = lane; slot < grp.count; slot += 32) {
+        double4 a = f.sum0[slot];
+        int nint = f.nint0[slot];
+        for (int i = 0; i < FORK_WALKS; i++) {
+            const double4 q = f.sum[i][slot];
+            a.x += q.x; a.y += q.y; a.z += q.z; a.w += q.w;
+            nint += f.nint[i][slot];
+        }
+        const int t = grp.first + slot, pi = p.tlist ? p.tlist[t] : t;
+        const float h = p.parts[pi].h;
+        write_target<POT>(p, t, pi, h > 0.f ? __frcp_rn(h) : INFINITY, a.x, a.y, a.z, a.w, nint, f.cost);
+        mycount += nint;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mycount += __shfl_xor_sync(FULL, mycount, o);
+    if (lane == 0) atomicAdd(p.interactions, (unsigned long long)mycount);
+}
+
+template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA, bool CUT>
+static void launch_walk_c(const WalkParams &p, int blocks, cudaStream_t st)
+{
+    const int smem = WALK_WARPS * WALK_WARP_FLOATS * (int)sizeof(float);
+    cudaFuncSetAttribute(k_walk<TPL, SPLIT, F64T, POT, TMA, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_walk<TPL, SPLIT, F64T, POT, TMA, CUT><<<blocks, WALK_THREADS, smem, st>>>(p);
+    gg_note_launches(1);
+    if (CUT && p.fork_max > 0) {   // the sub-walks of the walks that were cut
+        WalkParams q = p;
+        q.task_walk = 1;
+        k_walk<TPL, SPLIT, F64T, POT, TMA, CUT><<<blocks, WALK_THREADS, smem, st>>>(q);
+        k_walk_join<POT><<<(p.fork_max + WALK_WARPS - 1) / WALK_WARPS, WALK_THREADS, 0, st>>>(q);
+        gg_note_launches(2);
+    }
+}
+
+// walks that may be cut run a kernel of their own: the state of a cut costs registers
 template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA>
 static void launch_walk_t(const WalkParams &p, int blocks, cudaStream_t st)
 {
-    const int smem = WALK_WARPS * WALK_WARP_FLOATS * (int)sizeof(float);
-    cudaFuncSetAttribute(k_walk<TPL, SPLIT, F64T, POT, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_walk<TPL, SPLIT, F64T, POT, TMA><<<blocks, WALK_THREADS, smem, st>>>(p);
+    if (!F64T && p.may_fork) launch_walk_c<TPL, SPLIT, F64T, POT, TMA, !F64T>(p, blocks, st);
+    else launch_walk_c<TPL, SPLIT, F64T, POT, TMA, false>(p, blocks, st);
 }
 
 // The persistent grid is blocks_per_sm (1..3) blocks per SM, of which two are
@@ -1008,5 +1152,4 @@ void gg_launch_walk(const WalkParams &p, int blocks_per_sm, cudaStream_t st)
         if (wide) launch_walk_t<2, 1, false, false, false>(p, blocks, st);
         else launch_walk_t<2, 2, false, false, false>(p, blocks, st);
     }
-    gg_note_launches(1);
 }

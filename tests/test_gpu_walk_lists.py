@@ -46,3 +46,27 @@ def test_opening_every_node_is_the_direct_sum(n, group_size, flush, leaf_size, s
         # again: up to four roundings of 6e-8 of it stay behind per target
         own = 4 * 6e-8 * np.linalg.norm(2.8 * mass / h)
         assert np.linalg.norm(only - wpot) < 2e-6 * np.linalg.norm(wpot) + own
+
+
+def test_cut_walks_give_the_same_bits_alone_and_in_a_batch():
+    """A system in the range of sizes whose long walks are cut, opening every
+    node: its sub-walks run as tasks when it is alone, and as each warp's own
+    work in a batch too large for that.  Same interactions, same bits."""
+    n = 98304
+    pos, mass, h = _system(n, "one", 5)
+    big = 400001 - n
+    rng = np.random.default_rng(6)
+    more, mm = rng.normal(size=(big, 3)), np.full(big, 1.0)
+    theta = dict(err_tol_theta=0.15)     # a Barnes-Hut pass strict enough for long walks
+    with ggb200.GravityTree() as t:
+        t.load(pos, mass, h)
+        t.build()
+        alone = t.evaluate(want_ninter=True, **theta)
+        t.load(np.concatenate([pos, more]), np.concatenate([mass, mm]), np.concatenate([h, np.full(big, h[0])]),
+               counts=[n, big])
+        t.build()
+        batch = t.evaluate(want_ninter=True, **theta)
+    assert alone[3]["error_word"] == 0 and batch[3]["error_word"] == 0
+    assert alone[2].mean() > 8192        # long enough to be cut
+    for a, b in zip(alone[:3], batch[:3]):
+        assert np.array_equal(a, b[:n])
