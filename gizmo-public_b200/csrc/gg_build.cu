@@ -96,8 +96,10 @@ __device__ __forceinline__ void tb_st_status(unsigned *p, unsigned v)
 
 // Barrier of the whole (cooperatively launched) grid: the blocks count up one
 // word, and the n-th barrier is passed once n * gridDim.x have arrived.  A wait
-// that reaches its limit records GG_EBIT_SORT_TIMEOUT and returns false; the
-// block then leaves the kernel.
+// that reaches its limit (some ten seconds: the first one may wait for other
+// streams' walks to make room for the whole grid) records GG_EBIT_SORT_TIMEOUT and
+// returns false; the block then leaves the kernel.
+#define TB_BARRIER_LIMIT (1 << 24)
 __device__ __forceinline__ bool tb_grid_barrier(unsigned *word, unsigned &target, int *err)
 {
     __syncthreads();
@@ -108,8 +110,8 @@ __device__ __forceinline__ bool tb_grid_barrier(unsigned *word, unsigned &target
         __threadfence();
         atomicAdd(word, 1u);
         int spins = 0;
-        while (tb_ld_status(word) < target && ++spins < TB_SPIN_LIMIT) __nanosleep(20);
-        s_ok = spins < TB_SPIN_LIMIT;
+        while (tb_ld_status(word) < target && ++spins < TB_BARRIER_LIMIT) __nanosleep(20);
+        s_ok = spins < TB_BARRIER_LIMIT;
         if (!s_ok) atomicOr(err, GG_EBIT_SORT_TIMEOUT);
         __threadfence();
     }

@@ -34,8 +34,9 @@
 //   - the next round's node records are staged in shared memory while this
 //     round's leaves and flushes run (per-lane cp.async, or bulk copies of
 //     runs of consecutive records on an mbarrier);
-//   - stack pushes use prefix counts from bit ballots; the particles of opened
-//     leaves go through a per-warp queue and are classified 32 at a time;
+//   - a round tests up to 64 nodes, two per lane; the opened nodes' children are
+//     laid end to end by one scan, and the next round takes them from there; the
+//     particles of opened leaves queue as runs and are classified 32 at a time;
 //   - the lists are one array per component, evaluated two entries per packed
 //     FP32x2 instruction;
 //   - the persistent warps take groups in the order the host side planned
