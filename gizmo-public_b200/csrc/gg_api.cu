@@ -215,8 +215,8 @@ struct gg_ctx {
     DevBuf<char> sort_scratch;
     // tree
     int ncap = 0;
-    DevBuf<int> t_start, t_end, t_level, t_parent, t_sys, t_nch, t_child, t_bnd, t_depth, t_nnodes;
-    DevBuf<unsigned> t_bstat;
+    DevBuf<int> t_start, t_end, t_level, t_parent, t_sys, t_nch, t_child, t_bnd, t_depth;
+    DevBuf<unsigned> t_state;             // node count, barrier words, look-back words of the tree kernels
     DevBuf<double> t_mass64;
     DevBuf<GGNode> nodes;
     // walk
@@ -302,7 +302,7 @@ struct gg_ctx {
         f(poff); f(in_rec); f(part); f(dom); f(extent_mm); f(hmm); f(tkey); f(tval); f(tlist2); f(tout2);
         f(keys); f(perm); f(rank); f(sort_scratch);
         f(t_start); f(t_end); f(t_level); f(t_parent); f(t_sys); f(t_nch); f(t_child); f(t_bnd);
-        f(t_depth); f(t_nnodes); f(t_bstat); f(t_mass64); f(nodes);
+        f(t_depth); f(t_state); f(t_mass64); f(nodes);
         f(oldacc); f(vel); f(newpos); f(kin); f(kin_counter); f(dts); f(oldacc_save); f(tcost); f(gkey); f(gorder);
         f(e_chunks); f(e_first); f(e_part); f(e_out);
         f(groups); f(ngroups); f(gscan); f(toff); f(flag); f(flagscan); f(tlist); f(tout); f(scan_scratch);
@@ -614,7 +614,7 @@ static gg_status ensure_tree(gg_ctx *c)
         (st = c->t_parent.ensure(cap)) || (st = c->t_sys.ensure(cap)) || (st = c->t_nch.ensure(cap)) ||
         (st = c->t_child.ensure(cap)) || (st = c->t_bnd.ensure(cap * 8)) ||
         (st = c->t_mass64.ensure(cap)) || (st = c->nodes.ensure(cap)) || (st = c->t_depth.ensure(GG_MAX_DEPTH + 4)) ||
-        (st = c->t_nnodes.ensure(4)) || (st = c->t_bstat.ensure((size_t)GG_MAX_DEPTH * G + 2)))
+        (st = c->t_state.ensure(TREE_STATE_WORDS(G))))
         return st;
     c->ncap = (int)cap;
     return GG_OK;
@@ -625,13 +625,16 @@ static TreeBuf tree_buf(gg_ctx *c)
     TreeBuf tb;
     tb.start = c->t_start.p; tb.end = c->t_end.p; tb.level = c->t_level.p; tb.parent = c->t_parent.p;
     tb.sys = c->t_sys.p; tb.nch = c->t_nch.p; tb.child = c->t_child.p;
-    tb.bnd = c->t_bnd.p; tb.mass64 = c->t_mass64.p; tb.depth_beg = c->t_depth.p; tb.nnodes = c->t_nnodes.p;
-    tb.bstat = c->t_bstat.p; tb.barrier = nullptr; tb.err = c->err.p;
+    tb.bnd = c->t_bnd.p; tb.mass64 = c->t_mass64.p; tb.depth_beg = c->t_depth.p; tb.nnodes = (int *)c->t_state.p;
+    tb.barrier = c->t_state.p + 2; tb.bstat = c->t_state.p + 4; tb.err = c->err.p;
     tb.cap = c->ncap;
+    tb.wait_limit = TREE_WAIT_LIMIT;
+    tb.wait_extra[0] = tb.wait_extra[1] = 0;
     return tb;
 }
 
-extern "C" gg_status gg_build(gg_ctx *c, const gg_domain *domains)
+// vain: a self-test's tree kernel (0 nodes, 1 moments) whose barriers wait for one arrival too many, else -1
+static gg_status build(gg_ctx *c, const gg_domain *domains, int vain)
 {
     if (!c || c->S < 1) return GG_ERR_INVALID;
     gg_status st;
@@ -670,7 +673,12 @@ extern "C" gg_status gg_build(gg_ctx *c, const gg_domain *domains)
     }
     if (N > 0 && !gathered) gg_launch_permute(c->perm.p, c->in_rec.p, c->part.p, c->rank.p, N, s);
     if (timing) cudaEventRecord(c->ev[2], s);
-    if ((st = gg_launch_tree(c->keys.p, c->poff.p, S, N, c->cfg.leaf_size, c->ncap, tree_buf(c), c->part.p, c->dom.p,
+    TreeBuf tb = tree_buf(c);
+    if (vain >= 0) {
+        tb.wait_extra[vain] = 1;
+        tb.wait_limit = 1 << 12;
+    }
+    if ((st = gg_launch_tree(c->keys.p, c->poff.p, S, N, c->cfg.leaf_size, c->ncap, tb, c->part.p, c->dom.p,
                              c->nodes.p, s)))
         return st;
     if (timing) cudaEventRecord(c->ev[3], s);
@@ -679,6 +687,17 @@ extern "C" gg_status gg_build(gg_ctx *c, const gg_domain *domains)
     c->kin_valid = false;
     c->kin_any = false;
     return GG_OK;
+}
+
+extern "C" gg_status gg_build(gg_ctx *c, const gg_domain *domains) { return build(c, domains, -1); }
+
+static gg_status collect_stats(gg_ctx *c, gg_stats *out);
+
+extern "C" gg_status gg_selftest_tree_wait(gg_ctx *c, int32_t kernel)
+{
+    if (!c || kernel < 0 || kernel > 1) return GG_ERR_INVALID;
+    const gg_status st = build(c, nullptr, kernel);
+    return st ? st : collect_stats(c, nullptr);
 }
 
 extern "C" gg_status gg_get_domains(gg_ctx *c, gg_domain *out)
@@ -798,6 +817,7 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
     GG_CUDA_TRY(cudaMemsetAsync(c->inter.p, 0, 4 * sizeof(unsigned long long), s));
     WalkParams p;
     p.nodes = c->nodes.p;
+    p.nnodes = (const int *)c->t_state.p;
     p.parts = c->part.p;
     p.groups = c->groups.p;
     p.ngroups = c->ngroups.p;
@@ -837,8 +857,6 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
     GG_CUDA_TRY(cudaGetLastError());
     return GG_OK;
 }
-
-static gg_status collect_stats(gg_ctx *c, gg_stats *out);
 
 // A blocking walk: when a warp's node stack overflowed (its group's results
 // were skipped and the error bit set), the walk runs again with four times
@@ -882,7 +900,7 @@ static gg_status collect_stats(gg_ctx *c, gg_stats *out)
     int nn = 0, ng = 0;
     GG_CUDA_TRY(cudaMemcpyAsync(err, c->err.p, sizeof err, cudaMemcpyDeviceToHost, c->stream));
     GG_CUDA_TRY(cudaMemcpyAsync(inter4, c->inter.p, sizeof inter4, cudaMemcpyDeviceToHost, c->stream));
-    if (c->t_nnodes.p) GG_CUDA_TRY(cudaMemcpyAsync(&nn, c->t_nnodes.p, sizeof nn, cudaMemcpyDeviceToHost, c->stream));
+    if (c->t_state.p) GG_CUDA_TRY(cudaMemcpyAsync(&nn, c->t_state.p, sizeof nn, cudaMemcpyDeviceToHost, c->stream));
     if (c->ngroups.p) GG_CUDA_TRY(cudaMemcpyAsync(&ng, c->ngroups.p, sizeof ng, cudaMemcpyDeviceToHost, c->stream));
     GG_CUDA_TRY(cudaStreamSynchronize(c->stream));
     gg_stats &L = c->last;
@@ -1613,7 +1631,7 @@ static gg_status drift_common(gg_ctx *c, const double *dt_host, double dt_all)
     if (dt_host)
         GG_CUDA_TRY(cudaMemcpyAsync(c->dts.p, dt_host, (size_t)c->S * sizeof(double), cudaMemcpyHostToDevice, s));
     gg_launch_drift(c->in_rec.p, c->part.p, c->perm.p, c->vel.p, c->poff.p, c->S, dt_host ? c->dts.p : nullptr,
-                    dt_all, c->nodes.p, c->kin.p, c->t_sys.p, c->t_nnodes.p, (int)c->N, c->ncap, s);
+                    dt_all, c->nodes.p, c->kin.p, c->t_sys.p, (const int *)c->t_state.p, (int)c->N, c->ncap, s);
     GG_CUDA_TRY(cudaGetLastError());
     return GG_OK;
 }

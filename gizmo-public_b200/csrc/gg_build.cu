@@ -92,27 +92,28 @@ __device__ __forceinline__ void tb_st_status(unsigned *p, unsigned v)
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 #define TB_PUBLISHED 0x80000000u
-#define TB_SPIN_LIMIT (1 << 22)
 
 // Barrier of the whole (cooperatively launched) grid: the blocks count up one
 // word, and the n-th barrier is passed once n * gridDim.x have arrived.  A wait
 // that reaches its limit (some ten seconds: the first one may wait for other
 // streams' walks to make room for the whole grid) records GG_EBIT_SORT_TIMEOUT and
-// returns false; the block then leaves the kernel.
-#define TB_BARRIER_LIMIT (1 << 24)
-__device__ __forceinline__ bool tb_grid_barrier(unsigned *word, unsigned &target, int *err)
+// returns false; the block then leaves the kernel, so that later barriers give
+// up too and the number of nodes stays zero.
+__device__ __forceinline__ bool tb_grid_barrier(const TreeBuf &tb, int which, unsigned &target)
 {
     __syncthreads();
-    if (gridDim.x == 1) return true;
+    const unsigned extra = (unsigned)tb.wait_extra[which];
+    if (gridDim.x + extra == 1) return true;
     __shared__ int s_ok;
     if (threadIdx.x == 0) {
+        unsigned *const word = tb.barrier + which;
         target += gridDim.x;
         __threadfence();
         atomicAdd(word, 1u);
         int spins = 0;
-        while (tb_ld_status(word) < target && ++spins < TB_BARRIER_LIMIT) __nanosleep(20);
-        s_ok = spins < TB_BARRIER_LIMIT;
-        if (!s_ok) atomicOr(err, GG_EBIT_SORT_TIMEOUT);
+        while (tb_ld_status(word) < target + extra && ++spins < tb.wait_limit) __nanosleep(20);
+        s_ok = spins < tb.wait_limit;
+        if (!s_ok) atomicOr(tb.err, GG_EBIT_SORT_TIMEOUT);
         __threadfence();
     }
     __syncthreads();
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
         tb.depth_beg[0] = 0;
         tb.depth_beg[1] = S;
     }
-    if (!tb_grid_barrier(tb.barrier, target, tb.err)) return;
+    if (!tb_grid_barrier(tb, 0, target)) return;
 
     int lb = 0, le = S, depth = 0;
     const int g = tid / TB_GROUP, j = tid % TB_GROUP;
@@ -241,12 +242,14 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
 
             // ---- this block's first child index: the totals of the blocks before it
             int before = 0;
+            bool lost = false;
             for (int i = tid; i < blk; i += TB_THREADS) {
                 unsigned v = tb_ld_status(bstat + i);
                 int spins = 0;
                 while (!(v & TB_PUBLISHED)) {
-                    if (++spins > TB_SPIN_LIMIT) {
+                    if (++spins > tb.wait_limit) {
                         atomicOr(tb.err, GG_EBIT_SORT_TIMEOUT);
+                        lost = true;
                         break;
                     }
                     __nanosleep(20);
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
             }
             before = __reduce_add_sync(0xffffffffu, before);
             if ((tid & 31) == 0) s_red[tid >> 5] = before;
-            __syncthreads();
+            if (__syncthreads_or(lost)) return;   // without the total the children's places are not known
             if (tid == 0) {
                 int off = 0;
                 for (int w = 0; w < TB_THREADS / 32; w++) off += s_red[w];
@@ -268,7 +271,6 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
                         nxt = tb.cap;
                     }
                     tb.depth_beg[depth + 2] = (int)nxt;
-                    tb.nnodes[0] = (int)nxt;
                 }
             }
             __syncthreads();   // also orders this block's count-phase stores before the reads below
@@ -336,12 +338,17 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
                 }
             }
         }
-        if (!tb_grid_barrier(tb.barrier, target, tb.err)) return;
+        if (!tb_grid_barrier(tb, 0, target)) return;
         lb = le;
         le = __ldcg(tb.depth_beg + depth + 2);
         if (le <= lb || depth + 1 >= GG_MAX_DEPTH) break;   // no nodes at the next depth
     }
-    if (gtid == 0) tb.nnodes[1] = depth;   // the deepest depth: all leaves
+    // every node is written; after a wait that gave up or an overflow (its nodes
+    // point past the capacity) the number of nodes stays zero
+    if (gtid == 0 && !(__ldcg(tb.err) & (GG_EBIT_SORT_TIMEOUT | GG_EBIT_NODE_OVERFLOW))) {
+        tb.nnodes[0] = le;
+        tb.nnodes[1] = depth;   // the deepest depth: all leaves
+    }
 }
 
 // Moments, in one cooperative launch: every leaf sums its particles, then one
@@ -353,8 +360,11 @@ __global__ void __launch_bounds__(TB_THREADS, TB_MOM_PER_SM)
     k_tree_moments(TreeBuf tb, const GGPart *__restrict__ parts, const GGDomainDev *__restrict__ dom, GGNode *nodes)
 {
     const int gtid = blockIdx.x * TB_THREADS + threadIdx.x, gthreads = gridDim.x * TB_THREADS;
-    // (clamped: the node kernel leaves them unset when a wait of its own gave up)
-    const int total = min(tb.nnodes[0], tb.cap), depth = min(max(tb.nnodes[1], 0), GG_MAX_DEPTH - 1);
+    __shared__ int s_total;
+    if (threadIdx.x == 0) s_total = __ldcg(tb.nnodes);
+    __syncthreads();
+    const int total = s_total, depth = tb.nnodes[1];
+    if (total == 0) return;   // no tree
     unsigned target = 0;
     for (int k = gtid; k < total; k += gthreads) {
         if (tb.child[k] >= 0) continue;
@@ -372,7 +382,10 @@ __global__ void __launch_bounds__(TB_THREADS, TB_MOM_PER_SM)
     }
     // internal nodes, deepest first
     for (int d = depth - 1; d >= 0; d--) {
-        if (!tb_grid_barrier(tb.barrier + 1, target, tb.err)) return;
+        if (!tb_grid_barrier(tb, 1, target)) {
+            if (threadIdx.x == 0) *(volatile int *)tb.nnodes = 0;   // unfinished nodes are not to be read
+            return;
+        }
         const int db = __ldcg(tb.depth_beg + d), de = __ldcg(tb.depth_beg + d + 1);
         for (int k = db + gtid; k < de; k += gthreads) {
             const int c0 = tb.child[k];
@@ -415,8 +428,7 @@ gg_status gg_launch_tree(const unsigned long long *keys, const int *poff, int S,
     const int G = (int)std::min((long long)gg_tree_grid(), want);
     const int Gm = (int)std::min((long long)gg_num_sms() * TB_MOM_PER_SM, want);
     tb.cap = cap;
-    GG_CUDA_TRY(cudaMemsetAsync(tb.bstat, 0, ((size_t)GG_MAX_DEPTH * G + 2) * sizeof(unsigned), st));
-    tb.barrier = tb.bstat + (size_t)GG_MAX_DEPTH * G;
+    GG_CUDA_TRY(cudaMemsetAsync(tb.nnodes, 0, TREE_STATE_WORDS(G) * sizeof(unsigned), st));
     void *args[] = {&keys, &poff, &S, &tb, &leaf};
     GG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_tree_nodes, dim3(G), dim3(TB_THREADS), args, 0, st));
     void *margs[] = {&tb, &parts, &dom, &nodes};

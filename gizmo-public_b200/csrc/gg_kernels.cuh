@@ -12,12 +12,19 @@ struct TreeBuf {
     int *bnd;          // 8 digit boundaries per node
     double *mass64;    // FP64 node mass (parent sums)
     int *depth_beg;    // GG_MAX_DEPTH + 2 entries
-    int *nnodes;       // total nodes, deepest depth (device)
-    unsigned *bstat;   // per depth and block: published children totals (GG_MAX_DEPTH x grid), then two barrier words
-    unsigned *barrier; // set by gg_launch_tree
+    int *nnodes;       // total nodes, deepest depth (device); zero until the node kernel has written every node, and
+                       // again when the moments are given up: whatever reads the nodes takes their number from here
+    unsigned *barrier; // two barrier words
+    unsigned *bstat;   // per depth and block: published children totals (GG_MAX_DEPTH x grid)
     int cap;           // node capacity (set by gg_launch_tree)
     int *err;
+    int wait_limit;    // polls after which a wait between blocks gives up
+    int wait_extra[2]; // arrivals that the node and the moments kernel's barriers wait for in vain (self-test; else 0)
 };
+
+#define TREE_WAIT_LIMIT (1 << 24)
+// TreeBuf's nnodes, barrier and bstat lie in one array, cleared before each build
+#define TREE_STATE_WORDS(grid) (4 + (size_t)GG_MAX_DEPTH * (grid))
 
 size_t gg_extent_words(int S);   // 64-bit words of gg_launch_extent's scratch mm
 void gg_launch_extent(const GGPart *rec, int n, const int *poff, int S, unsigned long long *mm, unsigned *hmm,
@@ -88,6 +95,7 @@ struct WalkFork {
 
 struct WalkParams {
     const GGNode *nodes;
+    const int *nnodes;          // 0: there is no complete tree, and nothing is walked
     const GGPart *parts;        // sorted
     const GGGroup *groups;
     const int *ngroups;         // device count

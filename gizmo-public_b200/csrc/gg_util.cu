@@ -270,7 +270,8 @@ __device__ __forceinline__ void gt_publish(unsigned *p, unsigned v)
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__global__ void __launch_bounds__(GT_THREADS) k_groups_tree(int nt, const int *__restrict__ tlist,
+__global__ void __launch_bounds__(GT_THREADS) k_groups_tree(const int *__restrict__ nnodes, int nt,
+                                                            const int *__restrict__ tlist,
                                                             const int *__restrict__ gnode, const int *__restrict__ toff,
                                                             int S, int gs, int maxg, unsigned *__restrict__ stat,
                                                             GGGroup *__restrict__ groups, int *__restrict__ ngroups,
@@ -279,7 +280,8 @@ __global__ void __launch_bounds__(GT_THREADS) k_groups_tree(int nt, const int *_
     __shared__ int ws[33];
     __shared__ int s_tile, s_carry, s_before, s_wmax[GT_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    nt = min(nt, toff[S]);   // fewer when the list of active particles had invalid or repeated indices
+    // fewer when the list of active particles had invalid or repeated indices; none without a complete tree
+    nt = *nnodes ? min(nt, toff[S]) : 0;
     const int ntiles = max(1, (nt + GT_TILE - 1) / GT_TILE);
     unsigned *const seg = stat + 1, *const cnt = seg + ntiles;   // per tile: last segment start + 1, group counts
     if (tid == 0) s_tile = (int)atomicAdd(stat, 1u);
@@ -401,8 +403,8 @@ void gg_launch_groups_tree(int nt, const int *tlist, const int *tscan, const int
     }
     cudaMemsetAsync(gstat, 0, gg_group_stat_words(nt) * sizeof(unsigned), st);
     k_group_nodes<<<gg_num_sms() * 8, 256, 0, st>>>(tb, tscan, gs, order_dom, hmm, lmax, gnode);
-    k_groups_tree<<<(nt + GT_TILE - 1) / GT_TILE, GT_THREADS, 0, st>>>(nt, tlist, gnode, toff, S, gs, maxg, gstat, groups,
-                                                                       ngroups, err);
+    k_groups_tree<<<(nt + GT_TILE - 1) / GT_TILE, GT_THREADS, 0, st>>>(tb.nnodes, nt, tlist, gnode, toff, S, gs, maxg, gstat,
+                                                                       groups, ngroups, err);
     gg_note_launches(2);
 }
 

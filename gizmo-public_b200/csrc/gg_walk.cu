@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
     unsigned phase = 0;   // parity of the barrier phase the next wait is for
     constexpr bool tma = TMA;   // node staging by bulk copies (else per-lane cp.async)
     int *gstack = p.stack + (size_t)(blockIdx.x * WALK_WARPS + warp) * p.stack_cap;
-    const int ngroups = *p.ngroups;
+    const int ngroups = *p.nnodes ? *p.ngroups : 0;
     const double theta = p.theta;
 
     for (;;) {

@@ -117,6 +117,7 @@ def load_library():
             "gg_radix_sort_pairs_noalloc": (i32, [i64, P, P, i32, P]),
             "gg_kernel_launches": (i64, []),
             "gg_selftest_bounded_wait": (i32, [P]),
+            "gg_selftest_tree_wait": (i32, [P, i32]),
             "gg_load_velocities": (i32, [P, P, i64]),
             "gg_load_velocities_device": (i32, [P, P]),
             "gg_drift": (i32, [P, dbl]),

@@ -49,3 +49,47 @@ def test_every_particle_is_in_the_tree_once(sizes, duplicates):
         want = mass[a:b].sum() * d / np.linalg.norm(d) ** 3
         # FP32 offset, 1/r and mass: a few roundings of 6e-8
         assert np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("group_size", [1, 32])
+@pytest.mark.parametrize("kernel", [0, 1])
+def test_a_build_whose_waits_give_up_leaves_no_tree(kernel, group_size):
+    """The node kernel's (0) or the moments kernel's (1) blocks wait for one
+    block more than there are.  Nothing reads the unfinished tree, neither in a
+    context's first build nor over an earlier tree, and the next build is
+    whole again."""
+    import ctypes
+
+    import torch
+    sizes = [3000, 0, 40000]
+    parts = [_system(n, 50 + i, False) for i, n in enumerate(sizes)]
+    pos, mass, h = (np.concatenate([p[k] for p in parts]) for k in range(3))
+    n = len(mass)
+    with ggb200.GravityTree(group_size=group_size) as t:
+        t.load(pos, mass, h, counts=sizes)
+        t.build()
+        want = t.evaluate(err_tol_theta=0.7)[0]
+
+    def status(t):
+        st = ggb200.Stats()
+        return t._lib.gg_last_stats(t._h, ctypes.byref(st)), st
+
+    with ggb200.GravityTree(group_size=group_size) as t:
+        for first in (True, False):
+            t.load(pos, mass, h, counts=sizes)
+            t.load_velocities(np.ones((n, 3)))
+            assert t._lib.gg_selftest_tree_wait(t._h, kernel) == -5      # GG_ERR_TIMEOUT
+            if not first:      # a resident tree is moved by the drift; one that is not whole is left alone
+                t.drift(1e-3)
+            acc = torch.full((n, 3), 7.0, dtype=torch.float64, device="cuda")
+            pot = torch.full((n,), 7.0, dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            t.evaluate_device(acc, pot, err_tol_theta=0.7)
+            t.evaluate_potential_device(pot, err_tol_theta=0.7)
+            code, st = status(t)
+            assert code == -5 and st.n_nodes == 0 and st.interactions == 0 and st.nodes_tested == 0
+            assert bool((acc == 7.0).all()) and bool((pot == 7.0).all())
+            t.load(pos, mass, h, counts=sizes)
+            t.build()
+            got = t.evaluate(err_tol_theta=0.7)[0]
+            assert np.array_equal(got, want)
