@@ -216,7 +216,7 @@ struct gg_ctx {
     // tree
     int ncap = 0;
     DevBuf<int> t_start, t_end, t_level, t_parent, t_sys, t_nch, t_child, t_bnd, t_depth;
-    DevBuf<unsigned> t_state;             // node count, barrier words, look-back words of the tree kernels
+    DevBuf<unsigned> t_state;             // node count, tickets, wait and look-back words of the tree kernels
     DevBuf<double> t_mass64;
     DevBuf<GGNode> nodes;
     // walk
@@ -626,14 +626,15 @@ static TreeBuf tree_buf(gg_ctx *c)
     tb.start = c->t_start.p; tb.end = c->t_end.p; tb.level = c->t_level.p; tb.parent = c->t_parent.p;
     tb.sys = c->t_sys.p; tb.nch = c->t_nch.p; tb.child = c->t_child.p;
     tb.bnd = c->t_bnd.p; tb.mass64 = c->t_mass64.p; tb.depth_beg = c->t_depth.p; tb.nnodes = (int *)c->t_state.p;
-    tb.barrier = c->t_state.p + 2; tb.bstat = c->t_state.p + 4; tb.err = c->err.p;
+    tb.ticket = c->t_state.p + 2; tb.done = c->t_state.p + 4; tb.bstat = tb.done + 2 * TREE_PHASES;
+    tb.err = c->err.p;
     tb.cap = c->ncap;
     tb.wait_limit = TREE_WAIT_LIMIT;
     tb.wait_extra[0] = tb.wait_extra[1] = 0;
     return tb;
 }
 
-// vain: a self-test's tree kernel (0 nodes, 1 moments) whose barriers wait for one arrival too many, else -1
+// vain: a self-test's tree kernel (0 nodes, 1 moments) whose waits count one part too many, else -1
 static gg_status build(gg_ctx *c, const gg_domain *domains, int vain)
 {
     if (!c || c->S < 1) return GG_ERR_INVALID;

@@ -92,32 +92,71 @@ __device__ __forceinline__ void tb_st_status(unsigned *p, unsigned v)
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 #define TB_PUBLISHED 0x80000000u
+#define TB_GIVEN_UP 0x80000000u
 
-// Barrier of the whole (cooperatively launched) grid: the blocks count up one
-// word, and the n-th barrier is passed once n * gridDim.x have arrived.  A wait
-// that reaches its limit (some ten seconds: the first one may wait for other
-// streams' walks to make room for the whole grid) records GG_EBIT_SORT_TIMEOUT and
-// returns false; the block then leaves the kernel, so that later barriers give
-// up too and the number of nodes stays zero.
-__device__ __forceinline__ bool tb_grid_barrier(const TreeBuf &tb, int which, unsigned &target)
+// How the blocks of a tree kernel work together.  Each depth (each phase of the
+// moments) is cut into parts, at most one per block of the grid, and a block
+// takes one part after the other by ticket: all parts of a depth, then those of
+// the next.  A part waits only for parts with earlier tickets, which are
+// finished or held by a block that runs and whose earlier part is finished: so
+// however few blocks find room beside other kernels, the first unfinished part
+// can always go on.  (A grid barrier needs every block resident at once: a
+// kernel of another stream that holds a single warp slot kept a build of 600,000
+// particles from starting.)
+//
+// `first` (shared memory, thread 0's) is the ticket of the phase's first part, and
+// a block's place its ticket less that.  tb_step ends a block's turn at a phase of
+// `parts` parts: the part it worked on is counted as finished and its next ticket
+// taken; if that is not of this phase, it waits until all parts are finished and
+// goes on to the next phase (*moved).  It returns the new place, or -1 after a wait
+// that reached its limit (some ten seconds): that one records
+// GG_EBIT_SORT_TIMEOUT and marks the word, so that the others leave too; the
+// number of nodes stays zero.
+__device__ __forceinline__ int tb_step(const TreeBuf &tb, int kernel, int phase, int parts, int &first, int place,
+                                       bool *moved)
 {
+    __shared__ int s_place, s_moved;
     __syncthreads();
-    const unsigned extra = (unsigned)tb.wait_extra[which];
-    if (gridDim.x + extra == 1) return true;
-    __shared__ int s_ok;
+    if (gridDim.x + tb.wait_extra[kernel] == 1) {   // one block, one part per phase, nobody to wait for
+        *moved = true;
+        return 0;
+    }
     if (threadIdx.x == 0) {
-        unsigned *const word = tb.barrier + which;
-        target += gridDim.x;
-        __threadfence();
-        atomicAdd(word, 1u);
-        int spins = 0;
-        while (tb_ld_status(word) < target + extra && ++spins < tb.wait_limit) __nanosleep(20);
-        s_ok = spins < tb.wait_limit;
-        if (!s_ok) atomicOr(tb.err, GG_EBIT_SORT_TIMEOUT);
-        __threadfence();
+        unsigned *const word = tb.done + kernel * TREE_PHASES + phase;
+        const unsigned want = (unsigned)(parts + tb.wait_extra[kernel]);
+        int next = first + place;
+        if (place < parts) {
+            __threadfence();
+            atomicAdd(word, 1u);
+            next = (int)atomicAdd(tb.ticket + kernel, 1u);
+        }
+        unsigned v = tb_ld_status(word);   // in flight together with the ticket
+        const bool over = next - first >= parts;
+        if (over) first += parts;
+        s_place = next - first;
+        s_moved = over;
+        if (over) {
+            int spins = 0;
+            while (v < want && ++spins < tb.wait_limit) {   // (the mark ends it)
+                __nanosleep(20);
+                v = tb_ld_status(word);
+            }
+            if (v < want) {
+                atomicOr(tb.err, GG_EBIT_SORT_TIMEOUT);
+                atomicOr(word, TB_GIVEN_UP);
+            }
+            if (v < want || (v & TB_GIVEN_UP)) s_place = -1;
+            __threadfence();
+        }
     }
     __syncthreads();
-    return s_ok != 0;
+    *moved = s_moved;
+    return s_place;
+}
+// a block's first ticket
+__device__ __forceinline__ int tb_first(const TreeBuf &tb, int kernel)
+{
+    return gridDim.x == 1 ? 0 : (int)atomicAdd(tb.ticket + kernel, 1u);
 }
 
 // node k's record and FP64 mass from its sums
@@ -153,21 +192,21 @@ __device__ __forceinline__ void tb_finish_node(int k, const TreeBuf &tb, const G
     tb.mass64[k] = M;
 }
 
-// The tree's nodes in one cooperative launch: roots, then one depth after the
-// other.  Every dependence between blocks is a grid barrier (about 1.5 us)
-// instead of a kernel boundary, and the loop stops at the tree's own depth.  One
-// launch per depth and direction made 57 launches, most of them of empty depths
-// in a small tree.  Tree and moments together, B200: 1,000 particles 352 -> 62 us,
-// 65,536 430 -> 171, 16.8M 2.02 -> 1.82 ms (in one launch of both, at 64 registers and
-// half the threads per SM, 2.34 ms).
+// The tree's nodes in one launch: one depth after the other, down to the tree's
+// own depth.  A wait between two depths costs about 1.5 us instead of a kernel
+// boundary; one launch per depth and direction made 57 launches, most of them
+// of empty depths in a small tree.  Tree and moments together, B200: 1,000
+// particles 352 -> 63 us, 65,536 430 -> 176, 16.8M 2.02 -> 1.78 ms (in one launch of
+// both, at 64 registers and half the threads per SM, 2.34 ms; with a grid barrier
+// instead of the tickets 60 us, 170, 1.81).
 //
 // One depth: 8 threads per node find the 7 digit boundaries by binary search
 // (or the chunk split of a full-depth cell) and the child count; a block
-// publishes its children total, adds up the totals of the blocks before it
-// (they publish before they wait on anyone) and writes its nodes' children at
-// contiguous indices from there.  The last block with nodes sets the next
-// depth's range.  A child index at or past the node capacity is not written and
-// sets GG_EBIT_NODE_OVERFLOW (the capacity is sized so that it cannot happen).
+// publishes its part's children total, adds up the totals of the parts before it
+// (published before their blocks wait on anyone) and writes its nodes' children at
+// contiguous indices from there.  The last part sets the next depth's range.  A
+// child index at or past the node capacity is not written and sets
+// GG_EBIT_NODE_OVERFLOW (the capacity is sized so that it cannot happen).
 __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
     k_tree_nodes(const unsigned long long *__restrict__ keys, const int *__restrict__ poff, int S, TreeBuf tb, int leaf)
 {
@@ -175,33 +214,37 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
     __shared__ int s_red[TB_THREADS / 32];
     __shared__ int s_nch[TB_NODES];
     __shared__ int s_excl[TB_NODES];
-    const int G = gridDim.x, blk = blockIdx.x, tid = threadIdx.x;
-    const int gtid = blk * TB_THREADS + tid, gthreads = G * TB_THREADS;
-    unsigned target = 0;
-
-    // roots: one per system, geometric level 0 (the domain cube), depth 0
-    for (int s = gtid; s < S; s += gthreads) {
-        tb.start[s] = poff[s];
-        tb.end[s] = poff[s + 1];
-        tb.level[s] = 0;
-        tb.parent[s] = -1;
-        tb.sys[s] = s;
-    }
-    if (gtid == 0) {
-        tb.depth_beg[0] = 0;
-        tb.depth_beg[1] = S;
-    }
-    if (!tb_grid_barrier(tb, 0, target)) return;
-
-    int lb = 0, le = S, depth = 0;
+    const int G = gridDim.x, tid = threadIdx.x;
     const int g = tid / TB_GROUP, j = tid % TB_GROUP;
     const int gbase = (tid & 31) & ~(TB_GROUP - 1);
-    for (;; depth++) {   // depths 0 .. GG_MAX_DEPTH - 1; the last is all leaves
+    int lb = 0, le = S, depth = 0;   // nodes lb to le - 1 of a depth; depths 0 .. GG_MAX_DEPTH - 1, the last all leaves
+    __shared__ int s_first;
+    if (tid == 0) {
+        s_first = 0;
+        s_tot = tb_first(tb, 0);
+    }
+    __syncthreads();
+    int blk = s_tot;   // place in the depth
+    for (;;) {
         const int nl = le - lb;
-        const int chunk = max((nl + G - 1) / G, TB_NODES);   // nodes per block: whole passes of the block
-        const int cb = lb + blk * chunk, ce = min(le, cb + chunk);
-        if (cb < le) {
+        const int chunk = max((nl + G - 1) / G, TB_NODES);   // nodes per part: whole passes of the block
+        const int parts = (nl + chunk - 1) / chunk;
+        if (blk < parts) {
+            const int cb = lb + blk * chunk, ce = min(le, cb + chunk);
             const bool one = chunk <= TB_NODES;   // one node per 8 threads: boundaries stay in registers
+            if (depth == 0) {   // roots: one per system, geometric level 0 (the domain cube)
+                for (int s = cb + tid; s < ce; s += TB_THREADS) {
+                    tb.start[s] = poff[s];
+                    tb.end[s] = poff[s + 1];
+                    tb.level[s] = 0;
+                    tb.parent[s] = -1;
+                    tb.sys[s] = s;
+                }
+                if (tid == 0 && blk == 0) {
+                    tb.depth_beg[0] = 0;
+                    tb.depth_beg[1] = S;
+                }
+            }
             if (tid == 0) s_sum = 0;
             __syncthreads();
 
@@ -240,7 +283,7 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
             unsigned *const bstat = tb.bstat + (size_t)depth * G;
             if (tid == 0) tb_st_status(bstat + blk, TB_PUBLISHED | (unsigned)s_sum);
 
-            // ---- this block's first child index: the totals of the blocks before it
+            // ---- this part's first child index: the totals of the parts before it
             int before = 0;
             bool lost = false;
             for (int i = tid; i < blk; i += TB_THREADS) {
@@ -259,12 +302,15 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
             }
             before = __reduce_add_sync(0xffffffffu, before);
             if ((tid & 31) == 0) s_red[tid >> 5] = before;
-            if (__syncthreads_or(lost)) return;   // without the total the children's places are not known
+            if (__syncthreads_or(lost)) {   // without the total the children's places are not known
+                if (tid == 0) atomicOr(tb.done + depth, TB_GIVEN_UP);
+                return;
+            }
             if (tid == 0) {
                 int off = 0;
                 for (int w = 0; w < TB_THREADS / 32; w++) off += s_red[w];
                 s_off = off;
-                if (ce == le) {   // the last block with nodes: the depth's total is known
+                if (ce == le) {   // the last part: the depth's total is known
                     long long nxt = (long long)le + off + s_sum;
                     if (nxt > tb.cap) {
                         atomicOr(tb.err, GG_EBIT_NODE_OVERFLOW);
@@ -273,7 +319,7 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
                     tb.depth_beg[depth + 2] = (int)nxt;
                 }
             }
-            __syncthreads();   // also orders this block's count-phase stores before the reads below
+            __syncthreads();   // also orders this part's count-phase stores before the reads below
 
             // ---- write
             int run = le + s_off;
@@ -338,20 +384,25 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
                 }
             }
         }
-        if (!tb_grid_barrier(tb, 0, target)) return;
-        lb = le;
-        le = __ldcg(tb.depth_beg + depth + 2);
-        if (le <= lb || depth + 1 >= GG_MAX_DEPTH) break;   // no nodes at the next depth
+        bool moved;
+        blk = tb_step(tb, 0, depth, parts, s_first, blk, &moved);
+        if (blk < 0) return;
+        if (moved) {
+            depth++;
+            lb = le;
+            le = __ldcg(tb.depth_beg + depth + 1);
+            if (le <= lb || depth >= GG_MAX_DEPTH) break;   // no nodes at the next depth
+        }
     }
     // every node is written; after a wait that gave up or an overflow (its nodes
     // point past the capacity) the number of nodes stays zero
-    if (gtid == 0 && !(__ldcg(tb.err) & (GG_EBIT_SORT_TIMEOUT | GG_EBIT_NODE_OVERFLOW))) {
-        tb.nnodes[0] = le;
-        tb.nnodes[1] = depth;   // the deepest depth: all leaves
+    if (blk == 0 && tid == 0 && !(__ldcg(tb.err) & (GG_EBIT_SORT_TIMEOUT | GG_EBIT_NODE_OVERFLOW))) {
+        tb.nnodes[0] = lb;
+        tb.nnodes[1] = depth - 1;   // the deepest depth: all leaves
     }
 }
 
-// Moments, in one cooperative launch: every leaf sums its particles, then one
+// Moments, in one launch: every leaf sums its particles, then one
 // depth after the other from the deepest up, an internal node sums its
 // children, each in index order in FP64.  Nodes are numbered depth by depth
 // with the children of consecutive nodes consecutive, so the lanes of a warp
@@ -359,50 +410,60 @@ __global__ void __launch_bounds__(TB_THREADS, TB_PER_SM)
 __global__ void __launch_bounds__(TB_THREADS, TB_MOM_PER_SM)
     k_tree_moments(TreeBuf tb, const GGPart *__restrict__ parts, const GGDomainDev *__restrict__ dom, GGNode *nodes)
 {
-    const int gtid = blockIdx.x * TB_THREADS + threadIdx.x, gthreads = gridDim.x * TB_THREADS;
-    __shared__ int s_total;
-    if (threadIdx.x == 0) s_total = __ldcg(tb.nnodes);
-    __syncthreads();
-    const int total = s_total, depth = tb.nnodes[1];
-    if (total == 0) return;   // no tree
-    unsigned target = 0;
-    for (int k = gtid; k < total; k += gthreads) {
-        if (tb.child[k] >= 0) continue;
-        double M = 0, sx = 0, sy = 0, sz = 0;
-        float maxsoft = 0;
-        const int s = tb.start[k], e = tb.end[k];
-        for (int i = s; i < e; i++) {
-            const GGPart p = parts[i];
-            const double m = (double)p.m;
-            M += m;
-            sx += m * p.x; sy += m * p.y; sz += m * p.z;
-            maxsoft = fmaxf(maxsoft, p.h);
-        }
-        tb_finish_node(k, tb, parts, dom, nodes, M, sx, sy, sz, maxsoft, s, -(e - s));
+    __shared__ int s_total, s_ticket, s_first;
+    if (threadIdx.x == 0) {
+        s_first = 0;
+        s_total = __ldcg(tb.nnodes);
+        s_ticket = tb_first(tb, 1);
     }
-    // internal nodes, deepest first
-    for (int d = depth - 1; d >= 0; d--) {
-        if (!tb_grid_barrier(tb, 1, target)) {
+    __syncthreads();
+    const int depth = tb.nnodes[1];
+    int place = s_ticket;
+    if (s_total == 0) return;   // no tree
+    // phase 0: the leaves of every depth; phase p: the internal nodes of depth `depth - p`
+    for (int phase = 0;;) {
+        const int kb = phase == 0 ? 0 : tb.depth_beg[depth - phase];
+        const int ke = phase == 0 ? s_total : tb.depth_beg[depth - phase + 1];
+        const int nparts = min((int)gridDim.x, (ke - kb + TB_THREADS - 1) / TB_THREADS);
+        if (place < nparts) {
+            for (int k = kb + place * TB_THREADS + threadIdx.x; k < ke; k += nparts * TB_THREADS) {
+                const int c0 = tb.child[k];
+                if ((c0 < 0) != (phase == 0)) continue;
+                double M = 0, sx = 0, sy = 0, sz = 0;
+                float maxsoft = 0;
+                if (phase == 0) {
+                    const int s = tb.start[k], e = tb.end[k];
+                    for (int i = s; i < e; i++) {
+                        const GGPart p = parts[i];
+                        const double m = (double)p.m;
+                        M += m;
+                        sx += m * p.x; sy += m * p.y; sz += m * p.z;
+                        maxsoft = fmaxf(maxsoft, p.h);
+                    }
+                    tb_finish_node(k, tb, parts, dom, nodes, M, sx, sy, sz, maxsoft, s, -(e - s));
+                } else {
+                    const int nc = tb.nch[k];
+                    for (int c = c0; c < c0 + nc; c++) {   // written by other blocks of this launch: read through L2
+                        const double m = __ldcg(tb.mass64 + c);
+                        const double2 xy = __ldcg(reinterpret_cast<const double2 *>(&nodes[c].cx));
+                        const double z = __ldcg(&nodes[c].cz);
+                        M += m;
+                        sx += m * xy.x; sy += m * xy.y; sz += m * z;
+                        maxsoft = fmaxf(maxsoft, __ldcg(&nodes[c].maxsoft));
+                    }
+                    tb_finish_node(k, tb, parts, dom, nodes, M, sx, sy, sz, maxsoft, c0, nc);
+                }
+            }
+        } else if (phase == depth) {
+            return;
+        }
+        bool moved;
+        place = tb_step(tb, 1, phase, nparts, s_first, place, &moved);
+        if (place < 0) {
             if (threadIdx.x == 0) *(volatile int *)tb.nnodes = 0;   // unfinished nodes are not to be read
             return;
         }
-        const int db = __ldcg(tb.depth_beg + d), de = __ldcg(tb.depth_beg + d + 1);
-        for (int k = db + gtid; k < de; k += gthreads) {
-            const int c0 = tb.child[k];
-            if (c0 < 0) continue;
-            double M = 0, sx = 0, sy = 0, sz = 0;
-            float maxsoft = 0;
-            const int nc = tb.nch[k];
-            for (int c = c0; c < c0 + nc; c++) {   // written by other blocks of this launch: read through L2
-                const double m = __ldcg(tb.mass64 + c);
-                const double2 xy = __ldcg(reinterpret_cast<const double2 *>(&nodes[c].cx));
-                const double z = __ldcg(&nodes[c].cz);
-                M += m;
-                sx += m * xy.x; sy += m * xy.y; sz += m * z;
-                maxsoft = fmaxf(maxsoft, __ldcg(&nodes[c].maxsoft));
-            }
-            tb_finish_node(k, tb, parts, dom, nodes, M, sx, sy, sz, maxsoft, c0, nc);
-        }
+        if (moved && phase++ == depth) return;
     }
 }
 
@@ -421,18 +482,17 @@ int gg_tree_grid() { return gg_num_sms() * TB_PER_SM; }
 gg_status gg_launch_tree(const unsigned long long *keys, const int *poff, int S, int n, int leaf, int cap, TreeBuf tb,
                          const GGPart *parts, const GGDomainDev *dom, GGNode *nodes, cudaStream_t st)
 {
-    // about 1,024 particles per block: few blocks for a small tree, as a barrier
-    // of one block costs nothing (1,000 particles: 53 us in one block, 76 us in
+    // about 1,024 particles per block: few blocks for a small tree, as the waits
+    // of one block cost nothing (1,000 particles: 53 us in one block, 76 us in
     // two; 65,536: 165 us in 64 blocks, 192 us in 16)
     const long long want = ((long long)n + S + 1023) / 1024;
     const int G = (int)std::min((long long)gg_tree_grid(), want);
     const int Gm = (int)std::min((long long)gg_num_sms() * TB_MOM_PER_SM, want);
     tb.cap = cap;
     GG_CUDA_TRY(cudaMemsetAsync(tb.nnodes, 0, TREE_STATE_WORDS(G) * sizeof(unsigned), st));
-    void *args[] = {&keys, &poff, &S, &tb, &leaf};
-    GG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_tree_nodes, dim3(G), dim3(TB_THREADS), args, 0, st));
-    void *margs[] = {&tb, &parts, &dom, &nodes};
-    GG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_tree_moments, dim3(Gm), dim3(TB_THREADS), margs, 0, st));
+    k_tree_nodes<<<G, TB_THREADS, 0, st>>>(keys, poff, S, tb, leaf);
+    k_tree_moments<<<Gm, TB_THREADS, 0, st>>>(tb, parts, dom, nodes);
+    GG_CUDA_TRY(cudaGetLastError());
     gg_note_launches(2);
     return GG_OK;
 }

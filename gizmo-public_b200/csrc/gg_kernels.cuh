@@ -14,17 +14,19 @@ struct TreeBuf {
     int *depth_beg;    // GG_MAX_DEPTH + 2 entries
     int *nnodes;       // total nodes, deepest depth (device); zero until the node kernel has written every node, and
                        // again when the moments are given up: whatever reads the nodes takes their number from here
-    unsigned *barrier; // two barrier words
-    unsigned *bstat;   // per depth and block: published children totals (GG_MAX_DEPTH x grid)
+    unsigned *ticket;  // parts handed out: node kernel, moments kernel
+    unsigned *done;    // finished parts per depth of the node kernel, per phase of the moments kernel (TREE_PHASES each)
+    unsigned *bstat;   // per depth and part: published children totals (GG_MAX_DEPTH x grid)
     int cap;           // node capacity (set by gg_launch_tree)
     int *err;
     int wait_limit;    // polls after which a wait between blocks gives up
-    int wait_extra[2]; // arrivals that the node and the moments kernel's barriers wait for in vain (self-test; else 0)
+    int wait_extra[2]; // parts that the node and the moments kernel's waits count in vain (self-test; else 0)
 };
 
 #define TREE_WAIT_LIMIT (1 << 24)
-// TreeBuf's nnodes, barrier and bstat lie in one array, cleared before each build
-#define TREE_STATE_WORDS(grid) (4 + (size_t)GG_MAX_DEPTH * (grid))
+#define TREE_PHASES (GG_MAX_DEPTH + 1)
+// TreeBuf's nnodes, ticket, done and bstat lie in one array, cleared before each build
+#define TREE_STATE_WORDS(grid) (4 + 2 * TREE_PHASES + (size_t)GG_MAX_DEPTH * (grid))
 
 size_t gg_extent_words(int S);   // 64-bit words of gg_launch_extent's scratch mm
 void gg_launch_extent(const GGPart *rec, int n, const int *poff, int S, unsigned long long *mm, unsigned *hmm,

@@ -51,9 +51,10 @@ def test_every_particle_is_in_the_tree_once(sizes, duplicates):
         assert np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("sizes", [[300], [3000, 0, 40000]])
 @pytest.mark.parametrize("group_size", [1, 32])
 @pytest.mark.parametrize("kernel", [0, 1])
-def test_a_build_whose_waits_give_up_leaves_no_tree(kernel, group_size):
+def test_a_build_whose_waits_give_up_leaves_no_tree(kernel, group_size, sizes):
     """The node kernel's (0) or the moments kernel's (1) blocks wait for one
     block more than there are.  Nothing reads the unfinished tree, neither in a
     context's first build nor over an earlier tree, and the next build is
@@ -61,7 +62,6 @@ def test_a_build_whose_waits_give_up_leaves_no_tree(kernel, group_size):
     import ctypes
 
     import torch
-    sizes = [3000, 0, 40000]
     parts = [_system(n, 50 + i, False) for i, n in enumerate(sizes)]
     pos, mass, h = (np.concatenate([p[k] for p in parts]) for k in range(3))
     n = len(mass)
@@ -93,3 +93,33 @@ def test_a_build_whose_waits_give_up_leaves_no_tree(kernel, group_size):
             t.build()
             got = t.evaluate(err_tol_theta=0.7)[0]
             assert np.array_equal(got, want)
+
+
+def test_a_build_does_not_wait_for_other_kernels_to_end():
+    """A build large enough to take every thread slot of the GPU, next to a
+    kernel of another stream that holds one for about a second: the build ends
+    first, on the slots that are left."""
+    import torch
+    n = 800000
+    rng = np.random.default_rng(60)
+    rec = torch.from_numpy(ggb200.make_records(rng.normal(size=(n, 3)), np.ones(n), np.full(n, 1e-3)).view(np.uint8))
+    rec = rec.cuda()
+    mine, other, done = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Event()
+    acc = torch.empty((n, 3), dtype=torch.float64, device="cuda")
+    with ggb200.GravityTree() as t:
+        t.set_stream(mine.cuda_stream)
+        t.load_device(rec, [n])
+        t.build()
+        t.evaluate_device(acc, err_tol_theta=0.7)
+        torch.cuda.synchronize()
+        want = acc.clone()
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(2 * 10 ** 9)
+            done.record()
+        t.build()
+        mine.synchronize()
+        assert not done.query()
+        t.evaluate_device(acc, err_tol_theta=0.7)
+        torch.cuda.synchronize()
+        assert t.last_stats()["error_word"] == 0
+    assert torch.equal(acc, want)
