@@ -239,20 +239,20 @@ __global__ void k_group_nodes(TreeBuf tb, const int *__restrict__ tscan, int gs,
 }
 
 // Groups in one launch: a group starts at every gs-th target of a segment (a
-// run of consecutive targets of one group node).  Tiles of GT_TILE targets are
-// taken in ticket order.  A tile needs two things of its predecessors: the last
-// segment start before it (its own targets tell where segments start, so the
-// nearest tile with a start suffices), and then the number of groups before it.
-// Both are found by looking back over the words the predecessors publish, which
-// they do before they wait on anyone, so every wait ends; the waits are bounded
-// all the same.  (Two device-wide scans and four passes over the targets made ten
+// run of consecutive targets of one group node; it can be the whole system, see
+// group_node_pred).  Tiles of GT_TILE targets are taken in ticket order.  A tile
+// needs two things of its predecessors: the last segment start before it, and then
+// the number of groups before it.  Both are found by a warp looking back over the
+// words the predecessors publish, their own first, and the one up to and with
+// them once they know it.  They publish before they wait on anyone, so every wait
+// ends; the waits are bounded all the same.  (Two device-wide scans and four passes over the targets made ten
 // launches of this, about 35 us at 65,536 targets.)
 #define GT_THREADS 256
 #define GT_ITEMS 4
 #define GT_TILE (GT_THREADS * GT_ITEMS)
 #define GT_SPIN_LIMIT (1 << 22)
 #define GT_SET 0x80000000u        // the word is published
-#define GT_SUM 0x40000000u        // ... and holds the groups up to and with the tile, not the tile's own
+#define GT_SUM 0x40000000u        // ... and holds the last start, or the groups, up to and with the tile, not its own
 
 __device__ __forceinline__ unsigned gt_wait(const unsigned *p, int *err)
 {
@@ -316,11 +316,21 @@ __global__ void __launch_bounds__(GT_THREADS) k_groups_tree(const int *__restric
         tile_last = max(tile_last, s_wmax[i]);
     }
     // ---- the last segment start before the tile (target 0 starts one, so tile 0 has its own)
-    if (tid == 0) {
-        gt_publish(seg + tile, GT_SET | (unsigned)(tile_last + 1));
+    if (w == 0) {
+        if (lane == 0) gt_publish(seg + tile, GT_SET | (tile_last >= 0 ? GT_SUM : 0u) | (unsigned)(tile_last + 1));
         int c = -1;
-        for (int q = tile - 1; q >= 0 && c < 0; q--) c = (int)(gt_wait(seg + q, err) & 0x3fffffffu) - 1;
-        s_carry = c;
+        for (int q = tile - 1; q >= 0; q -= 32) {   // 32 predecessors at a time, up to the nearest that knows one
+            const unsigned v = q - lane >= 0 ? gt_wait(seg + q - lane, err) : GT_SET | GT_SUM;
+            const unsigned known = __ballot_sync(0xffffffffu, (v & GT_SUM) != 0);
+            if (known) {
+                c = (int)(__shfl_sync(0xffffffffu, v, __ffs(known) - 1) & 0x3fffffffu) - 1;
+                break;
+            }
+        }
+        if (lane == 0) {
+            if (tile_last < 0) gt_publish(seg + tile, GT_SET | GT_SUM | (unsigned)(c + 1));
+            s_carry = c;
+        }
     }
     __syncthreads();
     before = max(before, s_carry);

@@ -88,3 +88,36 @@ def test_group_count_matches_restatement(gs):
     assert full == expected_groups(keys, np.ones(n, bool), gs)
     assert sub == expected_groups(keys, is_act[order], gs)
     assert full > n // gs   # some group nodes end in partial groups
+
+
+@pytest.mark.gpu
+def test_one_segment_of_all_targets_takes_time_in_proportion():
+    """One particle's kernel radius is more than half the root cube: targets are
+    then ordered by softening class over the whole cube and form one segment, cut
+    into runs of the group size.  Eight times the targets take about eight times
+    as long (a look-back of one word at a time over all earlier tiles made it 14),
+    with a walk that uses the root's children at most."""
+    import torch
+    best = {}
+    for n in (1 << 20, 1 << 23):
+        gen = torch.Generator(device="cuda").manual_seed(73)
+        rec = torch.empty((n, 4), dtype=torch.float64, device="cuda")
+        rec[:, :3] = torch.rand((n, 3), dtype=torch.float64, device="cuda", generator=gen)
+        single = rec.view(torch.float32)
+        single[:, 6], single[:, 7] = 1.0, 1e-3
+        single[0, 7] = 0.9
+        acc = torch.empty((n, 3), dtype=torch.float64, device="cuda")
+        best[n] = 1e30
+        with ggb200.GravityTree() as t:
+            t.set_stream(torch.cuda.current_stream().cuda_stream)
+            t.load_device(rec, [n])
+            t.build()
+            for _ in range(6):
+                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                e0.record()
+                t.evaluate_device(acc, err_tol_theta=1e9)
+                e1.record()
+                torch.cuda.synchronize()
+                best[n] = min(best[n], e0.elapsed_time(e1))
+            assert t.last_stats()["n_groups"] == n // 32
+    assert best[1 << 23] < 10.0 * best[1 << 20], best
