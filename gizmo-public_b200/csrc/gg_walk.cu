@@ -406,8 +406,9 @@ __device__ __forceinline__ void flush_near(const float *__restrict__ near, int n
     add_sums<TPL, POT>(T, px, py, pz, pp);
 }
 
-// The same for groups of several kernel radii: h_g is formed per pair from the
-// entry's {h_source, 1/h_source, m}.
+// The same for groups of several kernel radii, or of one that near_one_radius
+// refuses: h_g is formed per pair from the entry's {h_source, 1/h_source, m}, and
+// Newtonian pairs have no part of it (any distance whose m/r^3 is an FP32 number).
 template <int TPL, int SPLIT, bool POT>
 __device__ __forceinline__ void flush_near_mixed(const float *__restrict__ near, int n, int part, Targets<TPL> &T)
 {
@@ -440,7 +441,7 @@ __device__ __forceinline__ void flush_near_mixed(const float *__restrict__ near,
             float2 fp = sel2(sx, sy, mul2(mul2(em, wp), hinv), make_float2(-mr.x, -mr.y));
             if (!POT) {
                 float2 fac =
-                    sel2(sx, sy, mul2(mul2(em, wf), mul2(mul2(hinv, hinv), hinv)), mul2(mul2(mr, rinv), rinv));
+                    sel2(sx, sy, mul2(mul2(em, wf), mul2(mul2(hinv, hinv), hinv)), mul2(mr, mul2(rinv, rinv)));
                 const bool ux = r2.x > 0.f, uy = r2.y > 0.f;
                 fac = sel2(ux, uy, fac, dup2(0.f));
                 fp = sel2(ux, uy, fp, dup2(0.f));
@@ -468,17 +469,26 @@ __device__ __forceinline__ void list_shift(float *list, int m, int r, int lane)
 }
 
 // Softening record of a near-list entry with kernel radius hsrc and mass m (see
-// flush_near).  hzero: the kernel radius that takes the place of zero, far below
-// the distances in the group's box, so that the products stay finite.
-__device__ __forceinline__ float4 near_soft(float hsrc, float m, bool homog, float hgroup, float hzero)
+// flush_near).  hone: the group's one kernel radius, negative if it takes the form
+// of several.  (A flag beside the radius cost the 16.8M walk 41.15 -> 41.82 ms.)
+__device__ __forceinline__ float4 near_soft(float hsrc, float m, float hone)
 {
-    if (homog) {
-        float hg = fmaxf(hgroup, hsrc);
-        if (hg == 0.f) hg = hzero;
-        const float hinv = __frcp_rn(hg);
-        return make_float4(hinv * hinv, m * hinv, m * (hinv * hinv * hinv), 0.f);
+    if (hone >= 0.f) {
+        const float hinv = __frcp_rn(fmaxf(hone, hsrc)), mh = m * hinv;
+        return make_float4(hinv * hinv, mh, mh * hinv * hinv, 0.f);
     }
     return make_float4(hsrc, hsrc > 0.f ? __frcp_rn(hsrc) : INFINITY, m, 0.f);
+}
+
+// Whether the near flush for one kernel radius h > 0 can take a group's
+// records {h_g^-2, m/h_g, m/h_g^3}.  It forms Newtonian pairs from them too, by u =
+// r/h_g, so the records must be finite, and u, which reaches 4 box half-widths hw
+// over h, must have a u^3.  Other groups (unsoftened ones, radii tiny against the
+// box or the mass M) take the form that has r and m themselves.
+__device__ __forceinline__ bool near_one_radius(float h, float hw, float M)
+{
+    const float hinv = __frcp_rn(h);   // infinite for h = 0
+    return h >= 1e-9f * hw && hinv * hinv < 1e37f && M * hinv * hinv * hinv < 1e37f;
 }
 
 __device__ __forceinline__ double warp_min_d(double v)
@@ -648,8 +658,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         const double hmaxd = (double)hmax, hmind = (double)hmin;
         const float hwf[3] = {__double2float_ru(hw[0]), __double2float_ru(hw[1]), __double2float_ru(hw[2])};
         const float aoldf = (float)aold_min, thetaf = (float)theta;
-        const bool homog = hmin == hmax;   // one kernel radius in the group (warp-uniform)
-        const float hwmax = fmaxf(hwf[0], fmaxf(hwf[1], hwf[2])), hzero = hwmax > 0.f ? 1e-6f * hwmax : 1.f;
+        const float hone = hmin == hmax && near_one_radius(hmax, fmaxf(hwf[0], fmaxf(hwf[1], hwf[2])),
+                                                           p.nodes[grp.root].mass) ? hmax : -1.f;   // warp-uniform
 
         // ---- traversal
         // Each round tests up to 32 NH nodes, NH per lane.  The next round's nodes
@@ -698,7 +708,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             const unsigned mu = __ballot_sync(FULL, use), mf = __ballot_sync(FULL, use && isfar), mn = mu & ~mf;
             if (use && isfar) list_put(far, nf + __popc(mf & lt_mask), e);
             if (mn) {   // warp-uniform
-                if (use && !isfar) near_put(near, nn + __popc(mn & lt_mask), e, near_soft(h, e.w, homog, hmax, hzero));
+                if (use && !isfar) near_put(near, nn + __popc(mn & lt_mask), e, near_soft(h, e.w, hone));
                 nn += __popc(mn);
                 list_near += __popc(mn);
             }
@@ -745,7 +755,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             if (nn >= nlimit) {
                 const int m = nn & ~(QUANTUM - 1);
                 __syncwarp();
-                if (homog) flush_near<TPL, SPLIT, POT>(near, m, part, T);
+                if (hone >= 0.f) flush_near<TPL, SPLIT, POT>(near, m, part, T);
                 else flush_near_mixed<TPL, SPLIT, POT>(near, m, part, T);
                 nn -= m;
                 list_shift<NEAR_ARRAYS, NEAR_CAP>(near, m, nn, lane);

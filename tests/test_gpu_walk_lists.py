@@ -48,6 +48,38 @@ def test_opening_every_node_is_the_direct_sum(n, group_size, flush, leaf_size, s
         assert np.linalg.norm(only - wpot) < 2e-6 * np.linalg.norm(wpot) + own
 
 
+# (box half-width, kernel radius, particle mass); a pair's force factor m/r^3 has to be an FP32 number
+@pytest.mark.parametrize("scale,h,m", [(1.0, 0.0, 1.0), (1e-8, 0.0, 1e-8), (1e8, 0.0, 1.0), (1.0, 1e-14, 1.0),
+                                       (1e8, 1e-6, 1.0), (1.0, 1e-25, 1e-6), (1e-8, 4e-9, 1.0), (1e8, 4e7, 1.0),
+                                       (1e13, 4e12, 1e30)])
+@pytest.mark.parametrize("group_size", [1, 32, 64])
+def test_close_pairs_at_any_scale(group_size, scale, h, m):
+    """One group's worth of particles in a box around the origin, two of them
+    1e-7 box widths apart at its centre (where the walk's FP32 offsets resolve
+    them), with and without softening, the kernel radius far below or near the
+    box."""
+    n = 32
+    rng = np.random.default_rng(11)
+    pos = rng.uniform(-0.9, 0.9, (n, 3))
+    pos[0], pos[1] = [-1.0, -1.0, -1.0], [1.0, 1.0, 1.0]       # the box, centred on the origin
+    pos[2], pos[3] = [5e-8, 2e-8, -3e-8], [-5e-8, -2e-8, 3e-8]
+    pos *= scale
+    mass, hh = np.full(n, m), np.full(n, h)
+    with ggb200.GravityTree(group_size=group_size) as t:
+        t.load(pos, mass, hh)
+        t.build()
+        acc, pot, nint, st = t.evaluate(old_acc=np.zeros(n), err_tol_force_acc=0.001, want_ninter=True)
+    assert st["error_word"] == 0 and np.all(nint == n - 1)
+    want, wpot = oracle.direct_sum(pos, mass.astype(np.float32), hh.astype(np.float32))
+    # each pair carries about ten roundings of 6e-8, relative to its own size; the
+    # Newtonian pair bounds the softened one
+    d = pos[None] - pos[:, None]
+    r = np.sqrt((d ** 2).sum(-1)) + np.where(np.eye(n) > 0, np.inf, 0.0)
+    r = np.maximum(r, 0.3 * h)
+    assert np.all(np.linalg.norm(acc - want, axis=1) < 2e-6 * (m / r ** 2).sum(1))
+    assert np.all(np.abs(pot - wpot) < 2e-6 * (m / r).sum(1))
+
+
 def test_cut_walks_give_the_same_bits_alone_and_in_a_batch():
     """A system in the range of sizes whose long walks are cut, opening every
     node: its sub-walks run as tasks when it is alone, and as each warp's own
