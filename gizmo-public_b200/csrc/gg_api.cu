@@ -715,11 +715,14 @@ extern "C" gg_status gg_get_domains(gg_ctx *c, gg_domain *out)
 }
 
 // ---------------------------------------------------------------- walk
-// whether long walks may be cut: some system has as many targets as that takes
-// (of a subset, the targets per system are known on the device only)
-static bool may_fork(const gg_ctx *c, bool subset)
+// whether long walks may be cut: some system has as many targets as that takes.
+// Of a subset of several systems only the total nt is known on the host, so a
+// system has up to the smaller of its particles and nt; of one system's, nt (an
+// index listed twice counts twice here).
+static bool may_fork(const gg_ctx *c, bool subset, long long nt)
 {
-    if (c->cfg.group_size <= 1) return false;
+    if (c->cfg.group_size <= 1 || nt < FORK_MIN_TARGETS) return false;
+    if (c->S == 1) return nt <= FORK_MAX_TARGETS;
     for (int s = 0; s < c->S; s++) {
         const long long n = c->h_poff[s + 1] - c->h_poff[s];
         if (n >= FORK_MIN_TARGETS && (subset || n <= FORK_MAX_TARGETS)) return true;
@@ -727,7 +730,7 @@ static bool may_fork(const gg_ctx *c, bool subset)
     return false;
 }
 
-static gg_status walk_setup(gg_ctx *c, bool subset)
+static gg_status walk_setup(gg_ctx *c, bool subset, long long nt)
 {
     gg_status st;
     if (!c->stack_cap) c->stack_cap = c->cfg.walk_stack_entries > 0 ? c->cfg.walk_stack_entries : GG_STACK_CAP;
@@ -745,10 +748,15 @@ static gg_status walk_setup(gg_ctx *c, bool subset)
         (st = c->stack.ensure((size_t)c->walk_blocks * gg_num_sms() * (gg_walk_threads() / 32) * c->stack_cap)) ||
         (st = c->scan_scratch.ensure(gg_scan_scratch_ints())))
         return st;
-    if (may_fork(c, subset) &&
-        ((st = c->forks.ensure(FORK_RECORDS)) ||
-         (st = c->own_forks.ensure((size_t)c->walk_blocks * gg_num_sms() * (gg_walk_threads() / 32) * FORK_OWN_BYTES))))
-        return st;
+    if (may_fork(c, subset, nt)) {
+        // a first allocation moves no buffer that a captured graph could hold
+        const bool first = !c->forks.p && !c->own_forks.p;
+        const long long gen = c->buf_gen;
+        if ((st = c->forks.ensure(FORK_RECORDS)) ||
+            (st = c->own_forks.ensure((size_t)c->walk_blocks * gg_num_sms() * (gg_walk_threads() / 32) * FORK_OWN_BYTES)))
+            return st;
+        if (first) c->buf_gen = gen;
+    }
     if (c->cfg.group_order &&
         ((st = c->tcost.ensure(c->N + 1)) || (st = c->gkey.ensure(maxg)) || (st = c->gorder.ensure(maxg)) ||
          (st = c->sort_scratch.ensure(gg_sort_scratch_bytes(maxg)))))
@@ -763,7 +771,8 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
 {
     gg_status st;
     cudaStream_t s = c->stream;
-    if ((st = walk_setup(c, d_active != nullptr))) return st;
+    const int ntargets = d_active ? n_active : (int)c->N;
+    if ((st = walk_setup(c, d_active != nullptr, ntargets))) return st;
     if ((st = resolve_h_mixed(c))) return st;
     const int S = c->S, N = (int)c->N;
     const int *tlist = nullptr, *tout = nullptr;
@@ -837,8 +846,8 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
     p.toff = toff;
     p.forks = c->forks.p;
     p.own_forks = c->own_forks.p;
-    p.fork_max = (d_active ? n_active : N) <= FORK_TASK_TARGETS ? FORK_RECORDS : 0;
-    p.may_fork = may_fork(c, d_active != nullptr);
+    p.fork_max = ntargets <= FORK_TASK_TARGETS ? FORK_RECORDS : 0;
+    p.may_fork = may_fork(c, d_active != nullptr, ntargets);
     p.task_walk = 0;
     p.stack = c->stack.p;
     p.stack_cap = c->stack_cap;
@@ -1112,7 +1121,7 @@ extern "C" gg_status gg_graph_capture_step(gg_ctx *c, double tol, double theta, 
     if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
     if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
     // grow every buffer the walk may need, and read the kernel-radius ranges, before capturing
-    if ((st = walk_setup(c, false))) return st;
+    if ((st = walk_setup(c, false, c->N))) return st;
     if ((st = resolve_h_mixed(c))) return st;
     const int timing = c->cfg.timing;
     c->cfg.timing = 0;
@@ -1152,7 +1161,7 @@ extern "C" gg_status gg_graph_capture_parts(gg_ctx *c, double tol, double theta,
     gg_status st;
     if ((st = set_device(c))) return st;
     drop_part_graphs(c);
-    if ((st = walk_setup(c, false))) return st;
+    if ((st = walk_setup(c, false, c->N))) return st;
     if ((st = resolve_h_mixed(c))) return st;
     const int timing = c->cfg.timing;
     c->cfg.timing = 0;

@@ -102,3 +102,42 @@ def test_cut_walks_give_the_same_bits_alone_and_in_a_batch():
     assert alone[2].mean() > 8192        # long enough to be cut
     for a, b in zip(alone[:3], batch[:3]):
         assert np.array_equal(a, b[:n])
+
+
+def test_small_subsets_of_a_large_system_are_not_prepared_for_cuts():
+    """A subset walk pays for cuts (records, two more launches) only with as many
+    targets as a cut takes; the records of a later, larger one do not make a
+    captured step stale."""
+    import torch
+    n, small = 350000, 98303
+    rng = np.random.default_rng(12)
+    rec = torch.from_numpy(ggb200.make_records(rng.normal(size=(n, 3)), np.ones(n), np.full(n, 1e-3)).view(np.uint8))
+    rec = rec.cuda()
+    stream = torch.cuda.Stream()
+    acc = torch.empty((n, 3), dtype=torch.float64, device="cuda")
+    acc2 = torch.empty_like(acc)
+    act = torch.arange(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    walks = dict(err_tol_theta=0.7)
+    with ggb200.GravityTree() as t:
+        t.set_stream(stream.cuda_stream)
+        t.load_device(rec, [n])
+        t.build()
+        t.evaluate_device(acc, **walks)
+        t.evaluate_device(acc2, d_active=act, n_active=1000, **walks)     # allocates what any subset takes
+        t.evaluate_device(acc2, d_active=act, n_active=small, **walks)
+        t.evaluate_device(acc2, d_active=act, n_active=n, **walks)
+        before, launches = t.device_bytes(), []
+        for k in (1000, small, n, n, small + 1):     # (the last is the first that may be cut)
+            l0 = ggb200.kernel_launches()
+            t.evaluate_device(acc2, d_active=act, n_active=k, **walks)
+            launches.append(ggb200.kernel_launches() - l0)
+            if k == n:
+                assert t.device_bytes() == before
+                t.capture_step(acc, **walks)
+        stream.synchronize()
+        assert t.device_bytes() > before + (30 << 20)
+        assert launches[1] == launches[2] == launches[3] == launches[4] - 2
+        t.launch_step()
+        stream.synchronize()
+        assert t.last_stats()["error_word"] == 0
