@@ -56,8 +56,28 @@ __device__ __forceinline__ GGDomainDev extent_domain(const unsigned long long *m
 // system s's complemented min x, y, z, max x, y, z, complemented min h and max h
 // (kernel radii are not negative: their bit patterns are ordered), all from
 // zero, so that one memset prepares every one.  The block that finishes last
-// (`done` counts them) forms the root cubes and the ranges of kernel radii: one
-// launch instead of three.
+// (`done` counts them) forms the root cubes and the ranges of kernel radii of up to
+// ROOTS_ONE_BLOCK systems: one launch instead of three.
+// With more systems one block is a serial tail, and a launch over the systems
+// forms them.  Keys stage, one block / launch, us: 1 system 17.7 / 20.9, 256 22.1 /
+// 23.8, 512 25.0 / 24.2, 4,096 60 / 34, 100,000 888 / 172, 1,000,000 8,557 / 1,287.
+#define ROOTS_ONE_BLOCK 256
+
+// root cube and range of kernel radii of system s from its extremes
+__device__ __forceinline__ void extent_root(int s, const unsigned long long *mm, unsigned *hmm, GGDomainDev *dom)
+{
+    dom[s] = extent_domain(mm + 8 * (size_t)s);
+    const unsigned long long lo = ~__ldcg(mm + 8 * (size_t)s + 6);
+    hmm[2 * s] = lo >> 32 ? 0x7f800000u : (unsigned)lo;   // infinite for an empty system
+    hmm[2 * s + 1] = (unsigned)__ldcg(mm + 8 * (size_t)s + 7);
+}
+
+__global__ void k_extent_roots(int S, const unsigned long long *mm, unsigned *hmm, GGDomainDev *dom)
+{
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < S) extent_root(s, mm, hmm, dom);
+}
+
 __global__ void k_extent(const GGPart *__restrict__ rec, int n, const int *__restrict__ poff, int S, int chunk,
                          unsigned long long *mm, unsigned *done, unsigned *hmm, GGDomainDev *dom, int *err)
 {
@@ -106,6 +126,7 @@ __global__ void k_extent(const GGPart *__restrict__ rec, int n, const int *__res
         }
     }
     if (bad) atomicOr(err, GG_EBIT_BAD_INPUT);
+    if (S > ROOTS_ONE_BLOCK) return;
     __shared__ bool s_last;
     __threadfence();
     __syncthreads();
@@ -113,12 +134,7 @@ __global__ void k_extent(const GGPart *__restrict__ rec, int n, const int *__res
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    for (int s = threadIdx.x; s < S; s += blockDim.x) {
-        dom[s] = extent_domain(mm + 8 * (size_t)s);
-        const unsigned long long lo = ~__ldcg(mm + 8 * (size_t)s + 6);
-        hmm[2 * s] = lo >> 32 ? 0x7f800000u : (unsigned)lo;   // infinite for an empty system
-        hmm[2 * s + 1] = (unsigned)__ldcg(mm + 8 * (size_t)s + 7);
-    }
+    for (int s = threadIdx.x; s < S; s += blockDim.x) extent_root(s, mm, hmm, dom);
 }
 
 // 21 levels: the top one from the one-level table, then ten steps of two
@@ -209,6 +225,10 @@ void gg_launch_extent(const GGPart *rec, int n, const int *poff, int S, unsigned
     k_extent<<<std::max(blocks, 1), threads, 0, st>>>(rec, n, poff, S, chunk, mm, (unsigned *)(mm + 8 * (size_t)S), hmm, dom,
                                                       err);
     gg_note_launches(1);
+    if (S > ROOTS_ONE_BLOCK) {
+        k_extent_roots<<<(S + 127) / 128, 128, 0, st>>>(S, mm, hmm, dom);
+        gg_note_launches(1);
+    }
 }
 
 void gg_launch_keys(const GGPart *rec, int n, const int *poff, int S, const GGDomainDev *dom,

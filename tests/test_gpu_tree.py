@@ -123,3 +123,51 @@ def test_a_build_does_not_wait_for_other_kernels_to_end():
         torch.cuda.synchronize()
         assert t.last_stats()["error_word"] == 0
     assert torch.equal(acc, want)
+
+
+@pytest.mark.parametrize("S", [1, 255, 256, 257, 5000])
+def test_root_cubes_of_many_systems(S):
+    """Up to 256 systems' root cubes are formed by the extent kernel's last block,
+    more by a launch of their own: the FP64 expressions of the extent, to the bit,
+    empty systems and single particles included."""
+    rng = np.random.default_rng(S)
+    sizes = rng.integers(0, 9, S)
+    sizes[-1] = 3
+    n = int(sizes.sum())
+    pos = rng.normal(size=(n, 3)) * 10.0 ** rng.integers(-3, 4, (n, 1))
+    with ggb200.GravityTree() as t:
+        t.load(pos, np.ones(n), np.full(n, 1e-3), counts=sizes.tolist())
+        t.build()
+        got = t.domains()
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    for s in range(S):
+        p = pos[off[s]:off[s + 1]]
+        mn, mx = (p.min(0), p.max(0)) if len(p) else (np.zeros(3), np.zeros(3))
+        length = 1.001 * (mx - mn).max()
+        if length <= 0:
+            length = 1.0
+        mid = 0.5 * (mn + mx)
+        assert got[s]["len"] == length
+        assert np.array_equal(got[s]["center"], mid) and np.array_equal(got[s]["corner"], mid - 0.5 * length)
+
+
+def test_root_cubes_of_many_systems_are_no_serial_tail():
+    """2,097,152 particles as 262,144 systems of 8: the keys stage takes the time of
+    many blocks, not of one that forms every root cube (which took 30 times the
+    stage of 256 systems)."""
+    import torch
+    n = 1 << 21
+    rng = np.random.default_rng(61)
+    rec = torch.from_numpy(ggb200.make_records(rng.normal(size=(n, 3)), np.ones(n), np.full(n, 1e-3)).view(np.uint8))
+    rec = rec.cuda()
+    ms = {}
+    for S in (256, 262144):
+        with ggb200.GravityTree(timing=True) as t:
+            t.load_device(rec, [n // S] * S)
+            times = []
+            for _ in range(6):
+                t.build()
+                times.append(t.last_stats()["ms_keys"])
+        ms[S] = min(times)
+    print(ms)
+    assert ms[262144] < 12 * ms[256], ms
