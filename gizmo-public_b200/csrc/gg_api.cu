@@ -730,16 +730,14 @@ static bool may_fork(const gg_ctx *c, bool subset, long long nt)
     return false;
 }
 
+// blocks of the persistent walk per SM: two are resident (registers, shared memory), a third would find no work left
+static int walk_blocks_per_sm(int wanted) { return wanted == 1 ? 1 : 2; }
+
 static gg_status walk_setup(gg_ctx *c, bool subset, long long nt)
 {
     gg_status st;
     if (!c->stack_cap) c->stack_cap = c->cfg.walk_stack_entries > 0 ? c->cfg.walk_stack_entries : GG_STACK_CAP;
-    if (!c->walk_blocks) {
-        int per_sm = c->cfg.walk_blocks_per_sm;
-        if (per_sm <= 0) per_sm = 2;   // measured best or tied on the galaxy, clustered and Plummer workloads
-        if (per_sm > 3) per_sm = 3;
-        c->walk_blocks = per_sm;   // blocks per SM; the grid is that many per SM
-    }
+    if (!c->walk_blocks) c->walk_blocks = walk_blocks_per_sm(c->cfg.walk_blocks_per_sm);
     const long long maxg = gg_max_groups(c->N, c->S, c->cfg.group_size);
     if ((st = c->groups.ensure(maxg)) || (st = c->ngroups.ensure(2)) || (st = c->gscan.ensure(c->S + 1)) ||
         (st = c->toff.ensure(c->S + 1)) ||
@@ -1216,10 +1214,9 @@ extern "C" gg_status gg_graph_launch(gg_ctx *c)
 }
 
 // Timed search over the walk's tunables on the resident systems: leaf size
-// (rebuilds the tree), group size (targets per warp), blocks per SM (stack
-// depth per warp follows from it) and the list-flush threshold; then the
-// other node staging on the winner.  Every trial
-// walks from the same OldAcc, so trials see the same opening decisions for a
+// (rebuilds the tree), group size (targets per warp) and the list-flush
+// threshold, with two blocks per SM; then the other node staging on the winner.
+// Every trial walks from the same OldAcc, so trials see the same opening decisions for a
 // given tree; the fastest configuration is kept and the tree rebuilt with it.
 // ---------------------------------------------------------------- autotuner accuracy gate
 // A faster configuration is only taken if it is no less accurate than the
@@ -1394,7 +1391,7 @@ extern "C" gg_status gg_autotune_active(gg_ctx *c, const int32_t *d_active, int6
     GG_CUDA_TRY(cudaEventCreate(&e1));
     const gg_config base = c->cfg;
     const int base_blocks = c->walk_blocks;
-    static const int leafs[] = {8, 16}, groups[] = {32, 64}, bpss[] = {2, 3}, flushes[] = {64, 128};
+    static const int leafs[] = {8, 16}, groups[] = {32, 64}, flushes[] = {64, 128};
     float best = 1e30f;
     gg_config best_cfg = base;
     int best_blocks = base_blocks;
@@ -1443,20 +1440,19 @@ extern "C" gg_status gg_autotune_active(gg_ctx *c, const int32_t *d_active, int6
         c->cfg.leaf_size = leafs[li];
         if ((st = gg_build(c, nullptr))) break;
         for (int gi = 0; gi < 2 && !st; gi++)
-            for (int bi = 0; bi < 2 && !st; bi++)
-                for (int fi = 0; fi < 2 && !st; fi++) {
-                    c->cfg.group_size = groups[gi];
-                    c->cfg.flush_threshold = flushes[fi];
-                    c->walk_blocks = bpss[bi];
-                    float ms = 0;
-                    bool ok = false;
-                    if ((st = trial(&ms, &ok))) break;
-                    if (ok && ms < best) {
-                        best = ms;
-                        best_cfg = c->cfg;
-                        best_blocks = c->walk_blocks;
-                    }
+            for (int fi = 0; fi < 2 && !st; fi++) {
+                c->cfg.group_size = groups[gi];
+                c->cfg.flush_threshold = flushes[fi];
+                c->walk_blocks = walk_blocks_per_sm(0);
+                float ms = 0;
+                bool ok = false;
+                if ((st = trial(&ms, &ok))) break;
+                if (ok && ms < best) {
+                    best = ms;
+                    best_cfg = c->cfg;
+                    best_blocks = c->walk_blocks;
                 }
+            }
     }
     // the other node staging, on the winner
     if (!st) {
@@ -1529,7 +1525,7 @@ extern "C" gg_status gg_tune_accuracy(gg_ctx *c, double tol, double theta, const
     c->cfg.node_staging = cand->node_staging;
     c->cfg.target_order = cand->target_order;
     c->cfg.group_order = cand->group_order;
-    if (cand->walk_blocks_per_sm > 0) c->walk_blocks = cand->walk_blocks_per_sm;
+    if (cand->walk_blocks_per_sm > 0) c->walk_blocks = walk_blocks_per_sm(cand->walk_blocks_per_sm);
     const bool rebuild = cand->leaf_size != keep.leaf_size;
     if (rebuild) st = gg_build(c, nullptr);
     if (!st) st = walk_errors(cerr);

@@ -1144,8 +1144,7 @@ static void launch_walk_t(const WalkParams &p, int blocks, cudaStream_t st)
     else launch_walk_c<TPL, SPLIT, F64T, POT, TMA, false>(p, blocks, st);
 }
 
-// The persistent grid is blocks_per_sm (1..3) blocks per SM, of which two are
-// resident at a time (registers and shared memory).
+// The persistent grid is blocks_per_sm (1 or 2) blocks per SM.
 void gg_launch_walk(const WalkParams &p, int blocks_per_sm, cudaStream_t st)
 {
     const int blocks = gg_num_sms() * blocks_per_sm;

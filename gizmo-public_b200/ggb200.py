@@ -447,11 +447,10 @@ class GravityTree:
         _check(self._lib.gg_graph_launch_part(self._h, part), "gg_graph_launch_part")
 
     def autotune(self, err_tol_force_acc=0.0025, err_tol_theta=0.0, d_active=None, n_active=0):
-        """Pick leaf size, group size, blocks per SM, flush threshold and node
-        staging by timing the walk of the resident systems (of the active
-        targets d_active, a device int32 tensor, when given), refusing any
-        candidate less accurate than the context's configuration; returns
-        (config dict, ms)."""
+        """Pick leaf size, group size, flush threshold and node staging by
+        timing the walk of the resident systems (of the active targets d_active,
+        a device int32 tensor, when given), refusing any candidate less accurate
+        than the context's configuration; returns (config dict, ms)."""
         cfg = Config()
         ms = ctypes.c_double()
         if d_active is None:

@@ -53,8 +53,12 @@ typedef struct gg_config {
     int32_t device;           /* CUDA device ordinal */
     int32_t leaf_size;        /* max particles per leaf bucket, 1..32 (default 8) */
     int32_t group_size;       /* targets per walk group, 1..64 (default 32) */
-    int32_t flush_threshold;  /* interaction-list entries per flush, 32..128 (default 128) */
-    int32_t walk_blocks_per_sm; /* persistent walk blocks per SM, 0 = default */
+    int32_t flush_threshold;  /* interaction-list entries per flush, 32..128 (default 128); the
+                                 lists hold 96 entries without softening and 64 with, and
+                                 larger values are taken as those */
+    int32_t walk_blocks_per_sm; /* persistent walk blocks per SM, 0 = default (2); 1 leaves half
+                                 of each SM to other kernels, 3 is taken as 2, the number that
+                                 is resident */
     int32_t timing;           /* 1: record per-stage device times into gg_stats */
     int32_t target_order;     /* 1 (default): when a system holds several kernel radii, walk
                                  targets are ordered by Peano-Hilbert cell at the softening
@@ -290,8 +294,8 @@ gg_status gg_graph_capture_parts(gg_ctx *ctx, double err_tol_force_acc, double e
                                  double *d_pot_out);
 gg_status gg_graph_launch_part(gg_ctx *ctx, int32_t part);
 /* Times the walk of the resident systems with the context's configuration
- * and over leaf size {8,16}, group size {32,64}, blocks per SM {2,3} and flush
- * threshold {64,128}, then the other node staging on the winner, each trial
+ * and over leaf size {8,16}, group size {32,64} and flush threshold {64,128}
+ * with two blocks per SM, then the other node staging on the winner, each trial
  * from the same OldAcc, and keeps the fastest configuration that passes the
  * accuracy gate (rebuilding the tree with its leaf size); returns it in
  * *chosen and its walk time in *best_ms (nullable).  The gate: on a fixed

@@ -116,6 +116,36 @@ def test_autotune_keeps_the_force_error_and_returns_a_valid_config():
         t.close()
 
 
+def test_blocks_that_are_not_resident_are_neither_run_nor_tried():
+    """Two walk blocks are resident per SM.  A third is accepted and changes
+    nothing, the stack memory included, and the tuner does not time it: each of its
+    trials (the base, 2 leaf sizes x 2 group sizes x 2 flush thresholds, the other
+    staging; two walks each) differs from the others."""
+    import torch
+    ic = _ensemble(S=4, nmax=3000, seed=12)
+    stream = torch.cuda.Stream()
+    out = []
+    with torch.cuda.stream(stream):
+        for blocks in (0, 2, 3):
+            t, _, acc, pot = _setup(torch, ic, stream, blocks_per_sm=blocks)
+            stream.synchronize()
+            out.append((t.device_bytes(), acc.cpu().numpy()))
+            if blocks == 0:
+                l0 = ggb200.kernel_launches()
+                t.build()
+                l1 = ggb200.kernel_launches()
+                t.evaluate_device(acc, pot, err_tol_force_acc=0.001)
+                l2 = ggb200.kernel_launches()
+                cfg, _ = t.autotune(err_tol_force_acc=0.001)
+                # four builds (two leaf sizes, the staging trial, the winner), and per trial two kernels of the gate
+                most = 4 * (l1 - l0) + 20 * (l2 - l1) + 2 * 10 + 1
+                assert ggb200.kernel_launches() - l2 <= most
+                assert cfg["blocks_per_sm"] == 2
+            t.close()
+    assert out[0][0] == out[1][0] == out[2][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][1], out[2][1])
+
+
 def test_tuner_gate_refuses_a_less_accurate_configuration():
     """Leaf buckets of 16 on the reference's clustered golden put the potential
     energy further from the direct sum than the reference tree does (and than
