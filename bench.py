@@ -16,8 +16,8 @@ than L2 (no flush needed).
 Under torchrun each rank evaluates its own independent system (weak scaling,
 no collective on the data path; the process group only carries the barrier
 and the max-over-ranks timing).  --impl reference times the reference
-algorithm on the host cores (compiled GIZMO objects when present, else the C
-restatement) on a bounded sample of the same workload.
+algorithm on the host cores (compiled GIZMO) on a bounded sample of the same
+workload; without the compiled reference it says so and prints no rate.
 """
 import argparse
 import json
@@ -117,50 +117,6 @@ class ClockSampler:
 
 
 # ---------------------------------------------------------------- CPU baselines
-def cpu_reference_rate(ic, seconds=15.0, seed=1, tol=0.0025, active_n=None):
-    """Time the reference algorithm on the host cores on a bounded sample.
-
-    Cost model of one step: tree build (serial in the reference) plus the walk
-    of every particle; the walk is timed on a seeded random sample of targets
-    and scaled to N.  Uses the compiled reference when present, else the C
-    restatement in oracle/."""
-    sys.path.insert(0, os.path.join(ROOT, "oracle"))
-    import oracle
-    try:
-        import ref_runner
-        if ref_runner.available():
-            return ref_runner.rate(ic, seconds=seconds, seed=seed, tol=tol, active_n=active_n)
-    except ImportError:
-        pass
-    n = ic["pos"].shape[0]
-    cores = os.cpu_count() or 1
-    old = np.linalg.norm(ic.get("acc_hint", np.zeros((n, 3))), axis=1) if "acc_hint" in ic else None
-    if old is None:
-        # OldAcc from a cheap BH pass over a small sample is not enough for all particles;
-        # use |a| of the GPU pass when the caller supplied it, else the BH pass itself
-        old = np.full(n, 0.0)
-    rng = np.random.default_rng(seed)
-    t0 = time.perf_counter()
-    oracle.tree_gravity(ic["pos"], ic["mass"], ic["h"], old, tol, 0.0, targets=np.zeros(0, np.int32),
-                        nthreads=cores)
-    t_build = time.perf_counter() - t0
-    ns = 256
-    while True:
-        tg = np.sort(rng.choice(n, ns, replace=False)).astype(np.int32)
-        t0 = time.perf_counter()
-        oracle.tree_gravity(ic["pos"], ic["mass"], ic["h"], old, tol, 0.0, targets=tg, nthreads=cores)
-        t = time.perf_counter() - t0 - t_build
-        if t > 0.25 * seconds or ns >= n:
-            break
-        ns = min(n, int(ns * max(2.0, 0.3 * seconds / max(t, 1e-3))))
-    per = max(t, 1e-9) / ns
-    step = t_build + per * n
-    return {"value": n / step, "unit": "particles/s", "cores": cores, "kind": "port",
-            "sample": "C restatement (oracle/gg_oracle.c, FP64, OpenMP): full tree build + relative walk of %d "
-                      "seeded random targets of %d, walk time scaled to all targets" % (ns, n),
-            "t_build_s": t_build, "t_walk_per_particle_us": per * 1e6}
-
-
 REF_BLOCKS, REF_BLOCK_LEN = 64, 1024   # PH-contiguous sample of the reference timing: 64 runs of 1,024 targets
 REF_FULL_MAX = 262144                   # systems up to this size are walked whole by the reference
 
@@ -184,13 +140,12 @@ def cpu_reference(ic, ref_tg, args, n_eval):
     (random), with their walk time; (2) its timing on a Peano-Hilbert
     contiguous sample, the order GIZMO's own walk takes.  Each run times one
     rebuild (domain_Decomposition + tree build) and one walk of its sample on
-    the resident tree.  Returns (cpu_baseline, reference results on ref_tg);
-    the C restatement stands in, without forces, where the compiled reference
-    cannot run."""
+    the resident tree.  Returns (cpu_baseline, reference results on ref_tg),
+    both None where the compiled reference cannot run."""
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import ref_runner
     if not ref_runner.available():
-        return cpu_reference_rate(ic, seconds=args.cpu_seconds, tol=args.tol, active_n=n_eval), None
+        return None, None
     n = ic["pos"].shape[0]
     r_rand, i_rand = ref_runner.steps_rate(ic, steps=1, warmup=0, sample=ref_tg, tol=args.tol, active_n=n_eval,
                                            sample_kind="%d seeded random targets" % ref_tg.size)
@@ -250,36 +205,32 @@ def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return 0
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import ref_runner
+    if not ref_runner.available():
+        print(json.dumps({"impl": "reference", "unavailable": "compiled reference (oracle/_ref) not built"}))
+        return 0
     if args.workload in ("ensemble", "serve"):
         return run_reference_arm_systems(args)
     name, gen = WORKLOADS[args.workload]
     ic = gen(SEEDS[args.workload])
     n = ic["pos"].shape[0]
-    sys.path.insert(0, os.path.join(ROOT, "oracle"))
-    import ref_runner
     active_n = int(round(args.active_frac * n)) if args.active_frac < 1.0 else None
-    if not ref_runner.available():
-        vals = [cpu_reference_rate(ic, seconds=args.ref_seconds, seed=1000 + i, tol=args.tol)
-                for i in range(args.warmup + args.steps)][args.warmup:]
-        v = float(np.mean([x["value"] for x in vals]))
-        info = vals[-1]
-        step_ms, extra = 1e3 * n / v, {}
-    else:
-        smp, kind = reference_sample(ic)
-        whole = smp.size == n and active_n is None
-        rates, info = ref_runner.steps_rate(ic, steps=args.steps, warmup=args.warmup, sample=smp, tol=args.tol,
-                                            active_n=active_n, rebuild_steps="all" if whole else 1, sample_kind=kind)
-        v = float(np.mean(rates))
-        step_ms = 1e3 * float(np.mean(info["step_s"]))
-        extra = {"timed_step": "whole step (domain + build + walk of every particle)" if whole else
-                 "walk of the sample on the resident tree (the rebuild is timed once and enters the model)",
-                 "model": "n / (t_domain + t_build + t_walk_fixed + t_walk_per_particle x n)",
-                 "t_domain_s": info["t_domain_s"], "t_build_s": info["t_build_s"],
-                 "t_walk_fixed_s": info["t_walk_fixed_s"], "t_empty_walk_s": info["t_empty_walk_s"],
-                 "t_walk_per_particle_us": info["t_walk_per_particle_us"],
-                 "model_ms_per_full_step": 1e3 * n / v if active_n is None else 1e3 * active_n / v}
-        if args.calibrate:
-            extra["calibration"] = reference_calibration(ic, args, active_n, v, kind)
+    smp, kind = reference_sample(ic)
+    whole = smp.size == n and active_n is None
+    rates, info = ref_runner.steps_rate(ic, steps=args.steps, warmup=args.warmup, sample=smp, tol=args.tol,
+                                        active_n=active_n, rebuild_steps="all" if whole else 1, sample_kind=kind)
+    v = float(np.mean(rates))
+    step_ms = 1e3 * float(np.mean(info["step_s"]))
+    extra = {"timed_step": "whole step (domain + build + walk of every particle)" if whole else
+             "walk of the sample on the resident tree (the rebuild is timed once and enters the model)",
+             "model": "n / (t_domain + t_build + t_walk_fixed + t_walk_per_particle x n)",
+             "t_domain_s": info["t_domain_s"], "t_build_s": info["t_build_s"],
+             "t_walk_fixed_s": info["t_walk_fixed_s"], "t_empty_walk_s": info["t_empty_walk_s"],
+             "t_walk_per_particle_us": info["t_walk_per_particle_us"],
+             "model_ms_per_full_step": 1e3 * n / v if active_n is None else 1e3 * active_n / v}
+    if args.calibrate:
+        extra["calibration"] = reference_calibration(ic, args, active_n, v, kind)
     out = {"metric": METRIC, "value": v, "unit": "particles/s", "n_gpus": args.gpus, "steps": args.steps,
            "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True, "scaling": "weak",
            "vs_baseline": None, "dtype": "f64", "data": "synthetic",
@@ -1167,6 +1118,7 @@ def main():
     # at 0.001 the galaxy's p99 is 1.77e-3 but the clustered system's 2.0e-3
     ap.add_argument("--tol", type=float, default=None)
     ap.add_argument("--err-targets", type=int, default=65536)
+    # accepted and unused: the reference's samples have fixed sizes
     ap.add_argument("--ref-seconds", type=float, default=8.0)
     ap.add_argument("--ref-sample", type=int, default=16384)
     ap.add_argument("--cpu-seconds", type=float, default=15.0)
