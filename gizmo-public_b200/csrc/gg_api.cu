@@ -940,6 +940,16 @@ extern "C" gg_status gg_last_stats(gg_ctx *c, gg_stats *out)
     return collect_stats(c, out);
 }
 
+extern "C" gg_status gg_last_cuts(gg_ctx *c, int64_t *cuts)
+{
+    if (!c || !cuts) return GG_ERR_INVALID;
+    int n = 0;
+    GG_CUDA_TRY(cudaMemcpyAsync(&n, c->counters.p + WALK_FORK_COUNTER, sizeof n, cudaMemcpyDeviceToHost, c->stream));
+    GG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    *cuts = n;
+    return GG_OK;
+}
+
 extern "C" gg_status gg_evaluate_device(gg_ctx *c, const int32_t *d_active, int64_t n_active, const double *d_old_acc,
                                         double tol, double theta, double *d_acc, double *d_pot, int32_t *d_nint)
 {

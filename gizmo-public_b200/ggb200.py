@@ -110,6 +110,7 @@ def load_library():
             "gg_evaluate": (i32, [P, P, i64, P, dbl, dbl, P, P, P, ctypes.POINTER(Stats)]),
             "gg_evaluate_device": (i32, [P, P, i64, P, dbl, dbl, P, P, P]),
             "gg_last_stats": (i32, [P, ctypes.POINTER(Stats)]),
+            "gg_last_cuts": (i32, [P, ctypes.POINTER(i64)]),
             "gg_peano_hilbert_keys": (i32, [i64, P, ctypes.POINTER(Domain), P, P]),
             "gg_radix_sort_pairs": (i32, [i64, P, P, i32, P]),
             "gg_direct_sum_fp64": (i32, [i64, P, P, P, i64, P, P, P, P]),
@@ -293,6 +294,12 @@ class GravityTree:
         st = Stats()
         _check(self._lib.gg_last_stats(self._h, ctypes.byref(st)), "gg_last_stats")
         return st.as_dict()
+
+    def last_cuts(self):
+        """Walks of the last evaluation that were cut into sub-walks (see gg_last_cuts)."""
+        n = ctypes.c_int64()
+        _check(self._lib.gg_last_cuts(self._h, ctypes.byref(n)), "gg_last_cuts")
+        return n.value
 
     def load_velocities(self, vel):
         """Per-particle velocities (N,3) in load order: host array or device tensor."""

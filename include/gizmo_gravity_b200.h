@@ -169,6 +169,9 @@ gg_status gg_evaluate_device(gg_ctx *ctx, const int32_t *d_active, int64_t n_act
                              double *d_pot_out, int32_t *d_ninter_out);
 /* interaction count and error word of the last evaluation (synchronises) */
 gg_status gg_last_stats(gg_ctx *ctx, gg_stats *stats);
+/* how many walks of the last evaluation were cut into sub-walks, long ones of
+ * middle-sized systems (synchronises) */
+gg_status gg_last_cuts(gg_ctx *ctx, int64_t *cuts);
 
 /* device memory the context holds now (all its buffers), for callers that
  * admit work against a memory budget; no counterpart in the reference */

@@ -171,3 +171,48 @@ def test_root_cubes_of_many_systems_are_no_serial_tail():
         ms[S] = min(times)
     print(ms)
     assert ms[262144] < 12 * ms[256], ms
+
+
+def test_contexts_on_several_streams_build_beside_a_walk():
+    """Four contexts on four streams rebuild and walk while a fifth one's walks
+    keep the GPU busy: each gets the bits it gets alone."""
+    import torch
+    sizes = [1000, 40000, 150000, 700000]
+    busy_n = 300000
+
+    def records(n, seed):
+        rng = np.random.default_rng(seed)
+        r = ggb200.make_records(rng.normal(size=(n, 3)), np.ones(n), np.full(n, 1e-2))
+        return torch.from_numpy(r.view(np.uint8)).cuda()
+
+    trees, accs, recs, want = [], [], [], []
+    for i, n in enumerate(sizes + [busy_n]):
+        t = ggb200.GravityTree()
+        s = torch.cuda.Stream()
+        t.set_stream(s.cuda_stream)
+        recs.append(records(n, 80 + i))
+        accs.append(torch.empty((n, 3), dtype=torch.float64, device="cuda"))
+        torch.cuda.synchronize()
+        t.load_device(recs[-1], [n])
+        t.build()
+        t.evaluate_device(accs[-1], err_tol_theta=0.7)
+        t.synchronize()
+        want.append(accs[-1].clone())
+        trees.append(t)
+    torch.cuda.synchronize()
+    for _ in range(10):
+        trees[-1].evaluate_device(accs[-1], err_tol_theta=0.3)
+        for t, r, a, n in zip(trees[:-1], recs, accs, sizes):
+            a.zero_()
+        torch.cuda.current_stream().synchronize()
+        for t, r, a, n in zip(trees[:-1], recs, accs, sizes):
+            t.load_device(r, [n])
+            t.build()
+            t.evaluate_device(a, err_tol_theta=0.7)
+        for t, a, w in zip(trees[:-1], accs, want):
+            t.synchronize()
+            assert t.last_stats()["error_word"] == 0
+            assert torch.equal(a, w)
+    torch.cuda.synchronize()
+    for t in trees:
+        t.close()

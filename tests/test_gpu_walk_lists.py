@@ -94,14 +94,74 @@ def test_cut_walks_give_the_same_bits_alone_and_in_a_batch():
         t.load(pos, mass, h)
         t.build()
         alone = t.evaluate(want_ninter=True, **theta)
+        cuts = [t.last_cuts()]
         t.load(np.concatenate([pos, more]), np.concatenate([mass, mm]), np.concatenate([h, np.full(big, h[0])]),
                counts=[n, big])
         t.build()
         batch = t.evaluate(want_ninter=True, **theta)
+        cuts.append(t.last_cuts())
+    assert cuts == [cuts[0], cuts[0]] and cuts[0] > 0
     assert alone[3]["error_word"] == 0 and batch[3]["error_word"] == 0
     assert alone[2].mean() > 8192        # long enough to be cut
     for a, b in zip(alone[:3], batch[:3]):
         assert np.array_equal(a, b[:n])
+
+
+# one system as tasks (98,304 and 131,072 + 1 targets: both work limits) and, past the
+# records of tasks or beside a second system, each warp its own sub-walks
+@pytest.mark.parametrize("n,other", [(98304, 0), (131073, 0), (98304, 302000)])
+@pytest.mark.parametrize("group_size,staging", [(32, 0), (32, 1), (64, 0), (64, 1)])
+def test_cut_walks_that_open_every_node_are_the_direct_sum(n, other, group_size, staging):
+    pos, mass, h = _system(n, "one", 8)
+    if other:
+        rng = np.random.default_rng(9)
+        pos = np.concatenate([pos, rng.normal(size=(other, 3))])
+        mass, h = np.concatenate([mass, np.ones(other)]), np.full(n + other, h[0])
+    counts = [n, other] if other else [n]
+    old = np.zeros(n + other)
+    old[n:] = 1e30                     # the other system's nodes are used whole
+    with ggb200.GravityTree(group_size=group_size, node_staging=staging) as t:
+        t.load(pos, mass, h, counts=counts)
+        t.build()
+        acc, pot, nint, st = t.evaluate(old_acc=old, err_tol_force_acc=0.001, want_ninter=True)
+        # every group meets n - 1 particles, far beyond the work of a cut
+        assert t.last_cuts() > 0.5 * (n // group_size)
+        only, _ = t.evaluate_potential(old_acc=old, err_tol_force_acc=0.001)
+        assert t.last_cuts() > 0.5 * (n // group_size)
+    assert st["error_word"] == 0
+    assert np.all(nint[:n] == n - 1)
+    tg = np.arange(0, n, 401).astype(np.int32)
+    want, wpot = oracle.direct_sum(pos[:n], mass[:n], h[:n], targets=tg)
+    # as above: about ten roundings of 6e-8 per pair
+    assert np.linalg.norm(acc[tg] - want) < 3e-6 * np.linalg.norm(want)
+    assert np.linalg.norm(pot[tg] - wpot) < 2e-6 * np.linalg.norm(wpot)
+    own = 4 * 6e-8 * np.linalg.norm(2.8 * mass[tg] / h[tg])
+    assert np.linalg.norm(only[tg] - wpot) < 2e-6 * np.linalg.norm(wpot) + own
+
+
+@pytest.mark.parametrize("group_size", [32, 64])
+def test_cut_walks_of_a_subset_and_after_a_stack_overflow(group_size):
+    """An active subset inside the window, in an order of its own, and the same
+    with a node stack that overflows before and after cuts: the walk runs again
+    with a larger one and gives the same bits."""
+    n = 200000
+    pos, mass, h = _system(n, "two", 10)
+    act = np.random.default_rng(11).permutation(n)[:99000].astype(np.int32)
+    out = []
+    for entries in (0, 64):
+        with ggb200.GravityTree(group_size=group_size, walk_stack_entries=entries) as t:
+            t.load(pos, mass, h)
+            t.build()
+            out.append(t.evaluate(active=act, old_acc=np.zeros(n), err_tol_force_acc=0.001, want_ninter=True))
+            assert t.last_cuts() > 0
+    assert out[0][3]["error_word"] == 0 and out[1][3]["error_word"] == 0
+    for a, b in zip(out[0][:3], out[1][:3]):
+        assert np.array_equal(a, b)
+    assert np.all(out[0][2] == n - 1)
+    few = np.arange(0, act.size, 997)
+    want, wpot = oracle.direct_sum(pos, mass, h, targets=act[few])
+    assert np.linalg.norm(out[0][0][few] - want) < 3e-6 * np.linalg.norm(want)
+    assert np.linalg.norm(out[0][1][few] - wpot) < 2e-6 * np.linalg.norm(wpot)
 
 
 def test_small_subsets_of_a_large_system_are_not_prepared_for_cuts():

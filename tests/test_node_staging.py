@@ -48,9 +48,10 @@ def _walks(ic, staging, active=None, group_size=32):
     return out, st
 
 
-@pytest.mark.parametrize("case", ["galaxy", "ensemble", "subset", "exact"])
+@pytest.mark.parametrize("case", ["galaxy", "galaxy wide", "ensemble", "ensemble wide", "subset", "subset wide", "exact"])
 def test_bulk_copy_staging_equals_per_lane_staging(case):
-    active, gs = None, 32
+    active, gs = None, 64 if case.endswith("wide") else 32     # (wide: two node slots and two targets per lane)
+    case = case.split()[0]
     if case == "galaxy":
         ic = ics.galaxy(50000, 20000, seed=91)
         ic["counts"] = [ic["pos"].shape[0]]
