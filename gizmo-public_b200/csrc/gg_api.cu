@@ -430,6 +430,7 @@ extern "C" gg_status gg_create(const gg_config *cfg, gg_ctx **out)
         return st;
     }
     cudaMemset(ctx->err.p, 0, 8 * sizeof(int));
+    cudaMemset(ctx->counters.p, 0, 8 * sizeof(int));
     *out = ctx;
     return GG_OK;
 }
@@ -733,6 +734,21 @@ static bool may_fork(const gg_ctx *c, bool subset, long long nt)
 // blocks of the persistent walk per SM: two are resident (registers, shared memory), a third would find no work left
 static int walk_blocks_per_sm(int wanted) { return wanted == 1 ? 1 : 2; }
 
+// Work after which a walk is cut: FORK_WORK for the relative criterion at GIZMO's
+// tolerance and for the Barnes-Hut pass, and growing as fast as a mean group's work
+// does for stricter ones.  That measured (groups of 32, 262,144 particles; galaxy,
+// Plummer, clustered) 5,000, 3,600, 3,400 at tolerance 0.0025, 6,300, 5,300, 4,800 at
+// 0.001, 13,700, 15,000, 11,400 at 1e-4 and 35,200, 43,400, 27,100 at 1e-5; 3,800,
+// 2,900, 2,000 at opening angle 0.7 and 23,900, 18,100, 8,900 at 0.3.  Walk
+// ms uncut / cut after 16,384 / by this rule: galaxy at 0.0025 2.05 / 1.33 / 1.33,
+// at 1e-5 4.62 / 8.11 / 4.77; Plummer at 1e-5 6.20 / 11.04 / 6.32 (when nearly every
+// walk is cut, the few records are taken at random and the rest is a second round).
+static int fork_work(double tol, double theta)
+{
+    const double f = theta > 0 ? pow(0.7 / theta, 2.2) : tol > 0 ? pow(0.0025 / tol, 0.45) : 1e9;
+    return (int)std::min(1e9, FORK_WORK * std::max(1.0, f));
+}
+
 static gg_status walk_setup(gg_ctx *c, bool subset, long long nt)
 {
     gg_status st;
@@ -845,7 +861,9 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
     p.forks = c->forks.p;
     p.own_forks = c->own_forks.p;
     p.fork_max = ntargets <= FORK_TASK_TARGETS ? FORK_RECORDS : 0;
-    p.may_fork = may_fork(c, d_active != nullptr, ntargets);
+    // (without an OldAcc the relative criterion opens every node, and no walk is longer than the others)
+    p.may_fork = may_fork(c, d_active != nullptr, ntargets) && (theta > 0 || p.oldacc_in);
+    p.fork_work = fork_work(tol, theta);
     p.task_walk = 0;
     p.stack = c->stack.p;
     p.stack_cap = c->stack_cap;

@@ -64,11 +64,12 @@ gg_status gg_launch_tree(const unsigned long long *keys, const int *poff, int S,
 // 5.6).
 #define FORK_MIN_TARGETS 98304
 #define FORK_MAX_TARGETS 300000
-// Work (node tests, list entries; a softened entry counts four) after which a walk
-// is cut: about twice a mean group's, or four times in systems above
-// FORK_HALF_TARGETS.  Walk ms uncut / cut at 8192 / 16384 / 32768: Plummer 65,536
-// 0.34 / 0.31 / 0.35 / 0.35, galaxy 100,000 0.97 / 0.78 / 0.81 / 0.95, galaxy
-// 262,144 2.06 / 2.73 / 1.38 / 1.56.
+// Work (node tests, list entries; a softened entry counts three) after which a walk
+// is cut at GIZMO's tolerance: about twice a mean group's, or four times in systems
+// above FORK_HALF_TARGETS.  Walk ms uncut / cut at 8192 / 16384 / 32768: Plummer
+// 65,536 0.34 / 0.31 / 0.35 / 0.35, galaxy 100,000 0.97 / 0.78 / 0.81 / 0.95, galaxy
+// 262,144 2.06 / 2.73 / 1.38 / 1.56.  Stricter criteria make every walk longer; the
+// work of a cut grows with them (fork_work).
 #define FORK_HALF_TARGETS 131072
 #define FORK_WORK 16384
 #define FORK_WALKS 8        // sub-walks the pending nodes are dealt to
@@ -117,6 +118,7 @@ struct WalkParams {
     char *own_forks;            // a record of FORK_OWN_BYTES per resident warp
     int fork_max;
     int may_fork;               // some walk of this launch may be cut
+    int fork_work;              // ... after this much work (half of it up to FORK_HALF_TARGETS)
     int task_walk;              // this launch runs the sub-walks of the cuts
     int *stack;
     int stack_cap;

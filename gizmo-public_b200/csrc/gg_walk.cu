@@ -592,18 +592,13 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         // Long walks.  A group with far more work than most (a dense centre, a box
         // that reaches into one) would set the length of a walk that has only a few
         // groups per warp.  Once its work (node tests, list entries) reaches
-        // FORK_WORK the nodes still pending are dealt out to FORK_WALKS sub-walks
+        // p.fork_work the nodes still pending are dealt out to FORK_WALKS sub-walks
         // with sums of their own: tasks of a second launch, or, when the records of
         // cuts are used up, the same warp's next work.  The sums are added in order
-        // either way, and whether and where a walk is cut depends on the group and
-        // its system's size alone, so a system's results do not depend on what it is
-        // batched with.
+        // either way, and whether and where a walk is cut depends on the group, its
+        // system's size and the opening criterion alone, so a system's results do not
+        // depend on what it is batched with.
         int cut_at = INT_MAX;
-        if (CUT && !p.task_walk) {
-            const int nt = p.toff[grp.sys + 1] - p.toff[grp.sys];
-            if (nt >= FORK_MIN_TARGETS && nt <= FORK_MAX_TARGETS)
-                cut_at = nt <= FORK_HALF_TARGETS ? FORK_WORK / 2 : FORK_WORK;
-        }
 
         // ---- targets of the group
         Targets<TPL> T;
@@ -647,6 +642,11 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             hw[q] = fmax(0.5 * (bmax[q] - bmin[q]), fmax(bmax[q] - cg[q], cg[q] - bmin[q]));
         }
         aold_min = warp_min_d(aold_min);
+        if (CUT && !p.task_walk && (theta > 0.0 || aold_min > 0.0)) {   // (OldAcc 0 opens every node)
+            const int nt = p.toff[grp.sys + 1] - p.toff[grp.sys];
+            if (nt >= FORK_MIN_TARGETS && nt <= FORK_MAX_TARGETS)
+                cut_at = nt <= FORK_HALF_TARGETS ? p.fork_work / 2 : p.fork_work;
+        }
         hmin = (float)warp_min_d((double)hmin);
         hmax = (float)warp_max_d((double)hmax);
 #pragma unroll

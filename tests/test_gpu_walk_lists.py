@@ -80,27 +80,34 @@ def test_close_pairs_at_any_scale(group_size, scale, h, m):
     assert np.all(np.abs(pot - wpot) < 2e-6 * (m / r).sum(1))
 
 
-def test_cut_walks_give_the_same_bits_alone_and_in_a_batch():
+@pytest.mark.parametrize("every_node", [False, True])
+def test_cut_walks_give_the_same_bits_alone_and_in_a_batch(every_node):
     """A system in the range of sizes whose long walks are cut, opening every
     node: its sub-walks run as tasks when it is alone, and as each warp's own
-    work in a batch too large for that.  Same interactions, same bits."""
+    work in a batch too large for that.  Same interactions, same bits.  (A strict
+    Barnes-Hut pass has long walks too, but none longer than the work of a cut.)"""
     n = 98304
     pos, mass, h = _system(n, "one", 5)
     big = 400001 - n
     rng = np.random.default_rng(6)
     more, mm = rng.normal(size=(big, 3)), np.full(big, 1.0)
     theta = dict(err_tol_theta=0.15)     # a Barnes-Hut pass strict enough for long walks
+    old, both = None, None
+    if every_node:
+        theta = dict(err_tol_force_acc=0.001)
+        old = np.full(n, 1e-30)
+        both = np.concatenate([old, np.full(big, 1e30)])
     with ggb200.GravityTree() as t:
         t.load(pos, mass, h)
         t.build()
-        alone = t.evaluate(want_ninter=True, **theta)
+        alone = t.evaluate(old_acc=old, want_ninter=True, **theta)
         cuts = [t.last_cuts()]
         t.load(np.concatenate([pos, more]), np.concatenate([mass, mm]), np.concatenate([h, np.full(big, h[0])]),
                counts=[n, big])
         t.build()
-        batch = t.evaluate(want_ninter=True, **theta)
+        batch = t.evaluate(old_acc=both, want_ninter=True, **theta)
         cuts.append(t.last_cuts())
-    assert cuts == [cuts[0], cuts[0]] and cuts[0] > 0
+    assert cuts[0] == cuts[1] and (cuts[0] > 0) == every_node
     assert alone[3]["error_word"] == 0 and batch[3]["error_word"] == 0
     assert alone[2].mean() > 8192        # long enough to be cut
     for a, b in zip(alone[:3], batch[:3]):
@@ -118,7 +125,7 @@ def test_cut_walks_that_open_every_node_are_the_direct_sum(n, other, group_size,
         pos = np.concatenate([pos, rng.normal(size=(other, 3))])
         mass, h = np.concatenate([mass, np.ones(other)]), np.full(n + other, h[0])
     counts = [n, other] if other else [n]
-    old = np.zeros(n + other)
+    old = np.full(n + other, 1e-30)    # opens every node; no walk is cut with an OldAcc of 0
     old[n:] = 1e30                     # the other system's nodes are used whole
     with ggb200.GravityTree(group_size=group_size, node_staging=staging) as t:
         t.load(pos, mass, h, counts=counts)
@@ -152,7 +159,7 @@ def test_cut_walks_of_a_subset_and_after_a_stack_overflow(group_size):
         with ggb200.GravityTree(group_size=group_size, walk_stack_entries=entries) as t:
             t.load(pos, mass, h)
             t.build()
-            out.append(t.evaluate(active=act, old_acc=np.zeros(n), err_tol_force_acc=0.001, want_ninter=True))
+            out.append(t.evaluate(active=act, old_acc=np.full(n, 1e-30), err_tol_force_acc=0.001, want_ninter=True))
             assert t.last_cuts() > 0
     assert out[0][3]["error_word"] == 0 and out[1][3]["error_word"] == 0
     for a, b in zip(out[0][:3], out[1][:3]):
@@ -162,6 +169,33 @@ def test_cut_walks_of_a_subset_and_after_a_stack_overflow(group_size):
     want, wpot = oracle.direct_sum(pos, mass, h, targets=act[few])
     assert np.linalg.norm(out[0][0][few] - want) < 3e-6 * np.linalg.norm(want)
     assert np.linalg.norm(out[0][1][few] - wpot) < 2e-6 * np.linalg.norm(wpot)
+
+
+@pytest.mark.parametrize("criterion", ["strict", "all"])
+@pytest.mark.parametrize("group_size", [32, 64])
+def test_cuts_do_not_lengthen_walks_that_are_all_long(group_size, criterion):
+    """300,000 targets are the most a system is cut with.  Where a strict criterion
+    (or an OldAcc of 0) makes every walk long, one more target, which switches cuts
+    off, changes the time by little (cuts of most walks made it 1.3 to 1.8)."""
+    import torch
+    rng = np.random.default_rng(13)
+    pos = rng.normal(size=(300001, 3)) * (0.05 + rng.random((300001, 1)) ** 4)
+    best = {}
+    for n in (300000, 300001):
+        rec = torch.from_numpy(ggb200.make_records(pos[:n], np.ones(n), np.full(n, 1e-3)).view(np.uint8)).cuda()
+        acc = torch.empty((n, 3), dtype=torch.float64, device="cuda")
+        with ggb200.GravityTree(group_size=group_size, timing=True) as t:
+            t.set_stream(torch.cuda.current_stream().cuda_stream)
+            t.load_device(rec, [n])
+            t.build()
+            t.evaluate_device(acc, err_tol_theta=0.7)
+            old = acc.norm(dim=1) if criterion == "strict" else torch.zeros(n, dtype=torch.float64, device="cuda")
+            times = []
+            for _ in range(5):
+                t.evaluate_device(acc, d_old_acc=old, err_tol_force_acc=1e-5)
+                times.append(t.last_stats()["ms_walk"])
+            best[n] = min(times)
+    assert best[300000] < 1.15 * best[300001], best
 
 
 def test_small_subsets_of_a_large_system_are_not_prepared_for_cuts():
