@@ -356,6 +356,9 @@ __device__ __forceinline__ void flush_far(const float *__restrict__ far, int n, 
 // rsqrt give u and 1/u, and force and potential share t^4/u (t and the spline:
 // see spline_wf2).
 // r^2 = 0 gives u = 1e-18: a finite force factor, times an offset of zero.
+// Unrolled by two, so that few warps have two chains in flight: walk of 100
+// targets scattered over a galaxy of 500,000 (4 groups) 32.5 -> 32.0 ms, 4.2M galaxy
+// 44.7 -> 44.3 ms.  (The far flush unrolled spills: 45.8 ms.)
 template <int TPL, int SPLIT, bool POT>
 __device__ __forceinline__ void flush_near(const float *__restrict__ near, int n, int part, Targets<TPL> &T)
 {
@@ -367,7 +370,7 @@ __device__ __forceinline__ void flush_near(const float *__restrict__ near, int n
     }
     const float2 *X = reinterpret_cast<const float2 *>(near) + part;
     constexpr int c2 = NEAR_CAP / 2;
-#pragma unroll 1
+#pragma unroll 2
     for (int q = n / (2 * SPLIT); q > 0; q--, X += SPLIT) {
         const float2 ex = X[0], ey = X[c2], ez = X[2 * c2], h2 = X[3 * c2], mh = X[4 * c2], mh3 = X[5 * c2];
 #pragma unroll
@@ -588,7 +591,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         }
         if (CUT) __syncwarp();
         const GGGroup grp = p.groups[g];
-        const long long t_start = clock64();
+        const unsigned t_start = (unsigned)clock();
         // Long walks.  A group with far more work than most (a dense centre, a box
         // that reaches into one) would set the length of a walk that has only a few
         // groups per warp.  Once its work (node tests, list entries) reaches
@@ -603,7 +606,6 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         // ---- targets of the group
         Targets<TPL> T;
         double tx[TPL], ty[TPL], tz[TPL];
-        int tpi[TPL];
         double bmin[3] = {INFINITY, INFINITY, INFINITY}, bmax[3] = {-INFINITY, -INFINITY, -INFINITY};
         double aold_min = INFINITY;
         float hmin = INFINITY, hmax = 0.f;
@@ -612,14 +614,12 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             int k = s * LP + lane % LP;
             bool v = k < grp.count;
             T.valid[s] = v;
-            tpi[s] = -1;
             tx[s] = ty[s] = tz[s] = 0.0;
             T.h[s] = 0.f;
             T.hinv[s] = INFINITY;
             if (v) {
                 int t = grp.first + k;
                 int pi = p.tlist ? p.tlist[t] : t;
-                tpi[s] = pi;
                 GGPart q = load_part(p.parts + pi);
                 tx[s] = q.x; ty[s] = q.y; tz[s] = q.z;
                 T.h[s] = q.h;
@@ -1032,8 +1032,9 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         __syncwarp();   // the next group's entries overwrite the lists
 
         // ---- results
-        // this group's device cycles per target: the cost the next walk orders its groups by
-        const float tcost = (float)(clock64() - t_start) / (float)grp.count;
+        // this group's device cycles per target: the cost the next walk orders its groups
+        // by (from 32 bits: a walk beyond two seconds only loses its place)
+        const float tcost = (float)((unsigned)clock() - t_start) / (float)grp.count;
         int mycount = 0;
 #pragma unroll
         for (int s = 0; s < TPL; s++) {
@@ -1073,7 +1074,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
                     continue;
                 }
             }
-            write_target<POT>(p, grp.first + slot, tpi[s], T.hinv[s], ax, ay, az, ph, nint, tcost);
+            const int tt = grp.first + slot;   // (looked up again: a register less through the walk)
+            write_target<POT>(p, tt, p.tlist ? p.tlist[tt] : tt, T.hinv[s], ax, ay, az, ph, nint, tcost);
             mycount += nint;
         }
 #pragma unroll
