@@ -249,7 +249,7 @@ struct gg_ctx {
     DevBuf<unsigned> g_stat;
     DevBuf<WalkFork> forks;                // records of cut walks
     DevBuf<char> own_forks;
-    DevBuf<int> counters;                  // [0] group counter
+    DevBuf<int> counters;                  // of the walk (WALK_COUNTERS), then two words per record of a cut
     DevBuf<unsigned long long> inter;      // interaction total
     DevBuf<int> stack;
     DevBuf<int> err;
@@ -425,12 +425,12 @@ extern "C" gg_status gg_create(const gg_config *cfg, gg_ctx **out)
     for (int i = 0; i < 8; i++) cudaEventCreate(&ctx->ev[i]);
     ctx->have_events = true;
     memset(&ctx->last, 0, sizeof ctx->last);
-    if ((st = ctx->err.ensure(8)) || (st = ctx->counters.ensure(8)) || (st = ctx->inter.ensure(4))) {
+    if ((st = ctx->err.ensure(8)) || (st = ctx->counters.ensure(WALK_COUNTERS + 2 * FORK_RECORDS)) || (st = ctx->inter.ensure(4))) {
         gg_destroy(ctx);
         return st;
     }
     cudaMemset(ctx->err.p, 0, 8 * sizeof(int));
-    cudaMemset(ctx->counters.p, 0, 8 * sizeof(int));
+    cudaMemset(ctx->counters.p, 0, WALK_COUNTERS * sizeof(int));
     *out = ctx;
     return GG_OK;
 }
@@ -837,7 +837,7 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
             return st;
         gorder = c->gorder.p;
     }
-    GG_CUDA_TRY(cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(int), s));
+    GG_CUDA_TRY(cudaMemsetAsync(c->counters.p, 0, (WALK_COUNTERS + 2 * FORK_RECORDS) * sizeof(int), s));
     GG_CUDA_TRY(cudaMemsetAsync(c->inter.p, 0, 4 * sizeof(unsigned long long), s));
     WalkParams p;
     p.nodes = c->nodes.p;
@@ -864,7 +864,8 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
     // (without an OldAcc the relative criterion opens every node, and no walk is longer than the others)
     p.may_fork = may_fork(c, d_active != nullptr, ntargets) && (theta > 0 || p.oldacc_in);
     p.fork_work = fork_work(tol, theta);
-    p.task_walk = 0;
+    p.fork_ready = c->counters.p + WALK_COUNTERS;
+    p.fork_parts = p.fork_ready + FORK_RECORDS;
     p.stack = c->stack.p;
     p.stack_cap = c->stack_cap;
     p.err = c->err.p;

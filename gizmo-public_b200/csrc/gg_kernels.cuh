@@ -74,7 +74,7 @@ gg_status gg_launch_tree(const unsigned long long *keys, const int *poff, int S,
 #define FORK_WORK 16384
 #define FORK_WALKS 8        // sub-walks the pending nodes are dealt to
 #define FORK_PENDING 2048   // pending nodes at most
-#define FORK_RECORDS 512    // cuts whose sub-walks can run as tasks of their own
+#define FORK_RECORDS 512    // cuts whose sub-walks can run as tasks of any warp
 // ... in launches of at most this many targets; with more, there is work enough
 // for every warp, and each runs its own sub-walks
 #define FORK_TASK_TARGETS 400000
@@ -92,9 +92,11 @@ struct WalkFork {
     int nint[FORK_WALKS][64];
 };
 #define FORK_OWN_BYTES offsetof(WalkFork, sum)
-// places in WalkParams.group_counter: groups handed out, cuts made, tasks handed out
+// places in WalkParams.group_counter: groups handed out, cuts made, tasks handed out, groups finished
 #define WALK_FORK_COUNTER 1
 #define WALK_TASK_COUNTER 2
+#define WALK_DONE_COUNTER 3
+#define WALK_COUNTERS 8     // then, per record: whether it is complete, and how many of its parts are finished
 
 struct WalkParams {
     const GGNode *nodes;
@@ -112,14 +114,14 @@ struct WalkParams {
     double *pot;                // per output slot, may be NULL
     int *ninter;                // per output slot, may be NULL
     unsigned long long *interactions;   // [0] interactions, [1] far / [2] near list entries, [3] nodes tested
-    int *group_counter;         // three counters, zero at the launch
+    int *group_counter;         // counters, zero at the launch
     const int *toff;            // target offsets per system
     WalkFork *forks;            // fork_max records
     char *own_forks;            // a record of FORK_OWN_BYTES per resident warp
     int fork_max;
     int may_fork;               // some walk of this launch may be cut
     int fork_work;              // ... after this much work (half of it up to FORK_HALF_TARGETS)
-    int task_walk;              // this launch runs the sub-walks of the cuts
+    int *fork_ready, *fork_parts;   // per record, zero at the launch
     int *stack;
     int stack_cap;
     int *err;

@@ -358,8 +358,9 @@ __device__ __forceinline__ void flush_far(const float *__restrict__ far, int n, 
 // r^2 = 0 gives u = 1e-18: a finite force factor, times an offset of zero.
 // Unrolled by two, so that few warps have two chains in flight: walk of 100
 // targets scattered over a galaxy of 500,000 (4 groups) 32.5 -> 32.0 ms, 4.2M galaxy
-// 44.7 -> 44.3 ms.  (The far flush unrolled spills: 45.8 ms.)
-template <int TPL, int SPLIT, bool POT>
+// 44.7 -> 44.3 ms.  (The far flush unrolled spills: 45.8 ms; so does this one in the
+// kernel of cut walks of groups beyond 32, where it stays as it is.)
+template <int TPL, int SPLIT, bool POT, int UNROLL>
 __device__ __forceinline__ void flush_near(const float *__restrict__ near, int n, int part, Targets<TPL> &T)
 {
     float2 px[TPL], py[TPL], pz[TPL], pp[TPL], nx[TPL], ny[TPL], nz[TPL];
@@ -370,7 +371,7 @@ __device__ __forceinline__ void flush_near(const float *__restrict__ near, int n
     }
     const float2 *X = reinterpret_cast<const float2 *>(near) + part;
     constexpr int c2 = NEAR_CAP / 2;
-#pragma unroll 2
+#pragma unroll UNROLL
     for (int q = n / (2 * SPLIT); q > 0; q--, X += SPLIT) {
         const float2 ex = X[0], ey = X[c2], ez = X[2 * c2], h2 = X[3 * c2], mh = X[4 * c2], mh3 = X[5 * c2];
 #pragma unroll
@@ -529,6 +530,72 @@ __device__ __forceinline__ void write_target(const WalkParams &p, int t, int pi,
     if (p.cost_out) p.cost_out[li] = tcost;
 }
 
+// ---- cut walks (see k_walk)
+__device__ __forceinline__ int ld_flag(const int *p)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_flag(int *p, int v)
+{
+    asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// The next sub-walk for a warp that found no group left, or -1.  Sub-walks are
+// numbered by cut; a warp takes the next number and waits until that cut is made or
+// every group is finished.  All groups are held by running warps by then, so the
+// wait ends; it is bounded all the same (some twenty seconds).
+#define WALK_TASK_LIMIT (1 << 22)
+__device__ __noinline__ int next_task(const WalkParams &p, int ngroups)
+{
+    const int t = atomicAdd(p.group_counter + WALK_TASK_COUNTER, 1), f = t / FORK_WALKS;
+    if (f >= p.fork_max) return -1;
+    unsigned ns = 256;
+    for (int i = 0; i < WALK_TASK_LIMIT; i++) {
+        const bool over = ld_flag(p.group_counter + WALK_DONE_COUNTER) >= ngroups;
+        if (over) __threadfence();   // cuts of finished groups are seen from here on
+        if (ld_flag(p.fork_ready + f)) {
+            __threadfence();
+            return t;
+        }
+        if (over) return -1;
+        __nanosleep(ns);
+        ns = min(2 * ns, 4096u);
+    }
+    atomicOr(p.err, GG_EBIT_WALK_TIMEOUT);
+    return -1;
+}
+
+// The sums of a cut walk's parts, added in order, by one warp.
+template <bool POT>
+__device__ __noinline__ void join_cut(const WalkParams &p, const WalkFork *fork, int group, int lane)
+{
+    const GGGroup grp = p.groups[group];
+    int mycount = 0;
+    for (int slot = lane; slot < grp.count; slot += 32) {   // written by other warps of this launch: read through L2
+        auto part = [](const double4 *q) {
+            const double2 a = __ldcg(reinterpret_cast<const double2 *>(q)),
+                          b = __ldcg(reinterpret_cast<const double2 *>(q) + 1);
+            return make_double4(a.x, a.y, b.x, b.y);
+        };
+        double4 a = part(fork->sum0 + slot);
+        int nint = __ldcg(fork->nint0 + slot);
+        for (int i = 0; i < FORK_WALKS; i++) {
+            const double4 q = part(fork->sum[i] + slot);
+            a.x += q.x; a.y += q.y; a.z += q.z; a.w += q.w;
+            nint += __ldcg(fork->nint[i] + slot);
+        }
+        const int t = grp.first + slot, pi = p.tlist ? p.tlist[t] : t;
+        const float h = p.parts[pi].h;
+        write_target<POT>(p, t, pi, h > 0.f ? __frcp_rn(h) : INFINITY, a.x, a.y, a.z, a.w, nint, __ldcg(&fork->cost));
+        mycount += nint;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mycount += __shfl_xor_sync(FULL, mycount, o);
+    if (lane == 0) atomicAdd(p.interactions, (unsigned long long)mycount);
+}
+
 __device__ __forceinline__ int warp_incl_scan(int v, int lane)
 {
 #pragma unroll
@@ -542,7 +609,7 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane)
 // exactly the reference's); otherwise the tests run in FP32 on FP64-formed
 // offsets from the group centre, against a bounding box rounded outwards.
 template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA, bool CUT>
-__global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
+__global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(const __grid_constant__ WalkParams p)
 {
     extern __shared__ float4 walk_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -562,11 +629,12 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
     int *qbase = run + 32, *qend = qbase + RUNS;   // queued runs: first particle less its position, end position
     const unsigned bar = (unsigned)__cvta_generic_to_shared(qend + RUNS);
     // state of a cut walk (CUT): kept here, not in registers
-    struct CutState { WalkFork *fork; int sub, npend, own, group; };
+    struct CutState { WalkFork *fork; int sub, npend, own, group, tasks, at; };
     CutState &cut = *reinterpret_cast<CutState *>(qend + RUNS + 4);
     if (lane == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (CUT) cut.own = cut.tasks = 0;
     }
     __syncwarp();
     unsigned phase = 0;   // parity of the barrier phase the next wait is for
@@ -577,32 +645,51 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
 
     for (;;) {
         int g = 0;
-        if (lane == 0) g = atomicAdd(p.group_counter + (p.task_walk ? WALK_TASK_COUNTER : 0), 1);
-        g = __shfl_sync(FULL, g, 0);
-        if (CUT && p.task_walk) {
-            if (g >= min(p.group_counter[WALK_FORK_COUNTER], p.fork_max) * FORK_WALKS) break;
-            WalkFork *const fork = p.forks + g / FORK_WALKS;
-            if (lane == 0) cut = {fork, 1 + g % FORK_WALKS, fork->npend, 0, fork->group};
-            g = fork->group;
-        } else {
+        if (!CUT) {
+            if (lane == 0) g = atomicAdd(p.group_counter, 1);
+            g = __shfl_sync(FULL, g, 0);
             if (g >= ngroups) break;
             if (p.gorder) g = (int)p.gorder[g];
-            if (CUT && lane == 0) cut = {nullptr, 0, 0, 0, g};
+        } else {
+            if (lane == 0) {
+                if (cut.own && cut.sub < FORK_WALKS) {   // the warp's own next sub-walk
+                    cut.sub++;
+                    g = cut.group;
+                } else if (cut.tasks || (g = atomicAdd(p.group_counter, 1)) >= ngroups) {
+                    // groups have run out: sub-walks of cut ones
+                    cut.tasks = 1;
+                    const int t = next_task(p, ngroups);
+                    if (t >= 0) {
+                        WalkFork *const fork = p.forks + t / FORK_WALKS;
+                        cut.fork = fork;
+                        cut.sub = 1 + t % FORK_WALKS;
+                        cut.npend = __ldcg(&fork->npend);
+                        cut.group = __ldcg(&fork->group);
+                        cut.own = 0;
+                    }
+                    g = t >= 0 ? cut.group : -1;
+                } else {
+                    if (p.gorder) g = (int)p.gorder[g];
+                    cut.fork = nullptr;
+                    cut.sub = cut.npend = cut.own = 0;
+                    cut.group = g;
+                }
+            }
+            g = __shfl_sync(FULL, g, 0);
+            if (g < 0) break;
+            __syncwarp();
         }
-        if (CUT) __syncwarp();
         const GGGroup grp = p.groups[g];
         const unsigned t_start = (unsigned)clock();
         // Long walks.  A group with far more work than most (a dense centre, a box
         // that reaches into one) would set the length of a walk that has only a few
         // groups per warp.  Once its work (node tests, list entries) reaches
         // p.fork_work the nodes still pending are dealt out to FORK_WALKS sub-walks
-        // with sums of their own: tasks of a second launch, or, when the records of
-        // cuts are used up, the same warp's next work.  The sums are added in order
-        // either way, and whether and where a walk is cut depends on the group, its
+        // with sums of their own: tasks of the warps that have run out of groups, or,
+        // when the records of cuts are used up, the same warp's next work.  The sums
+        // are added in order either way, and whether and where a walk is cut depends on the group, its
         // system's size and the opening criterion alone, so a system's results do not
         // depend on what it is batched with.
-        int cut_at = INT_MAX;
-
         // ---- targets of the group
         Targets<TPL> T;
         double tx[TPL], ty[TPL], tz[TPL];
@@ -642,10 +729,12 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             hw[q] = fmax(0.5 * (bmax[q] - bmin[q]), fmax(bmax[q] - cg[q], cg[q] - bmin[q]));
         }
         aold_min = warp_min_d(aold_min);
-        if (CUT && !p.task_walk && (theta > 0.0 || aold_min > 0.0)) {   // (OldAcc 0 opens every node)
+        if (CUT && lane == 0) {
             const int nt = p.toff[grp.sys + 1] - p.toff[grp.sys];
-            if (nt >= FORK_MIN_TARGETS && nt <= FORK_MAX_TARGETS)
-                cut_at = nt <= FORK_HALF_TARGETS ? p.fork_work / 2 : p.fork_work;
+            // (sub-walks are not cut again; with an OldAcc of 0 every node is opened)
+            const bool may = cut.sub == 0 && nt >= FORK_MIN_TARGETS && nt <= FORK_MAX_TARGETS &&
+                             (theta > 0.0 || aold_min > 0.0);
+            cut.at = !may ? INT_MAX : nt <= FORK_HALF_TARGETS ? p.fork_work / 2 : p.fork_work;
         }
         hmin = (float)warp_min_d((double)hmin);
         hmax = (float)warp_max_d((double)hmax);
@@ -671,7 +760,6 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         // records is in flight during the tests.  One loop does whatever is due,
         // so that every part appears in the code once (the kernel is large
         // against the instruction cache).
-      for (;;) {   // sub-walks
 #pragma unroll
         for (int s = 0; s < TPL; s++) {
             T.self[s] = 0;
@@ -694,7 +782,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             node[0] = lane == 0 ? grp.root : -1;
             if (CUT && cut.sub > 0) {   // every FORK_WALKS-th pending node: at most FORK_PENDING / FORK_WALKS
                 const int sub = cut.sub, m = (cut.npend - sub + FORK_WALKS) / FORK_WALKS;
-                for (int i = lane; i < m; i += 32) sstack[i] = cut.fork->pending[sub - 1 + FORK_WALKS * i];
+                for (int i = lane; i < m; i += 32) sstack[i] = __ldcg(cut.fork->pending + sub - 1 + FORK_WALKS * i);
                 __syncwarp();
                 k = min(m, 32 * NH);
                 sp = m - k;
@@ -755,7 +843,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             if (nn >= nlimit) {
                 const int m = nn & ~(QUANTUM - 1);
                 __syncwarp();
-                if (hone >= 0.f) flush_near<TPL, SPLIT, POT>(near, m, part, T);
+                if (hone >= 0.f) flush_near<TPL, SPLIT, POT, CUT && SPLIT == 1 ? 1 : 2>(near, m, part, T);
                 else flush_near_mixed<TPL, SPLIT, POT>(near, m, part, T);
                 nn -= m;
                 list_shift<NEAR_ARRAYS, NEAR_CAP>(near, m, nn, lane);
@@ -921,34 +1009,6 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
                     sp = m;
                 }
                 __syncwarp();
-                if (CUT && tested + list_far + 3 * list_near >= cut_at && gsp + sp + ctot >= 2 * FORK_WALKS &&
-                    gsp + sp + ctot <= FORK_PENDING) {
-                    int f = 0;
-                    if (lane == 0) f = atomicAdd(p.group_counter + WALK_FORK_COUNTER, 1);
-                    f = __shfl_sync(FULL, f, 0);
-                    const bool own = f >= p.fork_max;
-                    WalkFork *const fork =
-                        own ? reinterpret_cast<WalkFork *>(p.own_forks + (size_t)(blockIdx.x * WALK_WARPS + warp) *
-                                                                             FORK_OWN_BYTES)
-                            : p.forks + f;
-                    for (int i = lane; i < gsp; i += 32) fork->pending[i] = gstack[i];
-                    for (int i = lane; i < sp; i += 32) fork->pending[gsp + i] = sstack[i];
-                    sp += gsp;
-                    for (int w = 0; w < ctot; w += 32) {
-                        const int i = expand(cbase, cbeg, cfin, w);
-                        if (w + lane < ctot) fork->pending[sp + w + lane] = i;
-                    }
-                    if (lane == 0) {
-                        fork->group = cut.group;
-                        fork->npend = sp + ctot;
-                        cut.fork = fork;
-                        cut.npend = sp + ctot;
-                        cut.own = own;
-                    }
-                    cut_at = INT_MAX;
-                    gsp = sp = ctot = 0;   // the rest of this sub-walk: queued particles and lists
-                    __syncwarp();
-                }
                 k = min(sp + ctot, 32 * NH);
                 const int w0 = ctot - k;   // first position taken now; negative: from the stack
                 int node[NH];
@@ -960,6 +1020,38 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
                     if (w + lane < 0) node[h] = sstack[sp + w + lane];
                 }
                 sp += min(w0, 0);
+                // (only where all children are among the next nodes: then those, in registers, and the
+                // stack are all that is pending)
+                if (CUT && tested + list_far + 3 * list_near >= cut.at && w0 <= 0 && gsp + sp + k >= 2 * FORK_WALKS &&
+                    gsp + sp + k <= FORK_PENDING) {
+                    int f = 0;
+                    if (lane == 0) f = atomicAdd(p.group_counter + WALK_FORK_COUNTER, 1);
+                    f = __shfl_sync(FULL, f, 0);
+                    const bool own = f >= p.fork_max;
+                    WalkFork *const fork =
+                        own ? reinterpret_cast<WalkFork *>(p.own_forks + (size_t)(blockIdx.x * WALK_WARPS + warp) *
+                                                                             FORK_OWN_BYTES)
+                            : p.forks + f;
+                    for (int i = lane; i < gsp; i += 32) fork->pending[i] = gstack[i];
+                    for (int i = lane; i < sp; i += 32) fork->pending[gsp + i] = sstack[i];
+#pragma unroll
+                    for (int h = 0; h < NH; h++)
+                        if (32 * h + lane < k) fork->pending[gsp + sp + 32 * h + lane] = node[h];
+                    __syncwarp();
+                    if (lane == 0) {
+                        fork->group = cut.group;
+                        fork->npend = gsp + sp + k;
+                        cut.fork = fork;
+                        cut.npend = gsp + sp + k;
+                        cut.own = own;
+                        if (!own) {   // the record is complete: tasks may start
+                            __threadfence();
+                            st_flag(p.fork_ready + f, 1);
+                        }
+                    }
+                    gsp = sp = k = 0;   // the rest of this part: queued particles and lists
+                    __syncwarp();
+                }
                 stage(node, k);
                 if (w0 > 0) {   // the other children go to the stack
                     while (sp + w0 > WALK_SSTACK) {   // up to half of it spills to global memory, oldest first (w0 < WALK_SSTACK)
@@ -1015,19 +1107,29 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
         }
         if (!tma) asm volatile("cp.async.wait_all;" ::: "memory");   // no copy into the slot outlives its group
         if (timed_out) {   // copies may still be in flight: wait once more, then leave
-            if (lane == 0) atomicOr(p.err, GG_EBIT_WALK_TIMEOUT);
+            if (lane == 0) {
+                atomicOr(p.err, GG_EBIT_WALK_TIMEOUT);
+                if (CUT && !cut.tasks) atomicAdd(p.group_counter + WALK_DONE_COUNTER, 1);
+            }
             bar_wait(bar, phase);
             return;
         }
         if (overflow) {
             if (tma && !bar_wait(bar, phase)) {   // the copies staged for a round that will not run
-                if (lane == 0) atomicOr(p.err, GG_EBIT_WALK_TIMEOUT);
+                if (lane == 0) {
+                    atomicOr(p.err, GG_EBIT_WALK_TIMEOUT);
+                    if (CUT && !cut.tasks) atomicAdd(p.group_counter + WALK_DONE_COUNTER, 1);
+                }
                 return;
             }
             if (tma) phase ^= 1u;
-            if (lane == 0) atomicOr(p.err, GG_EBIT_STACK_OVERFLOW);
+            if (lane == 0) {
+                atomicOr(p.err, GG_EBIT_STACK_OVERFLOW);
+                if (CUT && !cut.tasks) atomicAdd(p.group_counter + WALK_DONE_COUNTER, 1);
+                if (CUT) cut.own = 0;
+            }
             __syncwarp();
-            break;   // to the next group
+            continue;   // to the next group
         }
         __syncwarp();   // the next group's entries overwrite the lists
 
@@ -1086,40 +1188,20 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(WalkParams p)
             atomicAdd(p.interactions + 2, (unsigned long long)list_near);
             atomicAdd(p.interactions + 3, (unsigned long long)tested);
         }
-        if (!CUT || !cut.own || cut.sub == FORK_WALKS) break;
-        __syncwarp();
-        if (lane == 0) cut.sub++;
-        __syncwarp();   // also the pending nodes, written by other lanes
-      }
-    }
-}
-
-// The sums of the cut walks whose sub-walks ran as tasks, added in order: one
-// warp per cut.
-template <bool POT>
-__global__ void __launch_bounds__(WALK_THREADS) k_walk_join(WalkParams p)
-{
-    const int lane = threadIdx.x & 31, w = (blockIdx.x * WALK_THREADS + threadIdx.x) >> 5;
-    if (w >= min(p.group_counter[WALK_FORK_COUNTER], p.fork_max)) return;
-    const WalkFork &f = p.forks[w];
-    const GGGroup grp = p.groups[f.group];
-    int mycount = 0;
-    for (int slot = lane; slot < grp.count; slot += 32) {
-        double4 a = f.sum0[slot];
-        int nint = f.nint0[slot];
-        for (int i = 0; i < FORK_WALKS; i++) {
-            const double4 q = f.sum[i][slot];
-            a.x += q.x; a.y += q.y; a.z += q.z; a.w += q.w;
-            nint += f.nint[i][slot];
+        if (CUT) {
+            __syncwarp();   // also before lane 0 goes on to the next sub-walk
+            int last = 0;
+            if (lane == 0) {
+                if (cut.fork) __threadfence();
+                if (cut.fork && !cut.own) last = atomicAdd(p.fork_parts + (cut.fork - p.forks), 1) == FORK_WALKS;
+                if (!cut.tasks && (!cut.own || cut.sub == FORK_WALKS))
+                    atomicAdd(p.group_counter + WALK_DONE_COUNTER, 1);
+                if (last) __threadfence();
+            }
+            // the last part of a cut walk to finish adds them all up
+            if (__shfl_sync(FULL, last, 0)) join_cut<POT>(p, cut.fork, cut.group, lane);
         }
-        const int t = grp.first + slot, pi = p.tlist ? p.tlist[t] : t;
-        const float h = p.parts[pi].h;
-        write_target<POT>(p, t, pi, h > 0.f ? __frcp_rn(h) : INFINITY, a.x, a.y, a.z, a.w, nint, f.cost);
-        mycount += nint;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mycount += __shfl_xor_sync(FULL, mycount, o);
-    if (lane == 0) atomicAdd(p.interactions, (unsigned long long)mycount);
 }
 
 template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA, bool CUT>
@@ -1129,16 +1211,11 @@ static void launch_walk_c(const WalkParams &p, int blocks, cudaStream_t st)
     cudaFuncSetAttribute(k_walk<TPL, SPLIT, F64T, POT, TMA, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     k_walk<TPL, SPLIT, F64T, POT, TMA, CUT><<<blocks, WALK_THREADS, smem, st>>>(p);
     gg_note_launches(1);
-    if (CUT && p.fork_max > 0) {   // the sub-walks of the walks that were cut
-        WalkParams q = p;
-        q.task_walk = 1;
-        k_walk<TPL, SPLIT, F64T, POT, TMA, CUT><<<blocks, WALK_THREADS, smem, st>>>(q);
-        k_walk_join<POT><<<(p.fork_max + WALK_WARPS - 1) / WALK_WARPS, WALK_THREADS, 0, st>>>(q);
-        gg_note_launches(2);
-    }
 }
 
-// walks that may be cut run a kernel of their own: the state of a cut costs registers
+// Walks that may be cut run a kernel of their own: the state of a cut costs
+// registers and about 8% of a short walk (Plummer 300,000 0.59 -> 0.64 ms); it gains
+// where few long walks end last (galaxy 300,000 2.4 -> 1.5 ms).
 template <int TPL, int SPLIT, bool F64T, bool POT, bool TMA>
 static void launch_walk_t(const WalkParams &p, int blocks, cudaStream_t st)
 {
