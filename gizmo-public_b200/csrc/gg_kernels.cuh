@@ -56,12 +56,17 @@ int gg_tree_grid();
 gg_status gg_launch_tree(const unsigned long long *keys, const int *poff, int S, int n, int leaf, int cap, TreeBuf tb,
                          const GGPart *parts, const GGDomainDev *dom, GGNode *nodes, cudaStream_t st);
 
-// Long walks are cut (gg_walk.cu) in systems that have a few groups per resident
-// warp.  Smaller systems come in batches and gain little alone (with 65,536 in the
-// range a batch of 48 served systems took 7% longer); in larger ones the groups
-// outnumber the warps so far that the longest, started first, end with the rest
-// (cut at 500,000 targets, a 10% subset of 4.2M particles took 6.9 ms instead of
-// 5.6).
+// Long walks are cut (gg_walk.cu) in systems of this range: they have a few groups
+// per resident warp, and the longest end last.  Walk ms uncut / cut at tolerance
+// 0.0025 in groups of 32 (galaxy, Plummer, clustered): 65,536 0.73 / 0.44, 0.34 /
+// 0.30, 0.37 / 0.41; 98,304 0.90 / 0.70, 0.40 / 0.32, 0.51 / 0.45; 200,000 1.88 / 1.12,
+// 0.67 / 0.66, 0.67 / 0.69; 300,000 2.69 / 1.55, 0.66 / 0.63, 0.77 / 0.79; 350,000 3.00 /
+// 2.98, 0.71 / 0.77, 1.07 / 0.94; 500,000 4.32 / 4.42, 0.85 / 0.92, 1.22 / 1.27.  Beyond
+// 300,000 the groups outnumber the warps so far that the longest, started first, end
+// with the rest, and the cut's own cost is left (a 10% subset of 4.2M particles, cut:
+// 5.7 ms instead of 5.3).  Below 98,304 a cut gains alone, but such systems come in
+// batches, whose groups fill the GPU (48 served systems with 65,536 in the range:
+// no difference).
 #define FORK_MIN_TARGETS 98304
 #define FORK_MAX_TARGETS 300000
 // Work (node tests, list entries; a softened entry counts three) after which a walk
