@@ -2,8 +2,8 @@
 //
 // A warp serves one group of up to 64 targets that are consecutive in
 // Peano-Hilbert order (two targets per lane; see Targets).  The warp walks the tree once
-// for the whole group with an explicit node stack: each round pops up to 32
-// nodes, one per lane, and tests them against the group's bounding box with
+// for the whole group with an explicit node stack: each round takes up to 64
+// nodes, two per lane, and tests them against the group's bounding box with
 // the reference's opening rules made conservative over the group
 // (distance = from the node's centre of mass to the box, the smallest
 // ErrTolForceAcc*OldAcc of the group, the largest target softening):
@@ -268,8 +268,9 @@ __device__ __forceinline__ float2 spline_wf2(float2 u, float2 iu, float2 *wp)
 // target per lane L1 was 82% busy in the far flush).
 //
 // What bounds the walk is instruction issue.  A packed FP32x2 instruction takes
-// two issue slots; counting those twice, 91-93% of all slots are taken (issue
-// active 60% + half of the FMA pipe's 63%).  The far flush alone runs at 15.1
+// two issue slots; counting those twice, 89-94% of all slots are taken (1M
+// particles: clustered 63% issue active + half of the FMA pipe's 53%, in groups of
+// 64 61% + half of 64%, galaxy 65% + half of 58%).  The far flush alone runs at 15.1
 // slots per entry and 32 targets (13 FP32 operations, one rsqrt, a share of the
 // loads), the near flush at 43 (49.9 before its softening record was {h^-2, m/h,
 // m/h^3}).
@@ -544,8 +545,8 @@ __device__ __forceinline__ void st_flag(int *p, int v)
 
 // The next sub-walk for a warp that found no group left, or -1.  Sub-walks are
 // numbered by cut; a warp takes the next number and waits until that cut is made or
-// every group is finished.  All groups are held by running warps by then, so the
-// wait ends; it is bounded all the same (some twenty seconds).
+// too few groups are unfinished for it.  All groups are held by running warps by
+// then, so the wait ends; it is bounded all the same (some twenty seconds).
 #define WALK_TASK_LIMIT (1 << 22)
 __device__ __noinline__ int next_task(const WalkParams &p, int ngroups)
 {
@@ -553,8 +554,14 @@ __device__ __noinline__ int next_task(const WalkParams &p, int ngroups)
     if (f >= p.fork_max) return -1;
     unsigned ns = 256;
     for (int i = 0; i < WALK_TASK_LIMIT; i++) {
-        const bool over = ld_flag(p.group_counter + WALK_DONE_COUNTER) >= ngroups;
-        if (over) __threadfence();   // cuts of finished groups are seen from here on
+        // is a cut left for this number?  Each unfinished group makes one more at most
+        const int *const done = p.group_counter + WALK_DONE_COUNTER, *const cuts = p.group_counter + WALK_FORK_COUNTER;
+        bool over = f >= ld_flag(cuts) + (ngroups - ld_flag(done));
+        if (over) {   // for certain: the finished groups first, then their cuts
+            const int left = ngroups - ld_flag(done);
+            __threadfence();
+            over = f >= ld_flag(cuts) + left;
+        }
         if (ld_flag(p.fork_ready + f)) {
             __threadfence();
             return t;
@@ -617,7 +624,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) k_walk(const __grid_constant_
     constexpr int LP = 32 / SPLIT;   // lanes per part
     constexpr int QUANTUM = 4 * SPLIT;
     const int part = lane / LP;
-    const int swz = TMA ? 0 : (lane >> 1) & 3;   // node slot pieces, see stage_node
+    const int swz = TMA ? 0 : (lane >> 1) & 3;   // node slot pieces, see stage_lanes
     const int FL = min(p.flush, FAR_FLUSH_MAX), NL = min(p.flush, NEAR_FLUSH_MAX);
     float *far = reinterpret_cast<float *>(walk_smem) + (size_t)warp * WALK_WARP_FLOATS;
     float *near = far + FAR_ARRAYS * FAR_CAP;
