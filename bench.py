@@ -37,16 +37,12 @@ import ics  # noqa: E402
 import multi  # noqa: E402
 
 FLOPS_PER_INTERACTION = 20   # monopole force convention (3 sub, r^2, rsqrt, m/r^3, 3 fma)
-# DRAM bytes (read + write) per particle of one k_walk launch on the galaxy,
-# from the ncu capture of the 1,000,000-particle galaxy (114.8 MB read + 39.6 MB
-# written); the walk's traffic grows with the particle count, so a launch of
-# the 4.2M galaxy is scaled from it
 # dram__bytes_read.sum + dram__bytes_write.sum of one k_walk launch: on the
 # clustered system measured at full size (16,777,216 particles, groups of 64,
-# a 1-pass capture: 4.77 GB read + 1.67 GB written); on the galaxy from the
-# capture of the 1,000,000-particle galaxy (114.8 MB read + 39.6 MB written),
-# scaled to the 4.2M galaxy by particle count
-WALK_DRAM_BYTES_PER_PARTICLE = {"galaxy": 154.4, "galaxy1m": 154.4, "clustered": 6.36e9 / 16777216}
+# a 1-pass capture: 5.38 GB read + 1.85 GB written); on the galaxy from a
+# 1,000,000-particle galaxy (125.7 MB read + 40.1 MB written), scaled to the 4.2M
+# galaxy by particle count
+WALK_DRAM_BYTES_PER_PARTICLE = {"galaxy": 165.8, "galaxy1m": 165.8, "clustered": 7.23e9 / 16777216}
 WALK_DRAM_SOURCE = {"galaxy": "ncu dram bytes of one k_walk launch on the 1M galaxy, scaled by N",
                     "galaxy1m": "ncu dram bytes of one k_walk launch on the 1M galaxy",
                     "clustered": "ncu dram bytes of one k_walk launch at full size (groups of 64; 1-pass capture)"}
