@@ -805,8 +805,8 @@ def run_system(args, torch, ggb200, dist, world, rank, local):
     tree.evaluate_device(d_acc, d_pot, err_tol_theta=0.7)
     tree.build()
     tree.evaluate_device(d_acc, d_pot, err_tol_force_acc=args.tol, err_tol_theta=0.0)
-    # the project's autotuner picks leaf and group size, flush threshold,
-    # blocks per SM and node staging on this system, refusing any candidate
+    # the autotuner picks leaf and group size, flush threshold
+    # and node staging on this system, refusing any candidate
     # less accurate than the default configuration (outside the timed region)
     tuned, tuned_ms, t_tune = None, None, 0.0
     if not args.no_autotune:

@@ -837,7 +837,9 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
             return st;
         gorder = c->gorder.p;
     }
-    GG_CUDA_TRY(cudaMemsetAsync(c->counters.p, 0, (WALK_COUNTERS + 2 * FORK_RECORDS) * sizeof(int), s));
+    // (without an OldAcc the relative criterion opens every node, and no walk is longer than the others)
+    const bool forks = may_fork(c, d_active != nullptr, ntargets) && (theta > 0 || c->oldacc_valid);
+    GG_CUDA_TRY(cudaMemsetAsync(c->counters.p, 0, (WALK_COUNTERS + (forks ? 2 * FORK_RECORDS : 0)) * sizeof(int), s));
     GG_CUDA_TRY(cudaMemsetAsync(c->inter.p, 0, 4 * sizeof(unsigned long long), s));
     WalkParams p;
     p.nodes = c->nodes.p;
@@ -861,8 +863,7 @@ static gg_status run_walk(gg_ctx *c, const int *d_active, int n_active, const do
     p.forks = c->forks.p;
     p.own_forks = c->own_forks.p;
     p.fork_max = ntargets <= FORK_TASK_TARGETS ? FORK_RECORDS : 0;
-    // (without an OldAcc the relative criterion opens every node, and no walk is longer than the others)
-    p.may_fork = may_fork(c, d_active != nullptr, ntargets) && (theta > 0 || p.oldacc_in);
+    p.may_fork = forks;
     p.fork_work = fork_work(tol, theta);
     p.fork_ready = c->counters.p + WALK_COUNTERS;
     p.fork_parts = p.fork_ready + FORK_RECORDS;
